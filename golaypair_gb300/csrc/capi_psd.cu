@@ -54,7 +54,7 @@ int gp_ctx::enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf,
     const double* tw = twiddle64(L);
     if (!tw) return fail(GP_ERR_NOMEM, "twiddle table");
     if (mode == GP_PSD_FP64) {
-        gp::PsdF64Args a{src, tw, n, threshold(order, paf), d_mask, words};
+        gp::PsdF64Args a{src, tw, n, threshold(order, paf), d_mask, words, num_sms};
         cudaEvent_t tb;
         time_begin(st, &tb);
         GP_CUDA_TRY(this, gp::launch_psd_fp64(a, st));

@@ -138,6 +138,7 @@ struct PsdF64Args {
     double thr;
     uint32_t* mask;
     int64_t mask_words;
+    int num_sms;
 };
 cudaError_t launch_psd_fp64(const PsdF64Args& a, cudaStream_t st);
 
