@@ -18,18 +18,19 @@ float guard_band(int order) { return (float)(2e-3 * order); }
 
 }  // namespace
 
-const void* gp_ctx::twiddle_image(int L, bool int8_rows, int* shift) {
+const void* gp_ctx::twiddle_image(int L, bool int8_rows, int* shift, bool both) {
     const bool sh = int8_rows && gp::tc_i8_shifted(L);
     if (shift) *shift = sh ? 1 : 0;
     const int wrap = sh ? gp::tc_i8_wrap_rows(L) : 0;
-    const int key = 4 * L + wrap;
-    auto it = twiddles.find(key);
-    if (it != twiddles.end()) return it->second.p;
     const int K = gp::tc_k_for_len(L);
     if (!K) return nullptr;
-    const size_t bytes = gp::build_twiddle_image(L, K, nullptr, wrap);
+    const int halves = both ? 2 : gp::tc_image_halves(K);
+    const int key = 2 * (4 * L + wrap) + halves - 1;
+    auto it = twiddles.find(key);
+    if (it != twiddles.end()) return it->second.p;
+    const size_t bytes = gp::build_twiddle_image(L, K, halves, nullptr, wrap);
     std::vector<uint8_t> img(bytes);
-    gp::build_twiddle_image(L, K, img.data(), wrap);
+    gp::build_twiddle_image(L, K, halves, img.data(), wrap);
     DevBuf& b = twiddles[key];
     if (!b.ensure(bytes)) return nullptr;
     if (cudaMemcpy(b.p, img.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
@@ -76,6 +77,7 @@ int gp_ctx::enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf,
     a.n = n;
     a.L = L;
     a.bimage = img;
+    a.tw64 = tw;
     a.thr = (float)threshold(order, paf);
     a.guard_cfg = guard_band(order);
     a.err_coef = gp::tc_err_coef(gp::tc_k_for_len(L));
@@ -116,6 +118,7 @@ int gp_ctx::enqueue_filter_dev(const gp::RowSrc& src, int64_t cap, const unsigne
     a.grid_per_sm = grid_per_sm;
     a.L = L;
     a.bimage = img;
+    a.tw64 = tw;
     a.thr = (float)threshold(order, paf);
     a.guard_cfg = guard_band(order);
     a.err_coef = gp::tc_err_coef(gp::tc_k_for_len(L));
@@ -159,6 +162,7 @@ int gp_ctx::enqueue_filter_multi(const gp::RowSrc* src, const int64_t* cap, cons
         a.grid_per_sm = grid_per_sm;
         a.L = L;
         a.bimage = img;
+        a.tw64 = tw;
         a.thr = (float)threshold(order[j], paf[j]);
         a.guard_cfg = guard_band(order[j]);
         a.err_coef = gp::tc_err_coef(gp::tc_k_for_len(L));
@@ -532,8 +536,9 @@ int gp_psd_tc_values(gp_ctx* c, const int8_t* seqs, int64_t n, int L, float* out
         return c->fail(GP_ERR_NOMEM, "allocation failed");
     GP_CUDA_TRY(c, cudaMemcpy(ds.p, seqs, (size_t)n * L, cudaMemcpyHostToDevice));
     int shift = 0;
-    const void* img = c->twiddle_image(L, true, &shift);
+    const void* img = c->twiddle_image(L, true, &shift, true);
     if (!img) return c->fail(GP_ERR_UNSUPPORTED, "length %d", L);
+    const double* tw = nullptr;  // not read: every row is decided from both halves
     GP_CUDA_TRY(c, cudaMemset(c->counts.p, 0, sizeof(unsigned long long)));
     gp::PsdTcArgs a;
     a.i8_shift = shift;
@@ -544,6 +549,7 @@ int gp_psd_tc_values(gp_ctx* c, const int8_t* seqs, int64_t n, int L, float* out
     a.n = n;
     a.L = L;
     a.bimage = img;
+    a.tw64 = tw;
     a.thr = 1e30f;
     a.guard_cfg = 0.f;
     a.err_coef = 0.f;

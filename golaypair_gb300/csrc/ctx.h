@@ -114,7 +114,7 @@ struct gp_ctx {
     DevBuf seq_buf[2];
     DevBuf mask_buf[2];
     DevBuf unsure_buf[2];
-    std::map<int, DevBuf> twiddles;    // tensor-core B images, by 4 L + wrapped rows
+    std::map<int, DevBuf> twiddles;    // tensor-core B images, by 2 (4 L + wrapped rows) + halves - 1
     std::map<int, DevBuf> twiddles64;  // FP64 (cos, sin) tables, by L
     // optional CUDA-event timing of the main filter kernel (profiling)
     bool timing = false;
@@ -164,7 +164,8 @@ struct gp_ctx {
     // device twiddle image for length L (tensor-core filter)
     // tensor-core B image of length L: with the wrapped rows of shifted int8
     // loads when int8_rows and the length takes them (*shift set to 1)
-    const void* twiddle_image(int L, bool int8_rows = false, int* shift = nullptr);
+    // (both halves of the twiddles for the PSD values, the filter's otherwise)
+    const void* twiddle_image(int L, bool int8_rows = false, int* shift = nullptr, bool both = false);
     // Multi-job tensor-core filter of device batches (packed words) followed
     // by the FP64 recheck of every job's unsure rows: two launches on st for
     // up to eight jobs, each job's tiles at its own padded K.  Per job as

@@ -26,7 +26,8 @@ struct PsdTcArgs {
     const unsigned long long* n_dev = nullptr;  // optional: row count read on the device, min(n, *n_dev)
     int grid_per_sm = 0;     // CTAs per SM (0 = as many as fit)
     int L;
-    const void* bimage;      // twiddles: hi tile then lo tile, UMMA smem image
+    const void* bimage;      // twiddles, UMMA smem image (tc_image_halves(K) of them; both with psd_out)
+    const double* tw64;      // FP64 (cos, sin) table of length L
     float thr;               // T = 2n - paf + 0.001
     float guard_cfg;         // configured guard band (absolute)
     float err_coef;          // per-row |X| error bound = S_row * err_coef
@@ -59,12 +60,16 @@ enum TcTrace {
     kTrConvSt, kTrEpiTail, kTrCount
 };
 
-// Builds the B-operand image (hi and lo twiddles) for length L, K = padded L.
+// Halves of the twiddles (hi, or hi and lo) in the filter's B image.
+constexpr int kMaxHiLoK = 48;  // largest padded K that keeps both halves in the accumulator
+__host__ __device__ constexpr int tc_image_halves(int K) { return K <= kMaxHiLoK ? 2 : 1; }
+
+// Builds the B-operand image (hi, or hi and lo twiddles) for length L, K = padded L.
 // Rows j = L .. L + wrap - 1 of the sequence axis hold the twiddles of
 // j - L (the DFT's period), for int8 rows loaded with a shift; every other
 // row past L is zero.  Returns its size in bytes; writes it to out when
 // out != nullptr.
-size_t build_twiddle_image(int L, int K, void* out, int wrap = 0);
+size_t build_twiddle_image(int L, int K, int halves, void* out, int wrap = 0);
 int tc_k_for_len(int L);               // padded K (multiple of 16, > L), or 0 if unsupported
 
 // Shifted loads of int8 rows (PsdTcArgs::i8_shift).  A row of length L that
@@ -77,14 +82,14 @@ bool tc_i8_shifted(int L);
 int tc_i8_wrap_rows(int L);  // wrapped image rows for the shifted loads (max s), 0 if they do not apply
 
 // Where twiddle row `nrow` (0..K-1), column j (0..K-1), part (0 hi, 1 lo)
-// sits in the B image, as an index of fp16 elements.  The image is a 2K x K
-// fp16 matrix (hi part at row nrow, lo part at row K + nrow) in the
-// canonical no-swizzle K-major layout of 8 x 8 core matrices: core matrix
-// (n/8, j/8) at byte (j/8) * (2K/8) * 128 + (n/8) * 128, row n%8 at +16,
-// column j%8 at +2.
-__host__ __device__ inline size_t tc_image_index(int nrow, int j, int part, int K) {
+// sits in the B image, as an index of fp16 elements.  The image is an
+// (halves K) x K fp16 matrix (hi part at row nrow, lo part at row K + nrow)
+// in the canonical no-swizzle K-major layout of 8 x 8 core matrices: core
+// matrix (n/8, j/8) at byte (j/8) * (halves K/8) * 128 + (n/8) * 128, row
+// n%8 at +16, column j%8 at +2.
+__host__ __device__ inline size_t tc_image_index(int nrow, int j, int part, int K, int halves) {
     const int n = nrow + part * K;
-    return ((size_t)(j / 8) * (2 * K / 8) * 128 + (size_t)(n / 8) * 128 + (size_t)(n % 8) * 16 + (j % 8) * 2) / 2;
+    return ((size_t)(j / 8) * (halves * K / 8) * 128 + (size_t)(n / 8) * 128 + (size_t)(n % 8) * 16 + (j % 8) * 2) / 2;
 }
 
 // Bin of twiddle row nrow: cosine rows 0..K/2-1 are bins 1..K/2, sine rows

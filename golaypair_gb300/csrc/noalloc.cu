@@ -39,7 +39,7 @@ namespace gp {
 namespace {
 
 constexpr int64_t kNoAllocMaxRows = int64_t(1) << 20;
-constexpr size_t kImageBytes = 2 * (size_t)kMaxTcK * kMaxTcK * 2;  // hi + lo tiles at K = 128
+constexpr size_t kImageBytes = (size_t)kMaxTcK * kMaxTcK * 2;  // hi twiddles at K = 128 (both halves up to K = 48 take less)
 constexpr size_t kTw64Bytes = 2 * (size_t)kMaxTcK * sizeof(double);
 // layout of the scratch array (byte offsets, 256-aligned)
 constexpr size_t kOffStatus = 0;                            // int status
@@ -54,7 +54,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 // Twiddles built on the device: the tensor-core image in the same canonical
 // layout as build_twiddle_image (wrap: rows L .. L + wrap - 1 continue the
 // period, for shifted int8 loads), and the FP64 (cos, sin) table.
-__global__ void noalloc_twiddles_kernel(unsigned char* scratch, int L, int K, int wrap) {
+__global__ void noalloc_twiddles_kernel(unsigned char* scratch, int L, int K, int halves, int wrap) {
     uint16_t* img = reinterpret_cast<uint16_t*>(scratch + kOffImage);
     double* tw = reinterpret_cast<double*>(scratch + kOffTw64);
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < K * K; e += gridDim.x * blockDim.x) {
@@ -70,8 +70,8 @@ __global__ void noalloc_twiddles_kernel(unsigned char* scratch, int L, int K, in
         }
         const __half h = __double2half(w);
         const __half l = __double2half(w - (double)__half2float(h));
-        img[tc_image_index(nrow, j, 0, K)] = __half_as_ushort(h);
-        img[tc_image_index(nrow, j, 1, K)] = __half_as_ushort(l);
+        img[tc_image_index(nrow, j, 0, K, halves)] = __half_as_ushort(h);
+        if (halves == 2) img[tc_image_index(nrow, j, 1, K, halves)] = __half_as_ushort(l);
     }
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < L; m += gridDim.x * blockDim.x) {
         double s, c;
@@ -132,7 +132,7 @@ extern "C" int gp_psd_filter_noalloc(const int8_t* d_seqs, int64_t n, int L, int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // clear what the kernels count from zero; the rest is overwritten
     if (cudaMemsetAsync(s + kOffStatus, 0, 512, st) != cudaSuccess) return GP_ERR_CUDA;
-    noalloc_twiddles_kernel<<<64, 256, 0, st>>>(s, L, K, tc_i8_wrap_rows(L));
+    noalloc_twiddles_kernel<<<64, 256, 0, st>>>(s, L, K, tc_image_halves(K), tc_i8_wrap_rows(L));
     if (cudaGetLastError() != cudaSuccess) return GP_ERR_CUDA;
     const double thr = 2.0 * order - paf + 0.001;
     PsdTcArgs a;
@@ -143,6 +143,7 @@ extern "C" int gp_psd_filter_noalloc(const int8_t* d_seqs, int64_t n, int L, int
     a.n = n;
     a.L = L;
     a.bimage = s + kOffImage;
+    a.tw64 = reinterpret_cast<const double*>(s + kOffTw64);
     a.i8_shift = tc_i8_shifted(L) ? 1 : 0;
     a.thr = (float)thr;
     a.guard_cfg = (float)(2e-3 * order);

@@ -28,6 +28,9 @@
 // decides from the hi columns alone, with a guard widened by the hi-only
 // twiddle error; only a warp with a row inside that wider band reads the lo
 // columns too and decides again (about 1e-5 of the warps on int8 input).
+// Above K = 48 the accumulator holds the hi columns alone (N = K), so that two
+// CTAs fit an SM, and a row inside the band is decided again in fp32 by its
+// epilogue warp.
 //
 // Each candidate is classified against T = 2n - paf + 0.001 with a guard g
 // (the configured band, widened per row to a rigorous bound on the fp32
@@ -67,7 +70,7 @@ namespace gp {
 namespace {
 
 template <int K, int B, bool WRITE_PSD, bool TR, bool SH>
-__global__ void __launch_bounds__(kThreads, TcCfg<K>::MIN_BLOCKS) psd_tc_kernel(PsdTcArgs a, SmemLayout lay) {
+__global__ void __launch_bounds__(kThreads, TcCfg<K, WRITE_PSD>::MIN_BLOCKS) psd_tc_kernel(PsdTcArgs a, SmemLayout lay) {
     tc_body<K, B, WRITE_PSD, TR, SH>(a, lay, blockIdx.x, gridDim.x);
 }
 
@@ -76,8 +79,8 @@ constexpr int kMaxShiftK = 64;
 
 template <int K, int B, bool WP>
 cudaError_t launch_kb(const PsdTcArgs& a, int num_sms, cudaStream_t st) {
-    using C = TcCfg<K>;
-    const SmemLayout lay = smem_layout<K>(B == 0 ? a.L : 16);
+    using C = TcCfg<K, WP>;
+    const SmemLayout lay = smem_layout<K, WP>(B == 0 ? a.L : 16);
     const int64_t ntiles = (a.n + kTileM - 1) / kTileM;
     if (ntiles == 0) return cudaSuccess;
     if (a.n >= (int64_t(1) << 31)) return cudaErrorInvalidValue;  // 32-bit row indices
@@ -195,10 +198,10 @@ float tc_err_coef(int K) {
     return (float)(std::sqrt(2.0) * (std::ldexp(1.0, -24) + steps * 17.0 * std::ldexp(1.0, -22)));
 }
 
-size_t build_twiddle_image(int L, int K, void* out, int wrap) {
-    const size_t bytes = (size_t)2 * K * K * 2;
+size_t build_twiddle_image(int L, int K, int halves, void* out, int wrap) {
+    const size_t bytes = (size_t)halves * K * K * 2;
     if (!out) return bytes;
-    std::vector<uint16_t> img((size_t)2 * K * K, 0);
+    std::vector<uint16_t> img((size_t)halves * K * K, 0);
     const double two_pi = 6.283185307179586476925286766559;
     const int jend = L + wrap < K ? L + wrap : K;
     for (int nrow = 0; nrow < K; ++nrow) {
@@ -210,8 +213,8 @@ size_t build_twiddle_image(int L, int K, void* out, int wrap) {
             const double w = kind == 3 ? 1.0 : kind == 2 ? std::sin(two_pi * m / L) : std::cos(two_pi * m / L);
             const uint16_t h = half_bits(w);
             const uint16_t l = half_bits(w - half_value(h));
-            img[tc_image_index(nrow, j, 0, K)] = h;
-            img[tc_image_index(nrow, j, 1, K)] = l;
+            img[tc_image_index(nrow, j, 0, K, halves)] = h;
+            if (halves == 2) img[tc_image_index(nrow, j, 1, K, halves)] = l;
         }
     }
     std::memcpy(out, img.data(), bytes);

@@ -9,6 +9,7 @@
 
 #include "gp_device.cuh"
 #include "gp_internal.h"
+#include "rows.cuh"
 
 namespace gp {
 
@@ -22,34 +23,43 @@ constexpr uint32_t kSmemBudget2Cta = 112 * 1024;  // two CTAs per SM
 constexpr uint32_t kSmemBudget1Cta = 220 * 1024;
 constexpr int kLutBytes = 4096;
 
-// accumulator buffers and TMEM A stages per K (columns: NACC*N + AS*K/2)
-constexpr int tc_nacc(int K) { return K == 16 ? 4 : K == 32 ? 3 : K == 48 ? 2 : K == 64 ? 3 : K <= 96 ? 2 : K == 112 ? 2 : 1; }
-constexpr int tc_as(int K) { return K == 16 ? 4 : K == 32 ? 3 : K == 48 ? 2 : K <= 80 ? 4 : K == 96 ? 2 : K == 112 ? 1 : 4; }
-
-template <int K>
+// Up to K = 48 the accumulator holds both halves of the twiddles (N = 2K: an
+// MMA takes as long as N = K, and two accumulators fit a CTA's 256 columns).
+// Above, both halves cost MMA time and TMEM: one CTA of 512 columns per SM.
+// There the filter keeps the hi half alone (N = K), so that two CTAs fit, and
+// the rare rows inside the hi-only band are decided again from fp32 twiddles
+// (near_rows).  The PSD values always take both halves.
+// 2^24 x 57 rows: 0.261 ms against 0.420 with both halves and one CTA; 2^24 x
+// 98: 0.47 against 0.92.  (K = 96: one accumulator and three A stages, 0.241 ms
+// for 2^23 x 85; two and one: 0.271.)
+template <int K, bool WRITE_PSD>
 struct TcCfg {
+    static constexpr bool HILO = WRITE_PSD || tc_image_halves(K) == 2;
     static constexpr int M = kTileM;
-    static constexpr int N = 2 * K;                    // UMMA N: K/2 cosine + K/2 sine bins, hi then lo
+    static constexpr int N = HILO ? 2 * K : K;         // UMMA N: K/2 cosine + K/2 sine bins (hi, then lo)
     static constexpr int KCH = K / 8;                  // 8-element chunks along K
     static constexpr int KW = K / 4 + 1;               // 32-bit words covering a row's K bytes + misalignment
     static constexpr int KSTEPS = K / 16;              // UMMA K steps (instructions) per tile
-    static constexpr int B_BYTES = 2 * K * K * 2;      // whole B image (hi and lo)
+    static constexpr int B_BYTES = N * K * 2;          // whole B image
     static constexpr int B_KSTRIDE = (N / 8) * 128;    // bytes between core matrices adjacent in K
-    static constexpr int MIN_BLOCKS = K <= 48 ? 2 : 1;
+    static constexpr int MIN_BLOCKS = K > kMaxHiLoK && HILO ? 1 : 2;
     static constexpr int TMEM_COLS = MIN_BLOCKS == 2 ? 256 : 512;
-    static constexpr int NACC = tc_nacc(K);
-    static constexpr int AS = tc_as(K);                // A stages in TMEM
+    // accumulator buffers and TMEM A stages (columns: NACC * N + AS * K/2)
+    static constexpr int NACC = !HILO ? (K <= 80 ? 2 : 1)
+                                : K == 16 ? 4 : K == 32 ? 3 : K == 48 ? 2 : K == 64 ? 3 : K <= 112 ? 2 : 1;
+    static constexpr int AS = !HILO ? (K == 96 ? 3 : 2)
+                              : K == 16 ? 4 : K == 32 ? 3 : K == 48 ? 2 : K <= 80 ? 4 : K == 96 ? 2 : K == 112 ? 1 : 4;
     static constexpr int A_COL0 = NACC * N;            // first TMEM column of the A stages
     static_assert(NACC * N + AS * K / 2 <= TMEM_COLS, "TMEM budget");
 };
 
 struct SmemLayout {
-    uint32_t b_off, lut_off, raw_off, raw_stride, raw_stages, bar_off, misc_off, total;
+    uint32_t b_off, lut_off, tw_off, raw_off, raw_stride, raw_stages, bar_off, misc_off, total;
 };
 
-template <int K>
+template <int K, bool WRITE_PSD>
 SmemLayout smem_layout(int row_bytes) {
-    using C = TcCfg<K>;
+    using C = TcCfg<K, WRITE_PSD>;
     SmemLayout s;
     uint32_t off = 0;
     s.b_off = off;
@@ -57,6 +67,8 @@ SmemLayout smem_layout(int row_bytes) {
     off = (off + 1023) & ~1023u;
     s.lut_off = off;
     off += kLutBytes;
+    s.tw_off = off;  // fp32 twiddles of near_rows
+    if (!C::HILO) off += kMaxTcK * (uint32_t)sizeof(float2);
     s.bar_off = off;
     off += (2 * kMaxRawStages + 2 * C::AS + 2 * C::NACC + 2) * 8;
     s.misc_off = off;
@@ -147,6 +159,23 @@ __device__ __forceinline__ uint4 packed_chunk(const uint32_t (&w)[4], const uint
         out = make_uint4(l[(field >> 24) & 255], l[(field >> 16) & 255], l[(field >> 8) & 255], l[field & 255]);
     }
     return out;
+}
+
+// 16 digits 16 g .. 16 g + 15 as the eight fp16 pairs of a TMEM store.
+template <int B, int G>
+__device__ __forceinline__ void packed_group(const uint32_t (&w)[4], const uint8_t* lut, uint32_t (&h)[8]) {
+    const uint4 u = packed_chunk<B, 2 * G>(w, lut), v = packed_chunk<B, 2 * G + 1>(w, lut);
+    h[0] = u.x, h[1] = u.y, h[2] = u.z, h[3] = u.w;
+    h[4] = v.x, h[5] = v.y, h[6] = v.z, h[7] = v.w;
+}
+template <int B, int G, int GEND>
+__device__ __forceinline__ void packed_store(const uint32_t (&w)[4], const uint8_t* lut, uint32_t aaddr) {
+    if constexpr (G < GEND) {
+        uint32_t h[8];
+        packed_group<B, G>(w, lut, h);
+        tmem_st8(aaddr + 8 * G, h);
+        packed_store<B, G + 1, GEND>(w, lut, aaddr);
+    }
 }
 
 template <int B, int CH, int CHEND>
@@ -269,6 +298,98 @@ __device__ __forceinline__ void psd_hi_all(uint32_t taddr, float& pmax, float& x
     pmax = fmaxf(pm[0], pm[1]);
 }
 
+// The same for HB > 32, 32 bins at a time (registers).
+template <int HB, int C0, bool TR>
+__device__ __forceinline__ void psd_hi_blocks(uint32_t taddr, float& pmax, float& x0, long long& t_ld) {
+    constexpr int W = HB - C0 < 32 ? HB - C0 : 32;
+    float chi[W], shi[W];
+    tmem_ld_cols<W>(taddr + C0, chi);
+    tmem_ld_cols<W>(taddr + HB + C0, shi);
+    tmem_wait_ld();
+    float pm[2] = {pmax, 0.f};  // two independent max chains
+#pragma unroll
+    for (int k = 0; k < W; k += 2) {
+        const float2 re = make_float2(chi[k], chi[k + 1]);
+        const float2 im = make_float2(shi[k], shi[k + 1]);
+        const float2 p = __ffma2_rn(re, re, __fmul2_rn(im, im));
+        float& m = pm[(k >> 1) & 1];
+        if (C0 + k + 1 == HB - 1) {
+            m = fmaxf(m, p.x);
+            x0 = re.y;
+        } else {
+            m = fmax3(m, p.x, p.y);
+        }
+    }
+    pmax = fmaxf(pm[0], pm[1]);
+    if constexpr (C0 + W < HB)
+        psd_hi_blocks<HB, C0 + W, TR>(taddr, pmax, x0, t_ld);
+    else
+        t_ld = tclock<TR>();
+}
+
+// Without the lo half: max p and X_0 of the warp's rows flagged in `near` (row
+// r0 + i for bit i) again, from the input and fp32 twiddles, one row at a time
+// with the bins over the lanes; lane i of a flagged row gets its pair, the
+// others keep theirs.  The sum over at most 127 terms of products rounded to
+// 2^-24 each is within the accumulator's own error bound (tc_err_coef).
+// Out of line: about 1e-5 of the rows of int8 input.
+template <int B>
+__device__ __noinline__ float2 near_rows(const PsdTcArgs& a, const float2* s_tw, uint32_t near, int r0, float2 mine) {
+    const int lane = threadIdx.x & 31, L = a.L, H = L / 2;
+    while (near) {
+        const int i = __ffs((int)near) - 1;
+        near &= near - 1u;
+        const int64_t row = r0 + i;
+        uint64_t lo = 0, hi = 0;
+        if constexpr (B != 0) {
+            const uint4 w = a.words[row];
+            lo = ((uint64_t)w.y << 32) | w.x;
+            hi = ((uint64_t)w.w << 32) | w.z;
+        }
+        int x[4];  // the row over the lanes: entries lane + 32 c (L <= 127)
+        int sum = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int j = lane + 32 * c;
+            x[c] = 0;
+            if (j < L) {
+                if constexpr (B == 0)
+                    x[c] = a.seqs[row * L + j];
+                else
+                    x[c] = 2 * word_digit(lo, hi, B, L, j) - a.alpha_c;
+            }
+            sum += x[c];
+        }
+        float pm = 0.f;
+        for (int k0 = 1; k0 <= H; k0 += 32) {
+            const int k = k0 + lane <= H ? k0 + lane : H;
+            float re = 0.f, im = 0.f;
+            int m = 0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int nj = L - 32 * c < 32 ? L - 32 * c : 32;
+                const float xc = (float)x[c];
+#pragma unroll 4
+                for (int j = 0; j < nj; ++j) {
+                    const float v = __shfl_sync(0xFFFFFFFFu, xc, j);
+                    const float2 w = s_tw[m];
+                    re = fmaf(v, w.x, re);
+                    im = fmaf(v, w.y, im);
+                    m += k;
+                    if (m >= L) m -= L;
+                }
+            }
+            pm = fmaxf(pm, fmaf(re, re, im * im));
+        }
+        for (int o = 16; o; o >>= 1) {
+            pm = fmaxf(pm, __shfl_xor_sync(0xFFFFFFFFu, pm, o));
+            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        }
+        if (lane == i) mine = make_float2(pm, (float)sum);
+    }
+    return mine;
+}
+
 // A row of a tile that is not whole or not bulk-copied (the last tile, or
 // an input not 16-byte aligned): byte loads from global memory, zeros past
 // row n or column L, stored as the A row at TMEM address aaddr.  Out of line: it runs at most once per CTA on aligned
@@ -312,12 +433,13 @@ __device__ __noinline__ float2 exact_pass(uint32_t taddr, float* psd_row) {
 // stride, ... of the job (the one-job kernel: its CTA index and grid size).
 template <int K, int B, bool WRITE_PSD, bool TR, bool SH = false>
 __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& lay, int first, int stride) {
-    using C = TcCfg<K>;
+    using C = TcCfg<K, WRITE_PSD>;
     extern __shared__ uint8_t smem_raw_base[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) & ~uintptr_t(1023));
 
     uint8_t* sB = smem + lay.b_off;
     uint8_t* sLut = smem + lay.lut_off;
+    float2* sTw = reinterpret_cast<float2*>(smem + lay.tw_off);
     uint8_t* sRaw = smem + lay.raw_off;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.bar_off);
     uint64_t* raw_full = bars;
@@ -372,6 +494,9 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
         mbar_fence_init();
     }
     if constexpr (B != 0) build_lut(sLut, B, a.alpha_c);
+    if constexpr (!C::HILO)
+        for (int m = threadIdx.x; m < L; m += blockDim.x)
+            sTw[m] = make_float2((float)a.tw64[2 * m], (float)a.tw64[2 * m + 1]);
     if (warp == 9) {
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tc_fence_before();
@@ -428,7 +553,8 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
             tc_fence_after();
             const int row = t * kTileM + r;
             const bool full_tile = t < nfull;
-            uint32_t h[K / 2];  // the row as fp16 pairs
+            constexpr bool kGroups = K > 64;  // stored 16 columns at a time (registers)
+            uint32_t h[kGroups ? 1 : K / 2];  // the row as fp16 pairs
             const uint32_t aaddr = lane_base + (uint32_t)(as * (K / 2));
             if constexpr (B == 0) {
                 if (full_tile) {
@@ -442,6 +568,20 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
                             biased_u8x4_to_h2x2((wp[2 * c] & mk[2 * c]) ^ 0x80808080u, h[4 * c], h[4 * c + 1]);
                             biased_u8x4_to_h2x2((wp[2 * c + 1] & mk[2 * c + 1]) ^ 0x80808080u, h[4 * c + 2],
                                                 h[4 * c + 3]);
+                        }
+                    } else if constexpr (kGroups) {
+                        const uint32_t sh = (uint32_t)(off & 3) * 8u;
+                        uint32_t w0 = wp[0];
+#pragma unroll
+                        for (int g = 0; g < K / 16; ++g) {
+                            uint32_t hg[8];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const uint32_t w1 = wp[4 * g + i + 1];
+                                i8x4_to_h2x2(__funnelshift_r(w0, w1, sh), hg[2 * i], hg[2 * i + 1]);
+                                w0 = w1;
+                            }
+                            tmem_st8(aaddr + 8 * g, hg);
                         }
                     } else {
                         const uint32_t sh = (uint32_t)(off & 3) * 8u;
@@ -468,12 +608,15 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
                 }
                 uint32_t sw[4];
                 shl128(wv, norm, sw);
-                packed_row<B, 0, C::KCH>(sw, sLut, h);
+                if constexpr (kGroups)
+                    packed_store<B, 0, K / 16>(sw, sLut, aaddr);
+                else
+                    packed_row<B, 0, C::KCH>(sw, sLut, h);
             }
             const long long c25t = tclock<TR>();
-            if (B != 0 || full_tile) {
+            if (!kGroups && (B != 0 || full_tile)) {
 #pragma unroll
-                for (int g = 0; g < K / 16; ++g) tmem_st8(aaddr + 8 * g, h + 8 * g);
+                for (int g = 0; g < (kGroups ? 0 : K / 16); ++g) tmem_st8(aaddr + 8 * g, h + 8 * g);
             }
             tmem_wait_st();
             const long long c3t = tclock<TR>();
@@ -551,24 +694,43 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
             // cos lo, [K + HB, 2K) sin lo; cos column HB - 1 is the row sum X_0.
             // First the hi columns alone, with the wider hi-only guard: a
             // row clearly below or above the bound is decided there.  Only
-            // a warp with a row inside that band reads the lo columns too
-            // (rare: about 1e-5 of the rows of the int8 workload).
+            // a warp with a row inside that band reads the lo columns too,
+            // or, where the accumulator has none, takes that row's bins
+            // again in fp32 (rare: about 1e-5 of the rows of the int8
+            // workload).
             float pmax = 0.f, x0 = 0.f, g = 0.f;
             long long c_ld = c1t;
             bool exact = WRITE_PSD;
             if constexpr (!WRITE_PSD) {
-                psd_hi_all<HB, TR>(taddr, pmax, x0, c_ld);
+                if constexpr (HB <= 32)
+                    psd_hi_all<HB, TR>(taddr, pmax, x0, c_ld);
+                else
+                    psd_hi_blocks<HB, 0, TR>(taddr, pmax, x0, c_ld);
                 g = guard(pmax, x0, sc_hi);
                 // only picks the warps that redo the row exactly: the verdict
                 // below is taken with the same bounds either way
                 const bool near = valid && fabsf(pmax - thr) <= g;
-                exact = __any_sync(0xFFFFFFFFu, near);
+                if constexpr (C::HILO) {
+                    exact = __any_sync(0xFFFFFFFFu, near);
+                } else {
+                    const uint32_t nm = __ballot_sync(0xFFFFFFFFu, near);
+                    if (nm) {
+                        const float2 px = near_rows<B>(a, sTw, nm, t * kTileM + q * 32, make_float2(pmax, x0));
+                        if (near) {
+                            pmax = px.x;
+                            x0 = px.y;
+                            g = guard(pmax, x0, sc_lo);
+                        }
+                    }
+                }
             }
-            if (exact) {
-                const float2 px = exact_pass<HB, WRITE_PSD>(taddr, valid ? a.psd_out + (int64_t)row * HB : nullptr);
-                pmax = px.x;
-                x0 = px.y;
-                g = guard(pmax, x0, sc_lo);
+            if constexpr (C::HILO) {
+                if (exact) {
+                    const float2 px = exact_pass<HB, WRITE_PSD>(taddr, valid ? a.psd_out + (int64_t)row * HB : nullptr);
+                    pmax = px.x;
+                    x0 = px.y;
+                    g = guard(pmax, x0, sc_lo);
+                }
             }
             tc_fence_before();
             __syncwarp();

@@ -77,10 +77,9 @@ __device__ __forceinline__ void with_k(int K, F&& f) {
     }
 }
 
-// KMAX 48: two CTAs per SM (every job's TMEM share is 256 columns);
-// KMAX 64: one CTA per SM.
+// Two CTAs per SM: every job's TMEM share is 256 columns.
 template <int KMAX>
-__global__ void __launch_bounds__(kThreads, KMAX <= 48 ? 2 : 1) psd_tc_multi_kernel(PsdTcMultiArgs m, SmemLayout lay) {
+__global__ void __launch_bounds__(kThreads, 2) psd_tc_multi_kernel(PsdTcMultiArgs m, SmemLayout lay) {
     const MultiSlot s = multi_slot(m);
     if (s.job < 0) return;
     const PsdTcArgs& a = m.job[s.job];
@@ -100,17 +99,20 @@ __global__ void __launch_bounds__(kThreads, KMAX <= 48 ? 2 : 1) psd_tc_multi_ker
     });
 }
 
-// The layout of the largest job's one-job kernel, with the barrier region
-// sized for any K's stage counts and at most one (KMAX 64) or two CTAs per SM.
+// The layout of the largest job's one-job kernel, with the B and barrier
+// regions sized for any K's image and stage counts and two CTAs per SM.
 template <int KMAX>
 SmemLayout multi_layout() {
     SmemLayout s;
     uint32_t off = 0;
     s.b_off = off;
-    off += TcCfg<KMAX>::B_BYTES;
+    off += KMAX > 48 && TcCfg<48, false>::B_BYTES > TcCfg<KMAX, false>::B_BYTES ? TcCfg<48, false>::B_BYTES
+                                                                              : TcCfg<KMAX, false>::B_BYTES;
     off = (off + 1023) & ~1023u;
     s.lut_off = off;
     off += kLutBytes;
+    s.tw_off = off;
+    off += kMaxTcK * (uint32_t)sizeof(float2);
     s.bar_off = off;
     off += (2 * kMaxRawStages + 2 * 4 + 2 * 4 + 2) * 8;  // AS, NACC <= 4 for every K
     s.misc_off = off;
@@ -118,16 +120,14 @@ SmemLayout multi_layout() {
     off = (off + 127) & ~127u;
     s.raw_stride = (uint32_t)((kTileM * 16 + kRawSlack + 127) & ~127);
     s.raw_off = off;
-    const uint32_t budget = (KMAX <= 48 ? kSmemBudget2Cta : kSmemBudget1Cta) - 1024;
+    const uint32_t budget = kSmemBudget2Cta - 1024;
     int st = budget > off ? (int)((budget - off) / s.raw_stride) : 0;
     if (st > kMaxRawStages) st = kMaxRawStages;
     if (st < 2) st = 2;
     s.raw_stages = (uint32_t)st;
     off += st * s.raw_stride;
     s.total = off + 1024;
-    // TMEM: two CTAs of 256 columns, or one of up to 512
-    const uint32_t floor = KMAX <= 48 ? 96 * 1024 : 116 * 1024;
-    if (s.total < floor) s.total = floor;
+    if (s.total < 96 * 1024) s.total = 96 * 1024;  // TMEM: at most two CTAs of 256 columns
     return s;
 }
 
@@ -140,7 +140,7 @@ cudaError_t launch_multi(const PsdTcMultiArgs& a, int num_sms, cudaStream_t st) 
     int64_t cap_tiles = 0;
     for (int j = 0; j < a.njobs; ++j) cap_tiles += (a.job[j].n + kTileM - 1) / kTileM;
     if (cap_tiles == 0) return cudaSuccess;
-    const int fit = KMAX <= 48 ? 2 : 1;
+    const int fit = 2;
     const int per_sm = a.grid_per_sm > 0 && a.grid_per_sm < fit ? a.grid_per_sm : fit;
     int64_t grid = (int64_t)num_sms * per_sm;
     if (grid > cap_tiles) grid = cap_tiles;
