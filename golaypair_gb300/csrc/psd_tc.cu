@@ -53,7 +53,7 @@
 //   warps 0-3  convert: staged tile -> fp16 row in TMEM
 //   warps 4-7  epilogue: TMEM -> registers -> PSD max -> mask / unsure list
 //   warp 8     producer: cp.async.bulk of each tile into a deep ring
-//   warp 9     MMA issuer (one lane) and TMEM owner
+//   warp 9     MMA issuer (one lane issues) and TMEM owner
 // Rings of mbarriers hand tiles between the roles; every wait is bounded
 // (a timeout records a site code and the CTA unwinds).  With as many A
 // stages as accumulators, the MMAs of a tile free its A stage when they

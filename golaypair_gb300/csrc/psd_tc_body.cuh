@@ -457,7 +457,7 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + lay.misc_off);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + lay.misc_off + 4);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);  // uniform
     const int lane = threadIdx.x & 31;
     const int L = a.L;
     int64_t n = a.n;
@@ -823,7 +823,14 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
         }
     } else {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // The whole warp runs the loop and lane 0 issues: an MMA every 27
+        // cycles instead of 90, so a tile's A stage is free sooner (2^24 rows
+        // of length 13: 0.205 -> 0.192 ms, 34: 0.195 -> 0.191, 45: 0.197 ->
+        // 0.194).  At K = 128, whose eight steps take the tensor pipe 64
+        // cycles each, lane 0 alone: the faster issue crowds out the other
+        // CTA there (2^23 x 122: 0.239 ms against 0.262).
+        if (K < 128 || lane == 0) {
+            const uint32_t lead = lane == 0 ? 1u : 0u;
             constexpr uint32_t idesc = idesc_f16_f32(C::M, C::N);
             // B descriptor of k-step 0; later steps add to the start-address
             // field (bits 0-13, address >> 4)
@@ -850,23 +857,23 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
                 // twiddles side by side (N = 2K)
 #pragma unroll
                 for (int ks = 0; ks < C::KSTEPS; ++ks)
-                    umma_f16_ts(d, a0 + (uint32_t)(8 * ks), bdesc0 + (uint64_t)((2 * ks * C::B_KSTRIDE) >> 4), idesc,
-                                ks != 0 ? 1u : 0u);
+                    umma_f16_ts_lead(d, a0 + (uint32_t)(8 * ks), bdesc0 + (uint64_t)((2 * ks * C::B_KSTRIDE) >> 4), idesc,
+                                ks != 0 ? 1u : 0u, lead);
                 const long long c3 = tclock<TR>();
-                if constexpr (C::AS != C::NACC) umma_commit(u_a_empty + 8u * as);
-                umma_commit(u_acc_full + 8u * b);
+                if constexpr (C::AS != C::NACC) umma_commit_lead(u_a_empty + 8u * as, lead);
+                umma_commit_lead(u_acc_full + 8u * b, lead);
                 const long long c4 = tclock<TR>();
                 tr2 += c3 - c2;
                 tr3 += c4 - c3;
             }
-            if (a.trace) {
+            if (a.trace && lane == 0) {
                 atomicAdd(&a.trace[kTrMmaWaitA], tr0);
                 atomicAdd(&a.trace[kTrMmaWaitAcc], tr1);
                 atomicAdd(&a.trace[kTrMmaIssue], tr2);
                 atomicAdd(&a.trace[kTrMmaCommit], tr3);
             }
             // every MMA this thread issued is complete before TMEM is freed
-            umma_commit(final_bar);
+            umma_commit_lead(smem_u32(final_bar), lead);
             const uint64_t t0 = globaltimer_ns();
             while (!mbar_try_wait(final_bar, 0)) {
                 if (globaltimer_ns() - t0 > kWaitTimeoutNs) {
