@@ -4,7 +4,7 @@
 //
 // Device pipeline per iteration (the batch engine below):
 //   enumerate_kernel   rank windows -> row-sum-gated necklaces (packed words)
-//   psd_tc_kernel      guarded FP32 tensor-core PSD filter (+ FP64 recheck)
+//   psd_tc_kernel      guarded FP32 tensor-core PSD filter (rows near the bound stay)
 //   mask_to_list       surviving rows
 //   finalize_kernel    exact FP64 PSD, canonical check, signature records
 // The host then orders each role's records by word (the reference's FKM
@@ -185,7 +185,6 @@ int write_records_binary(gp_ctx* c, const GenPlan& p, const RecordSet& recs, con
 //   enumerate_kernel          all jobs' rank windows, one launch
 //   per job, on its own stream branch:
 //     psd_tc_kernel           row count read on the device
-//     psd_recheck_kernel      FP64 recheck of the unsure rows
 //     mask_to_list_kernel     surviving rows
 //     finalize_kernel         FP64 PSD, canonical check, records (accumulate)
 //   copy     counters -> pinned host
@@ -212,7 +211,7 @@ struct BatchCfg {
     int tc_ctas_per_sm = 0;      // tensor-core filter CTAs per SM (0 = as many as fit)
     int use_graph = 1;
     // 1: one launch per kernel and iteration over every job (filter,
-    // recheck, listing, finalize); 0: per-job launches on the jobs' own
+    // listing, finalize); 0: per-job launches on the jobs' own
     // streams
     int multi_launch = 0;
 };
@@ -222,7 +221,7 @@ struct JobRun {
     GenPlan p;
     std::vector<std::pair<gp::u128, gp::u128>> ranges;
     int64_t soft = 0, hard = 0, rcap = 0, rec_bytes = 0;
-    size_t off_words = 0, off_roles = 0, off_mask = 0, off_unsure = 0, off_idx = 0, off_rec = 0, off_units = 0;
+    size_t off_words = 0, off_roles = 0, off_mask = 0, off_idx = 0, off_rec = 0, off_units = 0;
     std::vector<int16_t> units;
     RecordSet ra, rb;
     gp_gen_stats st{};
@@ -424,7 +423,6 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
         j.off_words = take((size_t)j.hard * 16);
         j.off_roles = take((size_t)j.hard);
         j.off_mask = take((size_t)(j.hard + 31) / 32 * 4);
-        j.off_unsure = take((size_t)j.hard * 4);
         j.off_idx = take((size_t)j.hard * 4);
         j.off_rec = take((size_t)rec_region_bytes(j.rcap, j.p.L));
         j.off_units = take(j.units.size() * 2);
@@ -547,7 +545,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
         int64_t cap[gp::kMaxTcJobs];
         const unsigned long long* ndev[gp::kMaxTcJobs];
         int order[gp::kMaxTcJobs], paf[gp::kMaxTcJobs];
-        uint32_t *mask[gp::kMaxTcJobs], *unsure[gp::kMaxTcJobs];
+        uint32_t* mask[gp::kMaxTcJobs];
         unsigned long long* ucount[gp::kMaxTcJobs];
         gp::ListMultiArgs la{};
         gp::FinalizeMultiArgs fm{};
@@ -562,13 +560,12 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
             order[ji] = j.p.order;
             paf[ji] = j.p.paf;
             mask[ji] = reinterpret_cast<uint32_t*>(A + j.off_mask);
-            unsure[ji] = reinterpret_cast<uint32_t*>(A + j.off_unsure);
             ucount[ji] = it + 1;
             la.job[ji] = gp::ListJob{mask[ji], j.hard, it + 0, reinterpret_cast<uint32_t*>(A + j.off_idx), it + 2,
                                      j.hard};
             fm.job[ji] = finalize_args(ji);
         }
-        int rc = c->enqueue_filter_multi(src, cap, ndev, order, paf, mask, unsure, ucount, nj, cfg.tc_ctas_per_sm, s);
+        int rc = c->enqueue_filter_multi(src, cap, ndev, order, paf, mask, ucount, nj, cfg.tc_ctas_per_sm, s);
         if (rc) return rc;
         GP_CUDA_TRY(c, gp::launch_mask_to_list_multi(la, c->num_sms, s));
         GP_CUDA_TRY(c, gp::launch_finalize_multi(fm, cap, c->num_sms, s));
@@ -608,8 +605,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
             const gp::RowSrc src = row_src(ji);
             uint32_t* mask = reinterpret_cast<uint32_t*>(A + j.off_mask);
             uint32_t* idx = reinterpret_cast<uint32_t*>(A + j.off_idx);
-            int rc = c->enqueue_filter_dev(src, j.hard, it + 0, p.order, p.paf, mask,
-                                           reinterpret_cast<uint32_t*>(A + j.off_unsure), it + 1, cfg.tc_ctas_per_sm, sj);
+            int rc = c->enqueue_filter_dev(src, j.hard, it + 0, p.order, p.paf, mask, it + 1, cfg.tc_ctas_per_sm, sj);
             if (rc) return rc;
             GP_CUDA_TRY(c, gp::launch_mask_to_list(mask, j.hard, idx, it + 2, j.hard, c->status.as<int>(), c->num_sms,
                                                    sj, it + 0));

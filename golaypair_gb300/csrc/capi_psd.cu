@@ -67,8 +67,10 @@ int gp_ctx::enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf,
     if (!img) return fail(GP_ERR_UNSUPPORTED, "tensor-core filter: unsupported length %d", L);
     if (src.words && !gp::tc_packed_supported(L, src.pack_bits))
         return fail(GP_ERR_UNSUPPORTED, "tensor-core filter: packed length %d x %d bits", L, src.pack_bits);
-    GP_CUDA_TRY(this, cudaMemsetAsync(d_ucount, 0, sizeof(unsigned long long), st));
+    if (d_ucount) GP_CUDA_TRY(this, cudaMemsetAsync(d_ucount, 0, sizeof(unsigned long long), st));
     gp::PsdTcArgs a;
+    a.recheck = 1;
+    a.thr64 = threshold(order, paf);
     a.i8_shift = shift;
     a.seqs = src.seqs;
     a.words = src.words;
@@ -85,7 +87,6 @@ int gp_ctx::enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf,
     a.mask_words = words;
     a.unsure = d_unsure;
     a.unsure_count = d_ucount;
-    a.unsure_cap = n;
     a.psd_out = nullptr;
     a.status = status.as<int>();
     a.trace = trace_on ? counts.as<unsigned long long>() + 16 : nullptr;
@@ -93,13 +94,12 @@ int gp_ctx::enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf,
     time_begin(st, &tb);
     GP_CUDA_TRY(this, gp::launch_psd_tc(a, num_sms, st));
     time_end(st, tb);
-    GP_CUDA_TRY(this, gp::launch_psd_recheck(src, tw, threshold(order, paf), d_unsure, d_ucount, n, d_mask, num_sms, st));
     return GP_OK;
 }
 
 int gp_ctx::enqueue_filter_dev(const gp::RowSrc& src, int64_t cap, const unsigned long long* n_dev, int order,
-                               int paf, uint32_t* d_mask, uint32_t* d_unsure, unsigned long long* d_ucount,
-                               int grid_per_sm, cudaStream_t st) {
+                               int paf, uint32_t* d_mask, unsigned long long* d_ucount, int grid_per_sm,
+                               cudaStream_t st) {
     const int L = src.L;
     const double* tw = twiddle64(L);
     int shift = 0;
@@ -124,25 +124,21 @@ int gp_ctx::enqueue_filter_dev(const gp::RowSrc& src, int64_t cap, const unsigne
     a.err_coef = gp::tc_err_coef(gp::tc_k_for_len(L));
     a.mask = d_mask;
     a.mask_words = (cap + 31) / 32;
-    a.unsure = d_unsure;
+    a.unsure = nullptr;
     a.unsure_count = d_ucount;
-    a.unsure_cap = cap;
     a.psd_out = nullptr;
     a.status = status.as<int>();
     a.trace = nullptr;
     GP_CUDA_TRY(this, gp::launch_psd_tc(a, num_sms, st));
-    GP_CUDA_TRY(this, gp::launch_psd_recheck(src, tw, threshold(order, paf), d_unsure, d_ucount, cap, d_mask, num_sms, st));
     return GP_OK;
 }
 
 int gp_ctx::enqueue_filter_multi(const gp::RowSrc* src, const int64_t* cap, const unsigned long long* const* n_dev,
                                  const int* order, const int* paf, uint32_t* const* d_mask,
-                                 uint32_t* const* d_unsure, unsigned long long* const* d_ucount, int njobs,
-                                 int grid_per_sm, cudaStream_t st) {
+                                 unsigned long long* const* d_ucount, int njobs, int grid_per_sm, cudaStream_t st) {
     if (njobs < 1 || njobs > gp::kMaxTcJobs) return fail(GP_ERR_ARG, "multi-job filter: %d jobs", njobs);
     gp::PsdTcMultiArgs m{};
-    gp::RecheckMultiArgs r{};
-    m.njobs = r.njobs = njobs;
+    m.njobs = njobs;
     m.grid_per_sm = grid_per_sm;
     for (int j = 0; j < njobs; ++j) {
         const int L = src[j].L;
@@ -168,23 +164,13 @@ int gp_ctx::enqueue_filter_multi(const gp::RowSrc* src, const int64_t* cap, cons
         a.err_coef = gp::tc_err_coef(gp::tc_k_for_len(L));
         a.mask = d_mask[j];
         a.mask_words = (cap[j] + 31) / 32;
-        a.unsure = d_unsure[j];
+        a.unsure = nullptr;
         a.unsure_count = d_ucount[j];
-        a.unsure_cap = cap[j];
         a.psd_out = nullptr;
         a.status = status.as<int>();
         a.trace = nullptr;
-        gp::RecheckJob& w = r.job[j];
-        w.src = src[j];
-        w.tw = tw;
-        w.thr = threshold(order[j], paf[j]);
-        w.unsure = d_unsure[j];
-        w.unsure_count = d_ucount[j];
-        w.cap = cap[j];
-        w.mask = d_mask[j];
     }
     GP_CUDA_TRY(this, gp::launch_psd_tc_multi(m, num_sms, st));
-    GP_CUDA_TRY(this, gp::launch_psd_recheck_multi(r, num_sms, st));
     return GP_OK;
 }
 
@@ -486,8 +472,9 @@ int gp_psd_filter_device(gp_ctx* c, const int8_t* d_seqs, int64_t n, int L, int 
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->s_comp;
     if (mode == GP_PSD_TC_GUARDED && !c->unsure_buf[0].ensure((size_t)std::max<int64_t>(n, 1) * 4))
         return c->fail(GP_ERR_NOMEM, "psd filter: device allocation failed");
+    // without stats nothing is counted: the call is one launch
     rc = c->enqueue_filter(int8_src(d_seqs, L), n, order, paf, mode, d_mask, c->unsure_buf[0].as<uint32_t>(),
-                           c->counts.as<unsigned long long>(), st);
+                           stats ? c->counts.as<unsigned long long>() : nullptr, st);
     if (rc) return rc;
     if (stats) {
         GP_CUDA_TRY(c, cudaStreamSynchronize(st));
@@ -557,7 +544,6 @@ int gp_psd_tc_values(gp_ctx* c, const int8_t* seqs, int64_t n, int L, float* out
     a.mask_words = (n + 31) / 32;
     a.unsure = du.as<uint32_t>();
     a.unsure_count = c->counts.as<unsigned long long>();
-    a.unsure_cap = n;
     a.psd_out = dp.as<float>();
     a.status = c->status.as<int>();
     a.trace = nullptr;

@@ -166,25 +166,25 @@ struct gp_ctx {
     // loads when int8_rows and the length takes them (*shift set to 1)
     // (both halves of the twiddles for the PSD values, the filter's otherwise)
     const void* twiddle_image(int L, bool int8_rows = false, int* shift = nullptr, bool both = false);
-    // Multi-job tensor-core filter of device batches (packed words) followed
-    // by the FP64 recheck of every job's unsure rows: two launches on st for
-    // up to eight jobs, each job's tiles at its own padded K.  Per job as
-    // enqueue_filter_dev; unsure counts must be zero.
+    // Multi-job tensor-core filter of device batches (packed words): one
+    // launch on st for up to eight jobs, each job's tiles at its own padded
+    // K.  Per job as enqueue_filter_dev.
     int enqueue_filter_multi(const gp::RowSrc* src, const int64_t* cap, const unsigned long long* const* n_dev,
-                             const int* order, const int* paf, uint32_t* const* d_mask, uint32_t* const* d_unsure,
+                             const int* order, const int* paf, uint32_t* const* d_mask,
                              unsigned long long* const* d_ucount, int njobs, int grid_per_sm, cudaStream_t st);
     // device FP64 twiddle table for length L
     const double* twiddle64(int L);
     // Enqueues the PSD filter of a device batch (int8 rows or packed words)
-    // on st: mask bit = pass; TC mode rechecks its unsure rows in FP64.
+    // on st: mask bit = pass; TC mode rechecks its unsure rows in FP64 and
+    // counts them in *d_ucount unless it is null.
     int enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf, int mode, uint32_t* d_mask,
                        uint32_t* d_unsure, unsigned long long* d_ucount, cudaStream_t st);
     // TC-mode filter of a device batch whose row count is read on the device
     // (*n_dev, at most cap rows): nothing here depends on the count, so the
-    // sequence can be captured in a CUDA graph.  *d_ucount must be zero.
+    // launch can be captured in a CUDA graph.  Unsure rows keep their mask
+    // bits (the finalize kernel filters exactly); *d_ucount += their count.
     int enqueue_filter_dev(const gp::RowSrc& src, int64_t cap, const unsigned long long* n_dev, int order, int paf,
-                           uint32_t* d_mask, uint32_t* d_unsure, unsigned long long* d_ucount, int grid_per_sm,
-                           cudaStream_t st);
+                           uint32_t* d_mask, unsigned long long* d_ucount, int grid_per_sm, cudaStream_t st);
     // reads the kernel status word; resets it; returns a GP code
     int check_status(const char* what);
 };

@@ -33,9 +33,14 @@ struct PsdTcArgs {
     float err_coef;          // per-row |X| error bound = S_row * err_coef
     uint32_t* mask;          // ceil(n/32) words; bit = sure pass or unsure
     int64_t mask_words;
-    uint32_t* unsure;        // indices of unsure candidates (chunk-local)
-    unsigned long long* unsure_count;
-    int64_t unsure_cap;
+    // Unsure rows (near the bound): with recheck, the CTA that found them
+    // decides them in FP64 against thr64 before it ends, from its own part of
+    // `unsure` (n entries: the p-th of a CTA at the place of its p-th row);
+    // without, their mask bits stay set for a caller that filters exactly.
+    int recheck = 0;
+    double thr64;
+    uint32_t* unsure;
+    unsigned long long* unsure_count;  // optional: += unsure rows
     float* psd_out;          // optional n x (K/2) PSD values
     // int8 rows: 1 = each row is read from the 4-byte boundary at or below
     // its first byte and sits s = (row * L) mod 4 columns along A, the bytes
@@ -146,28 +151,6 @@ struct PsdF64Args {
     int num_sms;
 };
 cudaError_t launch_psd_fp64(const PsdF64Args& a, cudaStream_t st);
-
-// FP64 recheck of the unsure list (one warp per row): clears the mask bit of
-// every unsure candidate that fails the exact filter.
-cudaError_t launch_psd_recheck(const RowSrc& src, const double* tw, double thr, const uint32_t* unsure,
-                               const unsigned long long* unsure_count, int64_t cap, uint32_t* mask,
-                               int num_sms, cudaStream_t st);
-
-// The same recheck for several jobs in one launch (one grid row per job).
-struct RecheckJob {
-    RowSrc src;
-    const double* tw;
-    double thr;
-    const uint32_t* unsure;
-    const unsigned long long* unsure_count;
-    int64_t cap;
-    uint32_t* mask;
-};
-struct RecheckMultiArgs {
-    RecheckJob job[8];
-    int njobs;
-};
-cudaError_t launch_psd_recheck_multi(const RecheckMultiArgs& a, int num_sms, cudaStream_t st);
 
 // Exact FP64 PSD values (all L bins) of rows 0..n-1 (testing)
 cudaError_t launch_psd_fp64_values(const RowSrc& src, const double* tw, int64_t n, double* out, cudaStream_t st);

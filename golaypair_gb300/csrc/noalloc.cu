@@ -5,8 +5,8 @@
 // framework's memory pool or allocator hooks, inside a real-time loop that
 // forbids allocator calls, or on a device whose memory is fully reserved by
 // its owner.  This entry point runs the same kernels as gp_psd_filter_device
-// (psd_tc_kernel, then the FP64 recheck) but takes every working buffer it
-// needs -- the unsure-row list and its counter, the kernel status word, the
+// (psd_tc_kernel with its FP64 recheck) but takes every working buffer it
+// needs -- the unsure-row list, the kernel status word, the
 // tensor-core twiddle image and the FP64 twiddle table -- from one fixed
 // array in static device memory, g_noalloc_scratch, instead of allocating.
 //
@@ -21,7 +21,7 @@
 //     A device reset (cudaDeviceReset) invalidates the kept address: do not
 //     call the entry point on that device again in the same process.
 //   * Every call shares the array and it keeps the last call's contents;
-//     the call clears the counter and status words it relies on.  Calls that
+//     the call clears the status word it relies on.  Calls that
 //     overlap on the GPU (other streams, other threads) race on it.
 //   * The call is synchronous: it reads the kernel status word on its own
 //     stream and waits for that stream (a timed-out device wait returns
@@ -43,8 +43,7 @@ constexpr size_t kImageBytes = (size_t)kMaxTcK * kMaxTcK * 2;  // hi twiddles at
 constexpr size_t kTw64Bytes = 2 * (size_t)kMaxTcK * sizeof(double);
 // layout of the scratch array (byte offsets, 256-aligned)
 constexpr size_t kOffStatus = 0;                            // int status
-constexpr size_t kOffCounter = 256;                         // unsigned long long unsure count
-constexpr size_t kOffImage = 512;                           // tensor-core twiddle image
+constexpr size_t kOffImage = 256;                           // tensor-core twiddle image
 constexpr size_t kOffTw64 = kOffImage + kImageBytes;        // FP64 twiddle table
 constexpr size_t kOffUnsure = kOffTw64 + kTw64Bytes;        // uint32 unsure rows
 constexpr size_t kNoAllocScratchBytes = kOffUnsure + (size_t)kNoAllocMaxRows * 4;
@@ -130,8 +129,8 @@ extern "C" int gp_psd_filter_noalloc(const int8_t* d_seqs, int64_t n, int L, int
     int rc = setup_device(dev, &s, &sms);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // clear what the kernels count from zero; the rest is overwritten
-    if (cudaMemsetAsync(s + kOffStatus, 0, 512, st) != cudaSuccess) return GP_ERR_CUDA;
+    // clear the status word; the rest is overwritten
+    if (cudaMemsetAsync(s + kOffStatus, 0, sizeof(int), st) != cudaSuccess) return GP_ERR_CUDA;
     noalloc_twiddles_kernel<<<64, 256, 0, st>>>(s, L, K, tc_image_halves(K), tc_i8_wrap_rows(L));
     if (cudaGetLastError() != cudaSuccess) return GP_ERR_CUDA;
     const double thr = 2.0 * order - paf + 0.001;
@@ -151,16 +150,13 @@ extern "C" int gp_psd_filter_noalloc(const int8_t* d_seqs, int64_t n, int L, int
     a.mask = d_pass_mask;
     a.mask_words = (n + 31) / 32;
     a.unsure = reinterpret_cast<uint32_t*>(s + kOffUnsure);
-    a.unsure_count = reinterpret_cast<unsigned long long*>(s + kOffCounter);
-    a.unsure_cap = n;
+    a.unsure_count = nullptr;
+    a.recheck = 1;
+    a.thr64 = thr;
     a.psd_out = nullptr;
     a.status = reinterpret_cast<int*>(s + kOffStatus);
     a.trace = nullptr;
     if (launch_psd_tc(a, sms, st) != cudaSuccess) return GP_ERR_CUDA;
-    RowSrc src{d_seqs, nullptr, L, 0, 0};
-    if (launch_psd_recheck(src, reinterpret_cast<const double*>(s + kOffTw64), thr, a.unsure, a.unsure_count, n,
-                           d_pass_mask, sms, st) != cudaSuccess)
-        return GP_ERR_CUDA;
     // the status word is read on the caller's stream: nothing here waits on
     // other streams of the device
     int status = 0;

@@ -35,7 +35,7 @@
 // Each candidate is classified against T = 2n - paf + 0.001 with a guard g
 // (the configured band, widened per row to a rigorous bound on the fp32
 // error): max p < T - g -> pass, max p > T + g -> reject, else "unsure",
-// appended to a list that an FP64 kernel rechecks exactly.  The pass mask
+// kept in a list that the CTA rechecks in FP64 at its end.  The pass mask
 // bit is set for pass and unsure; the recheck clears the failing unsure ones.
 //
 // Two input forms:

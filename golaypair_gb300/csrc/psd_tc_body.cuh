@@ -53,6 +53,9 @@ struct TcCfg {
     static_assert(NACC * N + AS * K / 2 <= TMEM_COLS, "TMEM budget");
 };
 
+// the FP64 recheck's tables take the place of the raw ring
+constexpr uint32_t kRecheckSmem = (kMaxTcK + (kThreads / 32) * ((kMaxTcK - 1) / 2 + 1)) * 16;
+
 struct SmemLayout {
     uint32_t b_off, lut_off, tw_off, raw_off, raw_stride, raw_stages, bar_off, misc_off, total;
 };
@@ -85,6 +88,7 @@ SmemLayout smem_layout(int row_bytes) {
     s.total = off + 1024;  // slack for the 1024-byte alignment of the base
     // At most two CTAs per SM: each holds 256 TMEM columns (512 per SM).
     if (s.total < 96 * 1024) s.total = 96 * 1024;
+    if (s.total < s.raw_off + kRecheckSmem + 1024) s.total = s.raw_off + kRecheckSmem + 1024;
     return s;
 }
 
@@ -390,6 +394,79 @@ __device__ __noinline__ float2 near_rows(const PsdTcArgs& a, const float2* s_tw,
     return mine;
 }
 
+// The CTA's unsure rows in FP64, once its tiles are done (raw ring free): the
+// reference's filter on the folded sums x_j +- x_{L-j}; a failing row's mask
+// bit is cleared.  Each row takes the smallest power-of-two group of lanes
+// that holds its bins (a whole warp from 17 bins on), so a warp has several
+// short rows in hand.  The filter is one launch, without the list counter's
+// memset and a recheck kernel: 2^12 rows of length 45 take 5.6 us (10.8 with
+// three), 2^20 rows 20.5 us (28.8), 2^26 rows of length 8, of which 4 % lie at
+// the bound, 1.02 ms (5.77: one atomic on one counter per warp, one warp per row).
+constexpr int kFoldEntries = (kMaxTcK - 1) / 2 + 1;
+template <int B>
+__device__ __noinline__ void recheck_own(const PsdTcArgs& a, uint8_t* smem, int cnt, int first, int stride) {
+    const int L = a.L, H = L / 2, J = (L - 1) / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double2* tw = reinterpret_cast<double2*>(smem);
+    double2* fold = tw + kMaxTcK + warp * kFoldEntries;
+    for (int m = threadIdx.x; m < L; m += blockDim.x) tw[m] = make_double2(a.tw64[2 * m], a.tw64[2 * m + 1]);
+    __syncthreads();
+    int G = 1;
+    while (G < H && G < 32) G <<= 1;
+    const int R = 32 / G, sub = lane / G, l = lane & (G - 1);
+    fold += sub * J;  // R J <= 32 when a row has no more bins than lanes
+    for (int i0 = warp * R; i0 < cnt; i0 += (kThreads / 32) * R) {
+        const int i = i0 + sub;
+        const bool has = i < cnt;
+        uint32_t row = 0;
+        uint64_t lo = 0, hi = 0;
+        if (has) {
+            row = a.unsure[(int64_t)(first + (i >> 7) * stride) * kTileM + (i & 127)];
+            if constexpr (B != 0) {
+                const uint4 w = a.words[row];
+                lo = ((uint64_t)w.y << 32) | w.x;
+                hi = ((uint64_t)w.w << 32) | w.z;
+            }
+        }
+        auto value = [&](int j) -> int {
+            if constexpr (B == 0)
+                return a.seqs[(int64_t)row * L + j];
+            else
+                return 2 * word_digit(lo, hi, B, L, j) - a.alpha_c;
+        };
+        __syncwarp();
+        int x0 = 0, xm = 0;
+        if (has) {
+            x0 = value(0);
+            if (!(L & 1)) xm = value(H);
+            for (int j = 1 + l; j <= J; j += G) {
+                const int p = value(j), q = value(L - j);
+                fold[j - 1] = make_double2((double)(p + q), (double)(p - q));
+            }
+        }
+        __syncwarp();
+        bool fail = false;
+        if (has) {
+            for (int k = 1 + l; k <= H; k += G) {
+                double re = (double)(x0 + ((k & 1) ? -xm : xm)), im = 0.0;
+                int m = 0;
+#pragma unroll 4
+                for (int j = 0; j < J; ++j) {
+                    m += k;
+                    if (m >= L) m -= L;
+                    const double2 eo = fold[j], w = tw[m];
+                    re = fma(eo.x, w.x, re);
+                    im = fma(eo.y, w.y, im);
+                }
+                fail = fail || re * re + im * im > a.thr64;
+            }
+        }
+        const uint32_t f = __ballot_sync(0xFFFFFFFFu, fail) >> (sub * G);
+        if (has && l == 0 && (G == 32 ? f : f & ((1u << G) - 1u)) != 0)
+            atomicAnd(&a.mask[row >> 5], ~(1u << (row & 31)));
+    }
+}
+
 // A row of a tile that is not whole or not bulk-copied (the last tile, or
 // an input not 16-byte aligned): byte loads from global memory, zeros past
 // row n or column L, stored as the A row at TMEM address aaddr.  Out of line: it runs at most once per CTA on aligned
@@ -456,6 +533,7 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
     const uint32_t u_acc_full = smem_u32(acc_full), u_acc_empty = smem_u32(acc_empty);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + lay.misc_off);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + lay.misc_off + 4);
+    int* n_unsure = reinterpret_cast<int*>(smem + lay.misc_off + 8);  // of this CTA
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);  // uniform
     const int lane = threadIdx.x & 31;
@@ -491,6 +569,7 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
         mbar_init(b_full, 1);
         mbar_init(final_bar, 1);
         *abort_flag = 0;
+        *n_unsure = 0;
         mbar_fence_init();
     }
     if constexpr (B != 0) build_lut(sLut, B, a.alpha_c);
@@ -744,15 +823,12 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
             if (lane == 0 && word < mask_words) a.mask[word] = bits;
             const uint32_t ub = __ballot_sync(0xFFFFFFFFu, unsure);
             if (ub) {
-                unsigned long long basei = 0;
-                if (lane == 0) basei = atomicAdd(a.unsure_count, (unsigned long long)__popc(ub));
-                basei = __shfl_sync(0xFFFFFFFFu, basei, 0);
-                if (unsure) {
-                    const unsigned long long pos = basei + __popc(ub & ((1u << lane) - 1u));
-                    if ((int64_t)pos < a.unsure_cap)
-                        a.unsure[pos] = (uint32_t)row;
-                    else
-                        atomicCAS(a.status, 0, GP_KSTATUS_OVERFLOW);
+                int base = 0;
+                if (lane == 0) base = atomicAdd(n_unsure, __popc(ub));
+                if (!WRITE_PSD && a.recheck) {
+                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                    const int pos = base + __popc(ub & ((1u << lane) - 1u));
+                    if (unsure) a.unsure[(int64_t)(first + (pos >> 7) * stride) * kTileM + (pos & 127)] = (uint32_t)row;
                 }
             }
             const long long c_end = tclock<TR>();
@@ -889,6 +965,11 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
         tc_fence_after();
         tmem_dealloc(tmem_base, C::TMEM_COLS);
     }
+    const int cnt = *n_unsure;
+    if (cnt == 0) return;
+    if (threadIdx.x == 0 && a.unsure_count) atomicAdd(a.unsure_count, (unsigned long long)cnt);
+    if constexpr (!WRITE_PSD)
+        if (a.recheck && !*abort_flag) recheck_own<B>(a, sRaw, cnt, first, stride);
 }
 
 }  // namespace
