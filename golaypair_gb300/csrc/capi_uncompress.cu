@@ -965,50 +965,92 @@ int build_level(gp_ctx* c, Level& lv, int order, int compress, int new_compress,
     return GP_OK;
 }
 
-// Device copies of a level's tables (context scratch ux[0..3]).
+// The terms C_i(d, k) of every position, row, choice and varying bin, one per
+// thread: sum_q v_q (cos, -sin)(2 pi (i + L q) k / L').  The cosines and sines
+// come as double pairs hi + lo and the sum is kept as one, so the FP64 table
+// is rounded once.  (They were made on the host: 8.7 of the 163 ms of 4,000
+// order-57 pairs and 4.0 of the 7.1 ms of 200 order-39 pairs, on a machine
+// whose long double is software; here 0.1 ms.)
+struct TablesArgs {
+    int L, r, Lnew, nrows, dmax, nb, np;
+    const int* cnt;         // [nrows]
+    const int8_t* vals;     // [nrows][dmax][r]
+    const int* bins;        // [nb]
+    const double2* cos2;    // [Lnew] (hi, lo)
+    const double2* sin2;    // [Lnew]
+    float4* ctab;           // [L][nrows][dmax][np]
+    double2* ctab64;        // [L][nrows][dmax][2 np]
+};
+
+// (hi, lo) += v * t
+__device__ __forceinline__ void add_pair(double& hi, double& lo, int v, double2 t) {
+    const double x = (double)v * t.x;  // |v| < 2^7: its rounding error goes to lo
+    const double ex = fma((double)v, t.x, -x);
+    const double s = hi + x, bb = s - hi;
+    lo += ((hi - (s - bb)) + (x - bb)) + fma((double)v, t.y, ex);
+    hi = s;
+}
+
+__global__ void __launch_bounds__(256) ux_tables_kernel(TablesArgs a) {
+    const int NB = 2 * a.np;
+    const int64_t n = (int64_t)a.L * a.nrows * a.dmax * NB;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+        const int b = (int)(e % NB);
+        const int64_t at = e / NB;  // (position, row, choice)
+        const int d = (int)(at % a.dmax), row = (int)(at / a.dmax % a.nrows), i = (int)(at / a.dmax / a.nrows);
+        double re = 0.0, rl = 0.0, im = 0.0, il = 0.0;
+        if (b < a.nb && d < a.cnt[row]) {
+            const int k = a.bins[b];
+            const int8_t* v = a.vals + ((size_t)row * a.dmax + d) * a.r;
+            for (int q = 0; q < a.r; ++q) {
+                const int m = (int)(((long long)(i + a.L * q) * k) % a.Lnew);
+                add_pair(re, rl, v[q], a.cos2[m]);
+                add_pair(im, il, -v[q], a.sin2[m]);
+            }
+        }
+        const double2 t = make_double2(re + rl, im + il);
+        a.ctab64[e] = t;
+        float* f = reinterpret_cast<float*>(a.ctab + at * a.np + b / 2);
+        f[b & 1] = (float)t.x;
+        f[2 + (b & 1)] = (float)t.y;
+    }
+}
+
+// A level's tables on the device (context scratch ux[0..3] and ux[34..36]).
 int upload_level(gp_ctx* c, const Level& lv, LevelDev& d, cudaStream_t s) {
     const int np = lv.np, NB = 2 * np;
     std::vector<int> cnt(lv.nrows);
     std::vector<int8_t> vals((size_t)lv.nrows * lv.dmax * lv.r, 0);
-    std::vector<float4> ct((size_t)lv.L * lv.nrows * lv.dmax * np, make_float4(0.f, 0.f, 0.f, 0.f));
-    std::vector<double2> ct64((size_t)lv.L * lv.nrows * lv.dmax * NB, make_double2(0.0, 0.0));
     for (int row = 0; row < lv.nrows; ++row) {
         cnt[row] = (int)lv.rowparts[row].size();
         for (int d = 0; d < cnt[row]; ++d)
             for (int q = 0; q < lv.r; ++q) vals[((size_t)row * lv.dmax + d) * lv.r + q] = (int8_t)lv.rowparts[row][d][q];
     }
-    for (int i = 0; i < lv.L; ++i)
-        for (int row = 0; row < lv.nrows; ++row)
-            for (int d = 0; d < cnt[row]; ++d) {
-                const size_t at = ((size_t)i * lv.nrows + row) * lv.dmax + d;
-                for (int b = 0; b < lv.nb; ++b) {
-                    const int k = lv.bins[b];
-                    long double re = 0, im = 0;
-                    for (int q = 0; q < lv.r; ++q) {
-                        const int m = (int)(((long long)(i + lv.L * q) * k) % lv.Lnew);
-                        const long double ang = 6.283185307179586476925286766559L * (long double)m / (long double)lv.Lnew;
-                        re += (long double)lv.rowparts[row][d][q] * cosl(ang);
-                        im -= (long double)lv.rowparts[row][d][q] * sinl(ang);
-                    }
-                    ct64[at * NB + b] = make_double2((double)re, (double)im);
-                    float4& f = ct[at * np + b / 2];
-                    if (b & 1) {
-                        f.y = (float)re;
-                        f.w = (float)im;
-                    } else {
-                        f.x = (float)re;
-                        f.z = (float)im;
-                    }
-                }
-            }
-    DevBuf &dcnt = c->ux[0], &dvals = c->ux[1], &dct = c->ux[2], &dct64 = c->ux[3];
-    if (!dcnt.ensure(cnt.size() * 4) || !dvals.ensure(vals.size() + 16) || !dct.ensure(ct.size() * 16) ||
-        !dct64.ensure(ct64.size() * 16))
+    std::vector<double2> tw(2 * (size_t)lv.Lnew);  // cosines, then sines, as (hi, lo)
+    for (int m = 0; m < lv.Lnew; ++m) {
+        const long double ang = 6.283185307179586476925286766559L * (long double)m / (long double)lv.Lnew;
+        const long double w[2] = {cosl(ang), sinl(ang)};
+        for (int t = 0; t < 2; ++t) {
+            const double hi = (double)w[t];
+            tw[t * (size_t)lv.Lnew + m] = make_double2(hi, (double)(w[t] - (long double)hi));
+        }
+    }
+    const size_t terms = (size_t)lv.L * lv.nrows * lv.dmax;
+    DevBuf &dcnt = c->ux[0], &dvals = c->ux[1], &dct = c->ux[2], &dct64 = c->ux[3], &dbins = c->ux[34],
+           &dtw = c->ux[35];
+    if (!dcnt.ensure(cnt.size() * 4) || !dvals.ensure(vals.size() + 16) || !dct.ensure(terms * np * 16) ||
+        !dct64.ensure(terms * NB * 16) || !dbins.ensure((size_t)lv.nb * 4 + 4) || !dtw.ensure(tw.size() * 16))
         return c->fail(GP_ERR_NOMEM, "uncompress: level tables");
     GP_CUDA_TRY(c, cudaMemcpyAsync(dcnt.p, cnt.data(), cnt.size() * 4, cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(dvals.p, vals.data(), vals.size(), cudaMemcpyHostToDevice, s));
-    GP_CUDA_TRY(c, cudaMemcpyAsync(dct.p, ct.data(), ct.size() * 16, cudaMemcpyHostToDevice, s));
-    GP_CUDA_TRY(c, cudaMemcpyAsync(dct64.p, ct64.data(), ct64.size() * 16, cudaMemcpyHostToDevice, s));
+    GP_CUDA_TRY(c, cudaMemcpyAsync(dbins.p, lv.bins.data(), lv.bins.size() * 4, cudaMemcpyHostToDevice, s));
+    GP_CUDA_TRY(c, cudaMemcpyAsync(dtw.p, tw.data(), tw.size() * 16, cudaMemcpyHostToDevice, s));
+    TablesArgs ta{lv.L, lv.r, lv.Lnew, lv.nrows, lv.dmax, lv.nb, np, dcnt.as<int>(), dvals.as<int8_t>(),
+                  dbins.as<int>(), dtw.as<double2>(), dtw.as<double2>() + lv.Lnew, dct.as<float4>(),
+                  dct64.as<double2>()};
+    const int64_t work = (int64_t)terms * NB;
+    ux_tables_kernel<<<(unsigned)std::min<int64_t>((work + 255) / 256, (int64_t)c->num_sms * 8), 256, 0, s>>>(ta);
+    GP_CUDA_TRY(c, cudaGetLastError());
     GP_CUDA_TRY(c, cudaStreamSynchronize(s));  // the host vectors go out of scope
     d.L = lv.L;
     d.r = lv.r;
