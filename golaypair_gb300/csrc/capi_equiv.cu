@@ -17,7 +17,8 @@
 // applies every element of the closure with the reference's application
 // rule (equivalence.cpp:97-144), hashing the images of several pairs per
 // pass over the transposed table and looking them up in a hash set of the
-// input pairs.  Either way the host then replays the reference's in-order
+// input pairs.  The pairs' text is read and written, and the pairs and least
+// images sorted, on the device too.  Either way the host then replays the reference's in-order
 // erase loop (filter.cpp:117-144) on those class sizes and member lists.
 #include <algorithm>
 #include <chrono>
@@ -31,6 +32,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "prims.h"
 
 namespace {
 
@@ -308,6 +310,169 @@ __global__ void __launch_bounds__(kCanonThreads) canon_kernel(CanonArgs a) {
     }
 }
 
+// ------------------------------------------------------------ pair text
+// The pair file is parsed, its pairs sorted and the kept ones written as text
+// on the device: on the host that took 57 of the 73 ms of 30,000 order-57
+// pairs (strtol, a vector per pair, std::sort, one digit at a time), here
+// about 1 ms beside the file itself.
+
+// What the text holds beside its values.
+struct TextInfo {
+    uint32_t bad;         // something strtol would read differently: the host parses
+    uint32_t present[8];  // bit v + 128: value v occurs
+};
+
+constexpr int kParseThreads = 256;
+constexpr int kParseEach = 16;                              // bytes per thread
+constexpr int kParseBlock = kParseThreads * kParseEach;     // the text is padded with blanks to a multiple
+
+__device__ __forceinline__ bool is_blank(int c) { return c == ' ' || (c >= '\t' && c <= '\r'); }
+__device__ __forceinline__ bool is_digit(int c) { return c >= '0' && c <= '9'; }
+
+// Values are runs of an optional '-' and one to three digits, at most 127,
+// between blanks.  WRITE = false counts a block's values, true stores them
+// from the block's offset.
+template <bool WRITE>
+__global__ void __launch_bounds__(kParseThreads) pair_values_kernel(const char* text, uint32_t* counts,
+                                                                    const uint32_t* offs, int8_t* vals,
+                                                                    TextInfo* info) {
+    __shared__ uint32_t s_warp[kParseThreads / 32];
+    __shared__ uint32_t s_present[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (WRITE && threadIdx.x < 8) s_present[threadIdx.x] = 0;
+    const int64_t p0 = (int64_t)blockIdx.x * kParseBlock + threadIdx.x * kParseEach;
+    const uint4 w = *reinterpret_cast<const uint4*>(text + p0);
+    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+    int prev = p0 ? text[p0 - 1] : ' ';
+    const int after = text[p0 + kParseEach];  // the buffer has a block of blanks past the text
+    uint32_t starts = 0;
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < kParseEach; ++k) {
+        const int c = (ww[k >> 2] >> (8 * (k & 3))) & 0xFF;
+        const int next = k + 1 < kParseEach ? (ww[(k + 1) >> 2] >> (8 * ((k + 1) & 3))) & 0xFF : after;
+        const bool minus = c == '-';
+        if ((is_digit(c) || minus) && is_blank(prev)) starts |= 1u << k;
+        if (!is_digit(c) && !minus && !is_blank(c)) bad = true;
+        if (minus && (!is_blank(prev) || !is_digit(next))) bad = true;
+        prev = c;
+    }
+    const uint32_t mine = (uint32_t)__popc(starts);
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (int q = 0; q < kParseThreads / 32; ++q) {
+        if (q < warp) before += s_warp[q];
+        total += s_warp[q];
+    }
+    if constexpr (!WRITE) {
+        if (threadIdx.x == 0) counts[blockIdx.x] = total;
+        if (bad) info->bad = 1;
+    } else {
+        int8_t* out = vals + offs[blockIdx.x] + before + incl - mine;
+        for (uint32_t m = starts; m; m &= m - 1u) {
+            const char* q = text + p0 + __ffs((int)m) - 1;
+            const bool neg = *q == '-';
+            q += neg ? 1 : 0;
+            int v = 0, n = 0;
+            for (; is_digit(*q) && n < 4; ++q, ++n) v = v * 10 + (*q - '0');
+            if (n > 3 || v > 127) info->bad = 1;
+            v = neg ? -v : v;
+            *out++ = (int8_t)v;
+            atomicOr(&s_present[((v + 128) & 255) >> 5], 1u << (v & 31));
+        }
+        __syncthreads();
+        if (threadIdx.x < 8 && s_present[threadIdx.x]) atomicOr(&info->present[threadIdx.x], s_present[threadIdx.x]);
+    }
+}
+
+// Sort keys of rows of W values: the values' ranks (code[(uint8_t)v], in the
+// order of the values) in b bits each, 32 / b to a word, first value highest.
+__global__ void pair_keys_kernel(const int8_t* rows, int64_t n, int W, const uint8_t* code, int b, int Wk,
+                                 uint32_t* keys) {
+    const int per = 32 / b;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * Wk; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = e / Wk;
+        const int o0 = (int)(e - i * Wk) * per;
+        uint32_t k = 0;
+        for (int q = 0; q < per; ++q) {
+            const int o = o0 + q;
+            k = (k << b) | (o < W ? (uint32_t)code[(uint8_t)rows[i * W + o]] : 0u);
+        }
+        keys[e] = k;
+    }
+}
+
+__global__ void gather_rows_kernel(const int8_t* rows, const uint32_t* idx, int64_t n, int W, int8_t* out) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * W; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = e / W;
+        out[e] = rows[(int64_t)idx[i] * W + (e - i * W)];
+    }
+}
+
+// Bytes of "%d ".
+__device__ __forceinline__ int value_bytes(int v) {
+    const int u = v < 0 ? -v : v;
+    return (v < 0 ? 1 : 0) + (u >= 100 ? 3 : u >= 10 ? 2 : 1) + 1;
+}
+
+// Bytes of each kept pair's line (0: left out): "%d " per entry of a, " ",
+// "%d " per entry of b, newline.
+__global__ void pair_line_bytes_kernel(const int8_t* rows, const uint8_t* alive, int64_t n, int W, uint32_t* bytes) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        uint32_t b = 0;
+        if (alive[i]) {
+            b = 2;
+            for (int o = 0; o < W; ++o) b += (uint32_t)value_bytes(rows[i * W + o]);
+        }
+        bytes[i] = b;
+    }
+}
+
+// The lines: a warp per pair, 32 entries at a time.
+__global__ void __launch_bounds__(256) pair_lines_kernel(const int8_t* rows, const uint8_t* alive, int64_t n, int W,
+                                                         const uint32_t* at, char* text) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+        if (!alive[i]) continue;
+        char* line = text + at[i];
+        for (int o0 = 0; o0 < W; o0 += 32) {
+            const int o = o0 + lane;
+            const int v = o < W ? rows[i * W + o] : 0;
+            // the blank between the halves before entry L, the newline after the last
+            int mine = o < W ? value_bytes(v) + (o == W / 2 ? 1 : 0) + (o == W - 1 ? 1 : 0) : 0;
+            int incl = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if (lane >= d) incl += y;
+            }
+            if (o < W) {
+                char* q = line + incl - mine;
+                if (o == W / 2) *q++ = ' ';
+                int u = v;
+                if (v < 0) {
+                    *q++ = '-';
+                    u = -v;
+                }
+                if (u >= 100) *q++ = (char)('0' + u / 100);
+                if (u >= 10) *q++ = (char)('0' + u / 10 % 10);
+                *q++ = (char)('0' + u % 10);
+                *q++ = ' ';
+                if (o == W - 1) *q = '\n';
+            }
+            line += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        }
+    }
+}
+
 std::vector<int16_t> all_units(int L) {
     std::vector<int16_t> u;
     for (int v = 1; v < L; ++v)
@@ -509,28 +674,157 @@ std::vector<int16_t> as_sources(const int16_t* item, int L) {
 
 uint64_t pair_group_size(int L, int compress);
 
-// Class sizes and members of the pairs P (sorted, distinct) by canonical
-// forms on the device (canon_kernel): member_list[span[i].first ..
-// span[i].second) are the pairs with the same least image as pair i (itself
-// included), csize[i] is the group order over the number of elements fixing
-// pair i.  L >= 3.
-int canonical_classes(gp_ctx* c, int L, int compress, const std::vector<std::vector<int8_t>>& P,
-                      std::vector<unsigned long long>& csize, std::vector<uint32_t>& member_list,
-                      std::vector<std::pair<uint32_t, uint32_t>>& span) {
+unsigned grid_of(int64_t n, int block) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + block - 1) / block, 1 << 16));
+}
+
+// The pair file's values as strtol reads them one after the other: whitespace-
+// separated integers up to the first token that is not one.
+std::vector<int8_t> host_values(const char* text) {
+    std::vector<int8_t> vals;
+    for (const char* q = text;;) {
+        char* e;
+        const long v = strtol(q, &e, 10);
+        if (e == q) break;
+        q = e;
+        vals.push_back((int8_t)v);
+    }
+    return vals;
+}
+
+// A pair set on the device: distinct pairs in order, and what sorting rows of
+// their values takes.  Buffers eq[..] of the context.
+struct PairSet {
+    gp_ctx* c;
+    int W;
+    int64_t np = 0;       // distinct pairs
+    int8_t* rows = nullptr;
+    int bits = 1, Wk = 1; // key layout
+    const uint8_t* code = nullptr;
+};
+
+enum EqBuf { kEqText, kEqCount, kEqOffs, kEqScan, kEqVals, kEqInfo, kEqCode, kEqKeys, kEqIdx, kEqTmp, kEqFlag, kEqPos,
+             kEqOut, kEqRows, kEqCanon, kEqUnits, kEqFix, kEqAlive, kEqBytes, kEqLine };
+
+// Sorts n rows: idx (device) in the rows' order, equal rows in index order,
+// flags[k] = 1 where the k-th row differs from the one before.
+int sort_rows(PairSet& ps, const int8_t* rows, int64_t n, uint32_t* idx, uint32_t* flags, cudaStream_t s) {
+    gp_ctx* c = ps.c;
+    DevBuf &keys = c->eq[kEqKeys], &tmp = c->eq[kEqTmp];
+    if (!keys.ensure((size_t)n * ps.Wk * 4) || !tmp.ensure(gp::radix_sort_tmp_bytes(n)))
+        return c->fail(GP_ERR_NOMEM, "equivalence filter: sort buffers");
+    pair_keys_kernel<<<grid_of(n * ps.Wk, 256), 256, 0, s>>>(rows, n, ps.W, ps.code, ps.bits, ps.Wk,
+                                                             keys.as<uint32_t>());
+    GP_CUDA_TRY(c, cudaGetLastError());
+    GP_CUDA_TRY(c, gp::iota_u32(idx, n, s));
+    GP_CUDA_TRY(c, gp::radix_sort_keys(keys.as<uint32_t>(), ps.Wk, ps.Wk, idx, n, tmp.p, s, 8));
+    GP_CUDA_TRY(c, gp::mark_unique(keys.as<uint32_t>(), ps.Wk, idx, n, ps.Wk, flags, s));
+    return GP_OK;
+}
+
+// filter.cpp:45-62: L values for a, then (if the stream is still good) L for
+// b: whitespace-separated integers up to the first token that is not one, W
+// per pair, a trailing partial pair dropped; then the set of the pairs.
+// `text` holds n bytes and a terminating zero.
+int load_pairs(PairSet& ps, const char* text, size_t n, cudaStream_t s) {
+    gp_ctx* c = ps.c;
+    if (n == 0) return GP_OK;
+    const bool huge = n >> 32;  // more text than the device's 32-bit offsets reach
+    const int64_t blocks = huge ? 1 : (int64_t)((n + kParseBlock - 1) / kParseBlock);
+    DevBuf &dt = c->eq[kEqText], &dcnt = c->eq[kEqCount], &doff = c->eq[kEqOffs], &dscan = c->eq[kEqScan],
+           &dv = c->eq[kEqVals], &dinfo = c->eq[kEqInfo], &dcode = c->eq[kEqCode];
+    // a value takes two bytes of text at least (one blank), but for the last
+    const size_t padded = (size_t)(blocks + 1) * kParseBlock;
+    if (!dt.ensure(padded) || !dcnt.ensure((size_t)blocks * 4) || !doff.ensure((size_t)blocks * 4) ||
+        !dscan.ensure(gp::scan_tmp_bytes(blocks)) || !dv.ensure(padded / 2 + 1) || !dinfo.ensure(sizeof(TextInfo)) ||
+        !dcode.ensure(256))
+        return c->fail(GP_ERR_NOMEM, "equivalence filter: text buffers");
+    TextInfo info{};
+    uint32_t last[2] = {0, 0};
+    if (!huge) {
+        GP_CUDA_TRY(c, cudaMemsetAsync(static_cast<char*>(dt.p) + n, ' ', padded - n, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(dt.p, text, n, cudaMemcpyHostToDevice, s));
+        GP_CUDA_TRY(c, cudaMemsetAsync(dinfo.p, 0, sizeof(TextInfo), s));
+        pair_values_kernel<false><<<(unsigned)blocks, kParseThreads, 0, s>>>(dt.as<char>(), dcnt.as<uint32_t>(), nullptr,
+                                                                             nullptr, dinfo.as<TextInfo>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        GP_CUDA_TRY(c, gp::exclusive_scan_u32(dcnt.as<uint32_t>(), doff.as<uint32_t>(), blocks, dscan.as<uint32_t>(), s));
+        pair_values_kernel<true><<<(unsigned)blocks, kParseThreads, 0, s>>>(dt.as<char>(), dcnt.as<uint32_t>(),
+                                                                            doff.as<uint32_t>(), dv.as<int8_t>(),
+                                                                            dinfo.as<TextInfo>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&info, dinfo.p, sizeof info, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&last[0], doff.as<uint32_t>() + blocks - 1, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&last[1], dcnt.as<uint32_t>() + blocks - 1, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    }
+    int64_t nvals = (int64_t)last[0] + last[1];
+    if (huge || info.bad) {  // signs, other characters or large values: as strtol takes them
+        const std::vector<int8_t> vals = host_values(text);
+        nvals = (int64_t)vals.size();
+        info = TextInfo{};
+        for (int8_t v : vals) info.present[(v + 128) >> 5] |= 1u << (v & 31);
+        if (!dv.ensure(vals.size() + 1)) return c->fail(GP_ERR_NOMEM, "equivalence filter: values");
+        GP_CUDA_TRY(c, cudaMemcpyAsync(dv.p, vals.data(), vals.size(), cudaMemcpyHostToDevice, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    }
+    const int64_t n0 = nvals / ps.W;
+    if (n0 == 0) return GP_OK;
+    if (n0 > INT32_MAX) return c->fail(GP_ERR_UNSUPPORTED, "equivalence filter: %lld pairs", (long long)n0);
+    // ranks of the values that occur and of their negatives (images change signs)
+    uint8_t code[256] = {};
+    int used = 0;
+    for (int v = -128; v < 128; ++v) {
+        const int8_t neg = (int8_t)-v;
+        if (((info.present[(v + 128) >> 5] >> (v & 31)) & 1u) || ((info.present[(neg + 128) >> 5] >> (neg & 31)) & 1u))
+            code[(uint8_t)v] = (uint8_t)used++;
+    }
+    ps.bits = 1;
+    while ((1 << ps.bits) < used) ++ps.bits;
+    const int per = 32 / ps.bits;
+    ps.Wk = (ps.W + per - 1) / per;
+    ps.code = dcode.as<uint8_t>();
+    GP_CUDA_TRY(c, cudaMemcpyAsync(dcode.p, code, 256, cudaMemcpyHostToDevice, s));
+    DevBuf &didx = c->eq[kEqIdx], &dflag = c->eq[kEqFlag], &dpos = c->eq[kEqPos], &dout = c->eq[kEqOut],
+           &drow = c->eq[kEqRows];
+    if (!didx.ensure((size_t)n0 * 4) || !dflag.ensure((size_t)n0 * 4) || !dpos.ensure((size_t)n0 * 4) ||
+        !dscan.ensure(gp::scan_tmp_bytes(n0)) || !dout.ensure((size_t)n0 * 4 + 4))
+        return c->fail(GP_ERR_NOMEM, "equivalence filter: sort buffers");
+    const int rc = sort_rows(ps, dv.as<int8_t>(), n0, didx.as<uint32_t>(), dflag.as<uint32_t>(), s);
+    if (rc) return rc;
+    uint32_t* d_cnt = dout.as<uint32_t>() + n0;
+    GP_CUDA_TRY(c, gp::compact_flags(dflag.as<uint32_t>(), didx.as<uint32_t>(), dout.as<uint32_t>(), n0,
+                                     dpos.as<uint32_t>(), dscan.as<uint32_t>(), d_cnt, s));
+    uint32_t nu = 0;
+    GP_CUDA_TRY(c, cudaMemcpyAsync(&nu, d_cnt, 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    ps.np = nu;
+    if (!drow.ensure((size_t)nu * ps.W)) return c->fail(GP_ERR_NOMEM, "equivalence filter: pairs");
+    ps.rows = drow.as<int8_t>();
+    gather_rows_kernel<<<grid_of((int64_t)nu * ps.W, 256), 256, 0, s>>>(dv.as<int8_t>(), dout.as<uint32_t>(), nu, ps.W,
+                                                                        ps.rows);
+    GP_CUDA_TRY(c, cudaGetLastError());
+    return GP_OK;
+}
+
+// Class sizes and members of a pair set by canonical forms (canon_kernel):
+// member_list[span[i].first .. span[i].second) are the pairs with the same
+// least image as pair i (itself included), csize[i] is the group order over
+// the number of elements fixing pair i.  L >= 3.
+int canonical_classes(PairSet& ps, int L, int compress, std::vector<unsigned long long>& csize,
+                      std::vector<uint32_t>& member_list, std::vector<std::pair<uint32_t, uint32_t>>& span,
+                      cudaStream_t s) {
+    gp_ctx* c = ps.c;
     const int W = 2 * L;
-    const int64_t np = (int64_t)P.size();
+    const int64_t np = ps.np;
     const std::vector<int16_t> units = all_units(L);
-    std::vector<int8_t> pairs((size_t)np * W);
-    for (int64_t i = 0; i < np; ++i) std::memcpy(&pairs[(size_t)i * W], P[i].data(), W);
-    cudaStream_t s = c->s_comp;
-    DevBuf dp, du, dc, df;
-    if (!dp.ensure(pairs.size()) || !du.ensure(units.size() * 2) || !dc.ensure(pairs.size()) ||
-        !df.ensure((size_t)np * 4))
+    DevBuf &du = c->eq[kEqUnits], &dc = c->eq[kEqCanon], &df = c->eq[kEqFix], &didx = c->eq[kEqIdx],
+           &dflag = c->eq[kEqFlag];
+    if (!du.ensure(units.size() * 2) || !dc.ensure((size_t)np * W) || !df.ensure((size_t)np * 4))
         return c->fail(GP_ERR_NOMEM, "equivalence filter: device allocation");
-    GP_CUDA_TRY(c, cudaMemcpyAsync(dp.p, pairs.data(), pairs.size(), cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(du.p, units.data(), units.size() * 2, cudaMemcpyHostToDevice, s));
     CanonArgs ca{};
-    ca.pairs = dp.as<int8_t>();
+    ca.pairs = ps.rows;
     ca.np = np;
     ca.L = L;
     ca.units = du.as<int16_t>();
@@ -541,10 +835,14 @@ int canonical_classes(gp_ctx* c, int L, int compress, const std::vector<std::vec
     const int64_t grid = std::min<int64_t>(np, (int64_t)c->num_sms * 16);
     canon_kernel<<<(unsigned)grid, kCanonThreads, 0, s>>>(ca);
     GP_CUDA_TRY(c, cudaGetLastError());
-    std::vector<int8_t> canon(pairs.size());
-    std::vector<uint32_t> fixers(np);
-    GP_CUDA_TRY(c, cudaMemcpyAsync(canon.data(), dc.p, canon.size(), cudaMemcpyDeviceToHost, s));
+    // the classes: runs of equal least images
+    const int rc = sort_rows(ps, ca.canon, np, didx.as<uint32_t>(), dflag.as<uint32_t>(), s);
+    if (rc) return rc;
+    std::vector<uint32_t> fixers(np), flags(np);
+    member_list.resize(np);
     GP_CUDA_TRY(c, cudaMemcpyAsync(fixers.data(), df.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaMemcpyAsync(flags.data(), dflag.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaMemcpyAsync(member_list.data(), didx.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
     GP_CUDA_TRY(c, cudaStreamSynchronize(s));
     const uint64_t G = pair_group_size(L, compress);
     for (int64_t i = 0; i < np; ++i) {
@@ -553,21 +851,49 @@ int canonical_classes(gp_ctx* c, int L, int compress, const std::vector<std::vec
                            (unsigned long long)G, (long long)i);
         csize[i] = G / fixers[i];
     }
-    // the classes: runs of equal least images
-    std::vector<uint32_t> ord(np);
-    for (int64_t i = 0; i < np; ++i) ord[i] = (uint32_t)i;
-    auto row = [&](uint32_t i) { return canon.data() + (size_t)i * W; };
-    std::sort(ord.begin(), ord.end(), [&](uint32_t x, uint32_t y) {
-        const int d = std::memcmp(row(x), row(y), (size_t)W);
-        return d != 0 ? d < 0 : x < y;
-    });
     for (int64_t r0 = 0; r0 < np;) {
         int64_t r1 = r0 + 1;
-        while (r1 < np && std::memcmp(row(ord[r0]), row(ord[r1]), (size_t)W) == 0) ++r1;
-        for (int64_t k = r0; k < r1; ++k) span[ord[k]] = {(uint32_t)r0, (uint32_t)r1};
+        while (r1 < np && !flags[r1]) ++r1;
+        for (int64_t k = r0; k < r1; ++k) span[member_list[k]] = {(uint32_t)r0, (uint32_t)r1};
         r0 = r1;
     }
-    member_list.swap(ord);
+    return GP_OK;
+}
+
+// The kept pairs' lines, in order.
+int pair_lines(PairSet& ps, const std::vector<char>& alive, std::string& out, cudaStream_t s) {
+    gp_ctx* c = ps.c;
+    out.clear();
+    if (ps.np == 0) return GP_OK;
+    const int64_t np = ps.np;
+    // rows at a time: a block's text stays below 2^31 bytes (5 bytes a value at most)
+    const int64_t step = std::min<int64_t>(np, (int64_t(1) << 31) / (5 * ps.W + 2));
+    DevBuf &da = c->eq[kEqAlive], &db = c->eq[kEqBytes], &dat = c->eq[kEqPos], &dscan = c->eq[kEqScan],
+           &dl = c->eq[kEqLine];
+    if (!da.ensure((size_t)np) || !db.ensure((size_t)step * 4) || !dat.ensure((size_t)step * 4) ||
+        !dscan.ensure(gp::scan_tmp_bytes(step)))
+        return c->fail(GP_ERR_NOMEM, "equivalence filter: line buffers");
+    GP_CUDA_TRY(c, cudaMemcpyAsync(da.p, alive.data(), (size_t)np, cudaMemcpyHostToDevice, s));
+    for (int64_t r0 = 0; r0 < np; r0 += step) {
+        const int64_t n = std::min(step, np - r0);
+        const int8_t* rows = ps.rows + r0 * ps.W;
+        const uint8_t* keep = da.as<uint8_t>() + r0;
+        pair_line_bytes_kernel<<<grid_of(n, 256), 256, 0, s>>>(rows, keep, n, ps.W, db.as<uint32_t>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        GP_CUDA_TRY(c, gp::exclusive_scan_u32(db.as<uint32_t>(), dat.as<uint32_t>(), n, dscan.as<uint32_t>(), s));
+        uint32_t last[2] = {0, 0};
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&last[0], dat.as<uint32_t>() + n - 1, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&last[1], db.as<uint32_t>() + n - 1, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+        const size_t bytes = (size_t)last[0] + last[1];
+        if (!dl.ensure(bytes + 1)) return c->fail(GP_ERR_NOMEM, "equivalence filter: text buffer");
+        pair_lines_kernel<<<grid_of(n, 8), 256, 0, s>>>(rows, keep, n, ps.W, dat.as<uint32_t>(), dl.as<char>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        const size_t at = out.size();
+        out.resize(at + bytes);
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&out[at], dl.p, bytes, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    }
     return GP_OK;
 }
 
@@ -672,36 +998,29 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
             if (t.joinable()) t.join();
         }
     } joiner{group_thread};
-    // filter.cpp:45-62: L values for a, then (if the stream is still good) L
-    // for b: whitespace-separated integers up to the first token that is not
-    // one, W per pair, a trailing partial pair dropped
-    std::vector<std::vector<int8_t>> P;
+    std::string text;
     {
-        std::string text;
         fseek(in, 0, SEEK_END);
         const long sz = ftell(in);
         fseek(in, 0, SEEK_SET);
         text.resize(sz > 0 ? (size_t)sz : 0);
         text.resize(sz > 0 ? fread(&text[0], 1, (size_t)sz, in) : 0);
         fclose(in);
-        std::vector<int8_t> cur;
-        const char* q = text.c_str();
-        for (;;) {
-            char* e;
-            const long v = strtol(q, &e, 10);
-            if (e == q) break;
-            q = e;
-            cur.push_back((int8_t)v);
-            if ((int)cur.size() == W) {
-                P.push_back(cur);
-                cur.clear();
-            }
-        }
     }
     lap("read");
-    std::sort(P.begin(), P.end());
-    P.erase(std::unique(P.begin(), P.end()), P.end());
-    const int64_t np = (int64_t)P.size();
+    struct OutCloser {  // an error leaves the output empty, as opened
+        FILE*& f;
+        ~OutCloser() {
+            if (f) fclose(f);
+        }
+    } out_closer{out};
+    cudaStream_t s = c->s_comp;
+    PairSet ps{c, W};
+    int rc = load_pairs(ps, text.c_str(), text.size(), s);
+    if (rc) return rc;
+    std::string().swap(text);
+    lap("pairs");
+    const int64_t np = ps.np;
     std::vector<char> alive(np, 1);
     if (np > 0) {
         std::vector<unsigned long long> csize(np);
@@ -709,20 +1028,12 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
         std::vector<uint32_t> member_list;
         std::vector<std::pair<uint32_t, uint32_t>> span(np);
         if (L >= 3) {
-            lap("sort");
-            int rc = canonical_classes(c, L, compress, P, csize, member_list, span);
-            if (rc) {
-                if (out) fclose(out);
-                return rc;
-            }
+            rc = canonical_classes(ps, L, compress, csize, member_list, span, s);
+            if (rc) return rc;
             lap("classes");
         } else {
-            lap("sort");
             group_thread.join();
-            if (group_failed) {
-                if (out) fclose(out);
-                return c->fail(GP_ERR_NOMEM, "equivalence filter: generator group of length %d", L);
-            }
+            if (group_failed) return c->fail(GP_ERR_NOMEM, "equivalence filter: generator group of length %d", L);
             lap("group");
             const int64_t ng = (int64_t)(gens.size() / (size_t)W);
             std::vector<int16_t> items((size_t)ng * W);  // transposed: items[o * ng + g]
@@ -742,15 +1053,15 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
             }
             lap("table");
             std::vector<int8_t> pairs((size_t)np * W);
-            for (int64_t i = 0; i < np; ++i)
-                for (int j = 0; j < W; ++j) pairs[i * W + j] = P[i][j];
+            GP_CUDA_TRY(c, cudaMemcpyAsync(pairs.data(), ps.rows, pairs.size(), cudaMemcpyDeviceToHost, s));
+            GP_CUDA_TRY(c, cudaStreamSynchronize(s));
             // hash set of the pairs (the image lookup), same hash as the kernel's
             uint32_t set_size = 1;
             while (set_size < 2 * (uint64_t)np) set_size <<= 1;
             std::vector<uint32_t> set_h(set_size, 0), set_i(set_size, 0xFFFFFFFFu);
             for (int64_t i = 0; i < np; ++i) {
                 uint32_t h = kFnvBasis;
-                for (int j = 0; j < W; ++j) h = fnv_step(h, P[i][j]);
+                for (int j = 0; j < W; ++j) h = fnv_step(h, pairs[i * W + j]);
                 h = fnv_fold(h);
                 uint32_t slot = h & (set_size - 1);
                 while (set_i[slot] != 0xFFFFFFFFu) slot = (slot + 1) & (set_size - 1);
@@ -758,14 +1069,12 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
                 set_i[slot] = (uint32_t)i;
             }
             const int64_t mcap = std::max<int64_t>(np * 64, 1 << 20);
-            cudaStream_t s = c->s_comp;
-            DevBuf di, dp, dsh, dsi, dst, dm, dmisc;
-            if (!di.ensure(items.size() * 2) || !dp.ensure(pairs.size()) || !dsh.ensure((size_t)set_size * 4) ||
+            DevBuf di, dsh, dsi, dst, dm, dmisc;
+            if (!di.ensure(items.size() * 2) || !dsh.ensure((size_t)set_size * 4) ||
                 !dsi.ensure((size_t)set_size * 4) || !dst.ensure(np * 4) || !dm.ensure((size_t)mcap * 8) ||
                 !dmisc.ensure(64))
                 return c->fail(GP_ERR_NOMEM, "equivalence filter: device allocation");
             GP_CUDA_TRY(c, cudaMemcpyAsync(di.p, items.data(), items.size() * 2, cudaMemcpyHostToDevice, s));
-            GP_CUDA_TRY(c, cudaMemcpyAsync(dp.p, pairs.data(), pairs.size(), cudaMemcpyHostToDevice, s));
             GP_CUDA_TRY(c, cudaMemcpyAsync(dsh.p, set_h.data(), (size_t)set_size * 4, cudaMemcpyHostToDevice, s));
             GP_CUDA_TRY(c, cudaMemcpyAsync(dsi.p, set_i.data(), (size_t)set_size * 4, cudaMemcpyHostToDevice, s));
             GP_CUDA_TRY(c, cudaMemsetAsync(dst.p, 0, np * 4, s));
@@ -773,7 +1082,7 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
             ClassArgs ca{};
             ca.srcT = di.as<int16_t>();
             ca.ng = ng;
-            ca.pairs = dp.as<int8_t>();
+            ca.pairs = ps.rows;
             ca.np = np;
             ca.W = W;
             ca.set_h = dsh.as<uint32_t>();
@@ -798,22 +1107,17 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
             GP_CUDA_TRY(c, cudaGetLastError());
             GP_CUDA_TRY(c, cudaStreamSynchronize(s));
             lap("classes");
-            int rc = c->check_status("equivalence filter");
-            if (rc) {
-                if (out) fclose(out);
-                return rc;
-            }
+            rc = c->check_status("equivalence filter");
+            if (rc) return rc;
             std::vector<uint32_t> stab(np);
             unsigned long long nmem = 0;
             GP_CUDA_TRY(c, cudaMemcpy(stab.data(), dst.p, np * 4, cudaMemcpyDeviceToHost));
             GP_CUDA_TRY(c, cudaMemcpy(&nmem, dmisc.p, 8, cudaMemcpyDeviceToHost));
             // orbit-stabiliser: class size = group order / generators fixing the pair
             for (int64_t i = 0; i < np; ++i) {
-                if (stab[i] == 0 || ng % stab[i] != 0) {
-                    if (out) fclose(out);
+                if (stab[i] == 0 || ng % stab[i] != 0)
                     return c->fail(GP_ERR_CUDA, "equivalence filter: stabiliser of pair %lld is %u of %lld generators",
                                    (long long)i, stab[i], (long long)ng);
-                }
                 csize[i] = (unsigned long long)(ng / stab[i]);
             }
             std::vector<uint32_t> mem((size_t)nmem * 2);
@@ -853,32 +1157,13 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
     }
     lap("erase");
     if (out) {
-        // "%d " per entry of a, " ", "%d " per entry of b, newline
-        std::string buf;
-        buf.reserve((size_t)np * (3 * W + 2));
-        auto put = [&](int v) {
-            if (v < 0) {
-                buf.push_back('-');
-                v = -v;
-            }
-            char tmp[8];
-            int n = 0;
-            do {
-                tmp[n++] = (char)('0' + v % 10);
-                v /= 10;
-            } while (v);
-            while (n) buf.push_back(tmp[--n]);
-            buf.push_back(' ');
-        };
-        for (int64_t i = 0; i < np; ++i) {
-            if (!alive[i]) continue;
-            for (int k = 0; k < L; ++k) put(P[i][k]);
-            buf.push_back(' ');
-            for (int k = 0; k < L; ++k) put(P[i][L + k]);
-            buf.push_back('\n');
-        }
-        const bool ok = buf.empty() || fwrite(buf.data(), 1, buf.size(), out) == buf.size();
-        if (fclose(out) != 0 || !ok) return c->fail(GP_ERR_IO, "equivalence filter: write failed: %s", out_path);
+        std::string lines;
+        rc = pair_lines(ps, alive, lines, s);
+        if (rc) return rc;
+        const bool ok = lines.empty() || fwrite(lines.data(), 1, lines.size(), out) == lines.size();
+        const int closed = fclose(out);
+        out = nullptr;
+        if (closed != 0 || !ok) return c->fail(GP_ERR_IO, "equivalence filter: write failed: %s", out_path);
     }
     lap("written");
     return GP_OK;

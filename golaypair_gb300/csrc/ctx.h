@@ -138,6 +138,7 @@ struct gp_ctx {
     // grow-only scratch of the uncompression stage (kept across pairs: a
     // cudaFree per pair would synchronise the device every pair)
     DevBuf ux[66];
+    DevBuf eq[20];  // grow-only scratch of the equivalence filter
     HostPinned hscratch[4];
     // batched generation: one stream per job branch, fork/join events
     static constexpr int kJobStreams = 8;
