@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "pair_text.cuh"
 #include "prims.h"
 
 namespace {
@@ -417,61 +418,18 @@ __global__ void gather_rows_kernel(const int8_t* rows, const uint32_t* idx, int6
     }
 }
 
-// Bytes of "%d ".
-__device__ __forceinline__ int value_bytes(int v) {
-    const int u = v < 0 ? -v : v;
-    return (v < 0 ? 1 : 0) + (u >= 100 ? 3 : u >= 10 ? 2 : 1) + 1;
-}
-
-// Bytes of each kept pair's line (0: left out): "%d " per entry of a, " ",
-// "%d " per entry of b, newline.
+// Bytes of each kept pair's line (0: left out).
 __global__ void pair_line_bytes_kernel(const int8_t* rows, const uint8_t* alive, int64_t n, int W, uint32_t* bytes) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t b = 0;
-        if (alive[i]) {
-            b = 2;
-            for (int o = 0; o < W; ++o) b += (uint32_t)value_bytes(rows[i * W + o]);
-        }
-        bytes[i] = b;
-    }
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        bytes[i] = alive[i] ? (uint32_t)gp::pair_line_bytes(rows + i * W, rows + i * W + W / 2, W / 2) : 0u;
 }
 
-// The lines: a warp per pair, 32 entries at a time.
+// The lines, a warp per pair.
 __global__ void __launch_bounds__(256) pair_lines_kernel(const int8_t* rows, const uint8_t* alive, int64_t n, int W,
                                                          const uint32_t* at, char* text) {
-    const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-        if (!alive[i]) continue;
-        char* line = text + at[i];
-        for (int o0 = 0; o0 < W; o0 += 32) {
-            const int o = o0 + lane;
-            const int v = o < W ? rows[i * W + o] : 0;
-            // the blank between the halves before entry L, the newline after the last
-            int mine = o < W ? value_bytes(v) + (o == W / 2 ? 1 : 0) + (o == W - 1 ? 1 : 0) : 0;
-            int incl = mine;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-                if (lane >= d) incl += y;
-            }
-            if (o < W) {
-                char* q = line + incl - mine;
-                if (o == W / 2) *q++ = ' ';
-                int u = v;
-                if (v < 0) {
-                    *q++ = '-';
-                    u = -v;
-                }
-                if (u >= 100) *q++ = (char)('0' + u / 100);
-                if (u >= 10) *q++ = (char)('0' + u / 10 % 10);
-                *q++ = (char)('0' + u % 10);
-                *q++ = ' ';
-                if (o == W - 1) *q = '\n';
-            }
-            line += __shfl_sync(0xFFFFFFFFu, incl, 31);
-        }
-    }
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps)
+        if (alive[i]) gp::put_pair_line(rows + i * W, rows + i * W + W / 2, W / 2, text + at[i]);
 }
 
 // Every unit mod L, ascending.
@@ -1018,6 +976,7 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
         }
     } out_closer{out};
     cudaStream_t s = c->s_comp;
+    KeepSmall keep{c->eq};
     PairSet ps{c, W};
     int rc = load_pairs(ps, text.c_str(), text.size(), s);
     if (rc) return rc;

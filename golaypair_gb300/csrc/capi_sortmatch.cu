@@ -19,28 +19,21 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
+
+#include <fcntl.h>
+#include <sys/stat.h>
+#include <unistd.h>
 
 #include "ctx.h"
 #include "prims.h"
 #include "host_par.h"
+#include "pair_text.cuh"
 #include "survivors.h"
 
 namespace {
-
-bool slurp(const char* path, std::string& out) {
-    FILE* f = fopen(path, "rb");
-    if (!f) return false;
-    fseek(f, 0, SEEK_END);
-    long sz = ftell(f);
-    fseek(f, 0, SEEK_SET);
-    out.resize(sz > 0 ? (size_t)sz : 0);
-    size_t got = sz > 0 ? fread(&out[0], 1, (size_t)sz, f) : 0;
-    fclose(f);
-    out.resize(got);
-    return true;
-}
 
 // 4-bit codes preserving byte order; 0 = padding
 __host__ __device__ inline int code4(unsigned char ch) {
@@ -54,7 +47,8 @@ __host__ __device__ inline int code4(unsigned char ch) {
     }
 }
 
-__global__ void build_keys_kernel(const char* text, const uint64_t* start, const uint32_t* len, int64_t n, int W,
+template <class Off>
+__global__ void build_keys_kernel(const char* text, const Off* start, const uint32_t* len, int64_t n, int W,
                                   int nibble, uint32_t* keys) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const char* s = text + start[i];
@@ -132,6 +126,299 @@ unsigned grid_for(int64_t n) {
     int64_t g = (n + 255) / 256;
     if (g > 65535 * 8) g = 65535 * 8;
     return (unsigned)(g < 1 ? 1 : g);
+}
+
+// ------------------------------------------------------------ text on the device
+// A file's bytes go to the device as they are; its lines are found, keyed,
+// compared and written out there.  Offsets are 32 bits: more text than that
+// takes the host's line index (gp_sort_text, gp_match_texts).  Sort and match
+// of the 430,000 lines of a whole order 51: 13.7 ms, 43.3 with the lines, the
+// parse, the merge and the copies on host threads.
+constexpr int kTextThreads = 256;
+constexpr int kTextEach = 16;                            // bytes per thread
+constexpr int kTextBlock = kTextThreads * kTextEach;
+constexpr uint64_t kMaxDeviceText = (uint64_t(1) << 32) - 2 * kTextBlock;
+
+// Newlines of a text padded to whole blocks (by anything but newlines).
+// WRITE = false: per block; true: line i + 1 starts after the i-th newline.
+// *other: set when a character is none of "0-9", "-", "P", "S", "D", blank, newline.
+template <bool WRITE>
+__global__ void __launch_bounds__(kTextThreads) line_starts_kernel(const char* text, uint32_t n, uint32_t* counts,
+                                                                   const uint32_t* offs, uint32_t* start,
+                                                                   int* other) {
+    __shared__ uint32_t s_warp[kTextThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t p0 = blockIdx.x * (uint32_t)kTextBlock + threadIdx.x * kTextEach;
+    const uint4 w = *reinterpret_cast<const uint4*>(text + p0);
+    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+    uint32_t nl = 0;
+    bool odd = false;
+#pragma unroll
+    for (int k = 0; k < kTextEach; ++k) {
+        const int c = (ww[k >> 2] >> (8 * (k & 3))) & 0xFF;
+        if (p0 + k >= n) break;
+        if (c == '\n')
+            nl |= 1u << k;
+        else if (code4((unsigned char)c) < 0)
+            odd = true;
+    }
+    const uint32_t mine = (uint32_t)__popc(nl);
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (int q = 0; q < kTextThreads / 32; ++q) {
+        if (q < warp) before += s_warp[q];
+        total += s_warp[q];
+    }
+    if constexpr (!WRITE) {
+        if (threadIdx.x == 0) counts[blockIdx.x] = total;
+        if (odd) *other = 1;
+    } else {
+        uint32_t* out = start + offs[blockIdx.x] + before + incl - mine + 1;
+        for (uint32_t m = nl; m; m &= m - 1u) *out++ = p0 + (uint32_t)__ffs((int)m);
+        if (blockIdx.x == 0 && threadIdx.x == 0) start[0] = 0;
+    }
+}
+
+// Lengths without the newline, and the longest.
+__global__ void line_lengths_kernel(const uint32_t* start, int64_t n, uint32_t* len, unsigned* longest) {
+    unsigned most = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t l = start[i + 1] - start[i] - 1;
+        len[i] = l;
+        most = l > most ? l : most;
+    }
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    if ((threadIdx.x & 31) == 0 && most) atomicMax(longest, most);
+}
+
+// Candidate lines: the first token's place, then exactly L integers, read
+// as parse_candidates reads them (the text holds none of the characters on
+// which the two could differ).  A line of blanks is no candidate (tok_len 0);
+// *bad: a line with fewer integers.
+__global__ void parse_lines_kernel(const char* text, const uint32_t* start, const uint32_t* len, int64_t n, int L,
+                                   uint32_t* tok_off, uint32_t* tok_len, int8_t* seqs, int* bad) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const char* q = text + start[i];
+        const char* const end = q + len[i];
+        while (q < end && *q == ' ') ++q;
+        const char* const t = q;
+        while (q < end && *q != ' ') ++q;
+        tok_off[i] = (uint32_t)(t - text);
+        tok_len[i] = (uint32_t)(q - t);
+        if (q == t) {
+            *bad = 1;  // a line of blanks (left to the host)
+            continue;
+        }
+        int got = 0;
+        for (; got < L; ++got) {
+            while (q < end && *q == ' ') ++q;
+            const bool neg = q < end && *q == '-';
+            if (neg) ++q;
+            if (q >= end || *q < '0' || *q > '9') break;
+            unsigned v = 0;
+            for (; q < end && *q >= '0' && *q <= '9'; ++q) v = v * 10 + (unsigned)(*q - '0');
+            seqs[i * L + got] = (int8_t)(neg ? 0u - v : v);
+        }
+        if (got != L) *bad = 1;
+    }
+}
+
+// -1, 0, 1: byte order of two tokens, a prefix first
+__device__ __forceinline__ int compare_tokens(const char* a, uint32_t la, const char* b, uint32_t lb) {
+    const uint32_t l = la < lb ? la : lb;
+    for (uint32_t k = 0; k < l; ++k) {
+        const unsigned char x = (unsigned char)a[k], y = (unsigned char)b[k];
+        if (x != y) return x < y ? -1 : 1;
+    }
+    return la == lb ? 0 : la < lb ? -1 : 1;
+}
+
+// *bad: a token above the next line's (the merge of unsorted files is the host's)
+__global__ void tokens_sorted_kernel(const char* text, const uint32_t* off, const uint32_t* len, int64_t n, int* bad) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i + 1 < n; i += (int64_t)gridDim.x * blockDim.x)
+        if (compare_tokens(text + off[i], len[i], text + off[i + 1], len[i + 1]) > 0) *bad = 1;
+}
+
+// For every a line the b lines with its token: [b0, b0 + nb).
+__global__ void token_ranges_kernel(const char* ta, const uint32_t* oa, const uint32_t* la, int64_t na,
+                                    const char* tb, const uint32_t* ob, const uint32_t* lb, int64_t nb_lines,
+                                    uint32_t* b0, uint32_t* nb, unsigned long long* total) {
+    unsigned long long sum = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < na; i += (int64_t)gridDim.x * blockDim.x) {
+        const char* t = ta + oa[i];
+        const uint32_t l = la[i];
+        uint32_t lo = 0, hi = (uint32_t)nb_lines;  // first line not below the token
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (compare_tokens(tb + ob[mid], lb[mid], t, l) < 0)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        uint32_t e = lo, step = 1;  // first line above it: a few lines on
+        while (e < nb_lines && compare_tokens(tb + ob[e], lb[e], t, l) == 0) {
+            ++e;
+            if (++step > 8) {
+                uint32_t top = (uint32_t)nb_lines;
+                while (e < top) {
+                    const uint32_t mid = e + (top - e) / 2;
+                    if (compare_tokens(tb + ob[mid], lb[mid], t, l) <= 0)
+                        e = mid + 1;
+                    else
+                        top = mid;
+                }
+                break;
+            }
+        }
+        b0[i] = lo;
+        nb[i] = e - lo;
+        sum += e - lo;
+    }
+    for (int o = 16; o; o >>= 1) sum += __shfl_down_sync(0xFFFFFFFFu, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(total, sum);
+}
+
+// one thread per candidate pair (a line, line of its range): flags[w] = 1 if
+// the pair is complementary
+__global__ void range_check_kernel(const uint32_t* first, const uint32_t* b0, int64_t na, uint32_t total,
+                                   const int* pafa, const int* pafb, int H, int target, uint32_t* flags,
+                                   uint32_t* ia, uint32_t* ib) {
+    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total;
+         w += (uint64_t)gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = na - 1;  // the last a line whose first pair is <= w
+        while (lo < hi) {
+            const int64_t mid = (lo + hi + 1) >> 1;
+            if (first[mid] <= w)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        const uint32_t b = b0[lo] + (uint32_t)(w - first[lo]);
+        ia[w] = (uint32_t)lo;
+        ib[w] = b;
+        const int* pa = pafa + lo * H;
+        const int* pb = pafb + (int64_t)b * H;
+        uint32_t ok = 1;
+        for (int s = 0; s < H; ++s)
+            if (pa[s] + pb[s] != target) {
+                ok = 0;
+                break;
+            }
+        flags[w] = ok;
+    }
+}
+
+// The kept pairs' lines (src/io.cpp PairWriter).
+__global__ void match_line_bytes_kernel(const int8_t* a, const int8_t* b, const uint32_t* ia, const uint32_t* ib,
+                                        const uint32_t* keep, int64_t n, int L, uint32_t* bytes) {
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
+        bytes[k] = (uint32_t)gp::pair_line_bytes(a + (int64_t)ia[keep[k]] * L, b + (int64_t)ib[keep[k]] * L, L);
+}
+__global__ void __launch_bounds__(256) match_lines_kernel(const int8_t* a, const int8_t* b, const uint32_t* ia,
+                                                          const uint32_t* ib, const uint32_t* keep, int64_t n, int L,
+                                                          const uint32_t* at, char* text) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t k = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < n; k += warps)
+        gp::put_pair_line(a + (int64_t)ia[keep[k]] * L, b + (int64_t)ib[keep[k]] * L, L, text + at[k]);
+}
+
+// A file's bytes, unset until read: pieces read by host threads.
+struct FileText {
+    std::unique_ptr<char[]> p;
+    size_t n = 0;
+};
+bool read_file(const char* path, FileText& t) {
+    const int fd = open(path, O_RDONLY);
+    if (fd < 0) return false;
+    struct stat sb;
+    const size_t size = fstat(fd, &sb) == 0 && S_ISREG(sb.st_mode) && sb.st_size > 0 ? (size_t)sb.st_size : 0;
+    t.p.reset(new char[size + 1]);
+    constexpr size_t kPiece = size_t(2) << 20;
+    const size_t pieces = (size + kPiece - 1) / kPiece;
+    std::vector<size_t> got(pieces, 0);
+    gp::par_for(pieces, [&](size_t k) {
+        const size_t lo = k * kPiece, hi = std::min(size, lo + kPiece);
+        size_t at = lo;
+        while (at < hi) {
+            const ssize_t r = pread(fd, t.p.get() + at, hi - at, (off_t)at);
+            if (r <= 0) break;
+            at += (size_t)r;
+        }
+        got[k] = at - lo;
+    });
+    close(fd);
+    t.n = 0;
+    for (size_t k = 0; k < pieces; ++k) {  // a file cut short meanwhile ends at its first short piece
+        t.n += got[k];
+        if (got[k] < std::min(kPiece, size - k * kPiece)) break;
+    }
+    t.p[t.n] = 0;
+    return true;
+}
+
+// Device text to a new file of the sort (an input may have the same name:
+// it has been read by now).
+int write_text(gp_ctx* c, const char* d_text, size_t n, const char* path, cudaStream_t s) {
+    std::unique_ptr<char[]> h(new char[n + 1]);
+    GP_CUDA_TRY(c, cudaMemcpyAsync(h.get(), d_text, n, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    FILE* f = fopen(path, "w");
+    if (!f) return c->fail(GP_ERR_IO, "sort: cannot write %s", path);
+    fwrite(h.get(), 1, n, f);
+    return fclose(f) == 0 ? GP_OK : c->fail(GP_ERR_IO, "sort: write failed");
+}
+
+// The context's sort and match buffers, one use each.
+enum TextBuf { kTbText, kTbTextB, kTbCount, kTbOffs, kTbScan, kTbMisc, kTbStart, kTbLen, kTbStartB, kTbLenB, kTbKeys, kTbIdx,
+               kTbTmp, kTbFlag, kTbPos, kTbOrder, kTbOutLen, kTbOutOff, kTbOut, kTbTokA, kTbTokLenA, kTbTokB,
+               kTbTokLenB, kTbSeqA, kTbSeqB, kTbPafA, kTbPafB, kTbIa, kTbIb };
+
+// A text of n bytes, ending in a newline, at d_text (room for a block past
+// it): its lines' starts (lines + 1 entries) and lengths, their number, the
+// longest, and whether it holds other characters than candidate lines do.
+struct Lines {
+    int64_t n = 0;
+    unsigned longest = 0;
+    int other = 0;
+};
+int find_lines(gp_ctx* c, const char* d_text, size_t n, DevBuf& start, DevBuf& len, Lines& out, cudaStream_t s) {
+    const int64_t blocks = (int64_t)((n + kTextBlock - 1) / kTextBlock);
+    DevBuf &cnt = c->st[kTbCount], &off = c->st[kTbOffs], &scan = c->st[kTbScan], &misc = c->st[kTbMisc];
+    if (!cnt.ensure((size_t)blocks * 4) || !off.ensure((size_t)blocks * 4) || !scan.ensure(gp::scan_tmp_bytes(blocks)) ||
+        !misc.ensure(64))
+        return c->fail(GP_ERR_NOMEM, "text: device allocation");
+    GP_CUDA_TRY(c, cudaMemsetAsync(misc.p, 0, 64, s));
+    int* d_other = misc.as<int>();
+    unsigned* d_longest = misc.as<unsigned>() + 1;
+    line_starts_kernel<false><<<(unsigned)blocks, kTextThreads, 0, s>>>(d_text, (uint32_t)n, cnt.as<uint32_t>(),
+                                                                        nullptr, nullptr, d_other);
+    GP_CUDA_TRY(c, cudaGetLastError());
+    GP_CUDA_TRY(c, gp::exclusive_scan_u32(cnt.as<uint32_t>(), off.as<uint32_t>(), blocks, scan.as<uint32_t>(), s));
+    uint32_t last[2] = {0, 0};
+    GP_CUDA_TRY(c, cudaMemcpyAsync(&last[0], off.as<uint32_t>() + blocks - 1, 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaMemcpyAsync(&last[1], cnt.as<uint32_t>() + blocks - 1, 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    out.n = (int64_t)last[0] + last[1];
+    if (!start.ensure((size_t)(out.n + 1) * 4) || !len.ensure((size_t)out.n * 4 + 4))
+        return c->fail(GP_ERR_NOMEM, "text: device allocation");
+    line_starts_kernel<true><<<(unsigned)blocks, kTextThreads, 0, s>>>(d_text, (uint32_t)n, nullptr, off.as<uint32_t>(),
+                                                                       start.as<uint32_t>(), nullptr);
+    line_lengths_kernel<<<(unsigned)std::min<int64_t>((out.n + 255) / 256 + 1, 4096), 256, 0, s>>>(
+        start.as<uint32_t>(), out.n, len.as<uint32_t>(), d_longest);
+    GP_CUDA_TRY(c, cudaGetLastError());
+    int h[2] = {0, 0};
+    GP_CUDA_TRY(c, cudaMemcpyAsync(h, misc.p, 8, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    out.other = h[0];
+    out.longest = (unsigned)h[1];
+    return GP_OK;
 }
 
 struct Cand {
@@ -513,7 +800,7 @@ __device__ __forceinline__ char* put_dec(char* o, unsigned v) {
 
 // each record's line (src/utils/io.cpp:14-36) at its offset
 __global__ void surv_format_kernel(const uint8_t* recs, int64_t n, SurvGeom g, const uint32_t* off, char* text,
-                                   uint64_t* start, uint32_t* len) {
+                                   uint32_t* start, uint32_t* len) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const uint8_t* r = recs + i * g.rec_bytes;
         uint64_t lo, hi;
@@ -543,7 +830,8 @@ __global__ void gather_len_kernel(const uint32_t* len, const uint32_t* order, in
 }
 
 // one warp per kept line: its bytes and newline at the line's output offset
-__global__ void gather_lines_kernel(const char* text, const uint64_t* start, const uint32_t* len,
+template <class Off>
+__global__ void gather_lines_kernel(const char* text, const Off* start, const uint32_t* len,
                                     const uint32_t* order, const uint32_t* out_off, int64_t n, char* out) {
     const int lane = threadIdx.x & 31;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -557,15 +845,57 @@ __global__ void gather_lines_kernel(const char* text, const uint64_t* start, con
     }
 }
 
-// Sorted, de-duplicated lines of the records (all of one geometry).
+// n lines on the device (text, starts, lengths without the newline that
+// follows each): sorted and de-duplicated by bytes, to a file.  codes: every
+// character has a 4-bit code.
+int sort_device_lines(gp_ctx* c, const char* d_text, const uint32_t* d_start, const uint32_t* d_len, int64_t n,
+                      unsigned longest, bool codes, const char* out_path, cudaStream_t s) {
+    const int per = codes ? 8 : 4;
+    const int Wk = std::max(1, (int)((longest + per - 1) / per));
+    DevBuf &dk = c->st[kTbKeys], &di = c->st[kTbIdx], &dtmp = c->st[kTbTmp], &dflag = c->st[kTbFlag],
+           &dpos = c->st[kTbPos], &dord = c->st[kTbOrder], &dlen2 = c->st[kTbOutLen], &dooff = c->st[kTbOutOff],
+           &dout = c->st[kTbOut], &dscan = c->st[kTbScan];
+    if (!dk.ensure((size_t)n * Wk * 4) || !di.ensure(n * 4) || !dtmp.ensure(gp::radix_sort_tmp_bytes(n)) ||
+        !dflag.ensure(n * 4) || !dpos.ensure(n * 4) || !dord.ensure(n * 4 + 4) || !dlen2.ensure(n * 4) ||
+        !dooff.ensure(n * 4) || !dscan.ensure(gp::scan_tmp_bytes(n)))
+        return c->fail(GP_ERR_NOMEM, "sort: device allocation");
+    build_keys_kernel<<<grid_for(n), 256, 0, s>>>(d_text, d_start, d_len, n, Wk, codes ? 1 : 0, dk.as<uint32_t>());
+    GP_CUDA_TRY(c, cudaGetLastError());
+    int bits = 8;
+    int rc = sort_radix_bits(c, dk.as<uint32_t>(), Wk, n, di.as<uint32_t>(), dtmp.p, s, &bits);
+    if (rc) return rc;
+    GP_CUDA_TRY(c, gp::iota_u32(di.as<uint32_t>(), n, s));
+    GP_CUDA_TRY(c, gp::radix_sort_keys(dk.as<uint32_t>(), Wk, Wk, di.as<uint32_t>(), n, dtmp.p, s, bits));
+    GP_CUDA_TRY(c, gp::mark_unique(dk.as<uint32_t>(), Wk, di.as<uint32_t>(), n, Wk, dflag.as<uint32_t>(), s));
+    uint32_t* d_cnt = dord.as<uint32_t>() + n;
+    GP_CUDA_TRY(c, gp::compact_flags(dflag.as<uint32_t>(), di.as<uint32_t>(), dord.as<uint32_t>(), n,
+                                     dpos.as<uint32_t>(), dscan.as<uint32_t>(), d_cnt, s));
+    uint32_t nu = 0;
+    GP_CUDA_TRY(c, cudaMemcpyAsync(&nu, d_cnt, 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    gather_len_kernel<<<grid_for(nu), 256, 0, s>>>(d_len, dord.as<uint32_t>(), nu, dlen2.as<uint32_t>());
+    GP_CUDA_TRY(c, cudaGetLastError());
+    GP_CUDA_TRY(c, gp::exclusive_scan_u32(dlen2.as<uint32_t>(), dooff.as<uint32_t>(), nu, dscan.as<uint32_t>(), s));
+    uint32_t o_last = 0, l_last = 0;
+    GP_CUDA_TRY(c, cudaMemcpyAsync(&o_last, dooff.as<uint32_t>() + nu - 1, 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaMemcpyAsync(&l_last, dlen2.as<uint32_t>() + nu - 1, 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    const uint64_t out_bytes = (uint64_t)o_last + l_last;
+    if (!dout.ensure(out_bytes + 16)) return c->fail(GP_ERR_NOMEM, "sort: device allocation");
+    gather_lines_kernel<<<(unsigned)std::min<int64_t>((nu + 7) / 8, 65535 * 8), 256, 0, s>>>(
+        d_text, d_start, d_len, dord.as<uint32_t>(), dooff.as<uint32_t>(), nu, dout.as<char>());
+    GP_CUDA_TRY(c, cudaGetLastError());
+    return write_text(c, dout.as<char>(), out_bytes, out_path, s);
+}
+
+// Sorted, de-duplicated lines of the records (all of one geometry), to a file.
 // Returns GP_ERR_FORMAT on a malformed record.
-int gp_sort_records(gp_ctx* c, const SurvGeom& g, const std::vector<uint8_t>& recs, int64_t n, std::string& out) {
-    out.clear();
-    if (n == 0) return GP_OK;
+int gp_sort_records(gp_ctx* c, const SurvGeom& g, const std::vector<uint8_t>& recs, int64_t n, const char* out_path) {
     cudaStream_t s = c->s_comp;
-    DevBuf dr, dl, dlen2, doff, dscan, dmisc, dt, ds, dk, di, dtmp, dflag, dpos, dord, dooff, dout;
+    if (n == 0) return write_text(c, nullptr, 0, out_path, s);
+    DevBuf dr, dl, doff, dscan, dmisc, dt, ds;
     if (!dr.ensure(recs.size() + 16) || !dl.ensure(n * 4 + 4) || !doff.ensure(n * 4 + 4) ||
-        !dscan.ensure(gp::scan_tmp_bytes(n)) || !dmisc.ensure(64) || !ds.ensure(n * 8))
+        !dscan.ensure(gp::scan_tmp_bytes(n)) || !dmisc.ensure(64) || !ds.ensure(n * 4))
         return c->fail(GP_ERR_NOMEM, "sort: device allocation");
     GP_CUDA_TRY(c, cudaMemcpyAsync(dr.p, recs.data(), recs.size(), cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemsetAsync(dmisc.p, 0, 64, s));
@@ -583,46 +913,11 @@ int gp_sort_records(gp_ctx* c, const SurvGeom& g, const std::vector<uint8_t>& re
     if (hm[1]) return c->fail(GP_ERR_FORMAT, "sort: malformed survivor record");
     const uint64_t total = (uint64_t)last_off + last_len;
     if (total >= (uint64_t(1) << 32)) return c->fail(GP_ERR_UNSUPPORTED, "sort: %llu bytes of lines", (unsigned long long)total);
-    const int Wk = std::max(1, (int)((hm[0] + 7) / 8));
-    if (!dt.ensure(total + 16) || !dk.ensure((size_t)n * Wk * 4) || !di.ensure(n * 4) ||
-        !dtmp.ensure(gp::radix_sort_tmp_bytes(n)) || !dflag.ensure(n * 4) || !dpos.ensure(n * 4) ||
-        !dord.ensure(n * 4 + 4) || !dlen2.ensure(n * 4) || !dooff.ensure(n * 4))
-        return c->fail(GP_ERR_NOMEM, "sort: device allocation");
+    if (!dt.ensure(total + 16)) return c->fail(GP_ERR_NOMEM, "sort: device allocation");
     surv_format_kernel<<<grid_for(n), 256, 0, s>>>(dr.as<uint8_t>(), n, g, doff.as<uint32_t>(), dt.as<char>(),
-                                                   ds.as<uint64_t>(), dl.as<uint32_t>());
-    build_keys_kernel<<<grid_for(n), 256, 0, s>>>(dt.as<char>(), ds.as<uint64_t>(), dl.as<uint32_t>(), n, Wk, 1,
-                                                  dk.as<uint32_t>());
+                                                   ds.as<uint32_t>(), dl.as<uint32_t>());
     GP_CUDA_TRY(c, cudaGetLastError());
-    int bits = 8;
-    int rc = sort_radix_bits(c, dk.as<uint32_t>(), Wk, n, di.as<uint32_t>(), dtmp.p, s, &bits);
-    if (rc) return rc;
-    GP_CUDA_TRY(c, gp::iota_u32(di.as<uint32_t>(), n, s));
-    GP_CUDA_TRY(c, gp::radix_sort_keys(dk.as<uint32_t>(), Wk, Wk, di.as<uint32_t>(), n, dtmp.p, s, bits));
-    GP_CUDA_TRY(c, gp::mark_unique(dk.as<uint32_t>(), Wk, di.as<uint32_t>(), n, Wk, dflag.as<uint32_t>(), s));
-    uint32_t* d_cnt = dord.as<uint32_t>() + n;
-    GP_CUDA_TRY(c, gp::compact_flags(dflag.as<uint32_t>(), di.as<uint32_t>(), dord.as<uint32_t>(), n,
-                                     dpos.as<uint32_t>(), dscan.as<uint32_t>(), d_cnt, s));
-    uint32_t nu = 0;
-    GP_CUDA_TRY(c, cudaMemcpyAsync(&nu, d_cnt, 4, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
-    if (nu == 0) return GP_OK;
-    gather_len_kernel<<<grid_for(nu), 256, 0, s>>>(dl.as<uint32_t>(), dord.as<uint32_t>(), nu, dlen2.as<uint32_t>());
-    GP_CUDA_TRY(c, cudaGetLastError());
-    GP_CUDA_TRY(c, gp::exclusive_scan_u32(dlen2.as<uint32_t>(), dooff.as<uint32_t>(), nu, dscan.as<uint32_t>(), s));
-    uint32_t o_last = 0, l_last = 0;
-    GP_CUDA_TRY(c, cudaMemcpyAsync(&o_last, dooff.as<uint32_t>() + nu - 1, 4, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaMemcpyAsync(&l_last, dlen2.as<uint32_t>() + nu - 1, 4, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
-    const uint64_t out_bytes = (uint64_t)o_last + l_last;
-    if (!dout.ensure(out_bytes + 16)) return c->fail(GP_ERR_NOMEM, "sort: device allocation");
-    gather_lines_kernel<<<(unsigned)std::min<int64_t>((nu + 7) / 8, 65535 * 8), 256, 0, s>>>(
-        dt.as<char>(), ds.as<uint64_t>(), dl.as<uint32_t>(), dord.as<uint32_t>(), dooff.as<uint32_t>(), nu,
-        dout.as<char>());
-    GP_CUDA_TRY(c, cudaGetLastError());
-    out.resize(out_bytes);
-    GP_CUDA_TRY(c, cudaMemcpyAsync(&out[0], dout.p, out_bytes, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
-    return GP_OK;
+    return sort_device_lines(c, dt.as<char>(), ds.as<uint32_t>(), dl.as<uint32_t>(), n, hm[0], true, out_path, s);
 }
 
 extern "C" {
@@ -643,14 +938,48 @@ int gp_tuned_settings(const gp_ctx* c, char* buf, int cap) {
     return (int)t.size() + 1;
 }
 
+// Text inputs of the sort, one after another on the device, each ended by a
+// newline.
+static int sort_files(gp_ctx* c, std::vector<FileText>& files, size_t bytes, const char* out_path) {
+    cudaStream_t s = c->s_comp;
+    DevBuf& dt = c->st[kTbText];
+    if (!dt.ensure(bytes + kTextBlock)) return c->fail(GP_ERR_NOMEM, "sort: device allocation");
+    size_t n = 0;
+    for (FileText& f : files) {
+        if (f.n == 0) continue;
+        GP_CUDA_TRY(c, cudaMemcpyAsync(dt.as<char>() + n, f.p.get(), f.n, cudaMemcpyHostToDevice, s));
+        n += f.n;
+        if (f.p[f.n - 1] != '\n') GP_CUDA_TRY(c, cudaMemsetAsync(dt.as<char>() + n++, '\n', 1, s));
+    }
+    if (n == 0) return write_text(c, nullptr, 0, out_path, s);
+    Lines ln;
+    const int rc = find_lines(c, dt.as<char>(), n, c->st[kTbStart], c->st[kTbLen], ln, s);
+    if (rc) return rc;
+    for (FileText& f : files) f.p.reset();  // find_lines has waited for the copies
+    return sort_device_lines(c, dt.as<char>(), c->st[kTbStart].as<uint32_t>(), c->st[kTbLen].as<uint32_t>(), ln.n,
+                             ln.longest, !ln.other, out_path, s);
+}
+
 static int gp_sort_impl(gp_ctx* c, const char** in_paths, int n_in, const char* out_path) {
     StageRange nvtx_range("gp_sort");
     if (!c || (!in_paths && n_in > 0) || !out_path) return GP_ERR_ARG;
     cudaSetDevice(c->device);
+    KeepSmall keep{c->st};
     // every input is read once
+    std::vector<FileText> files(n_in);
+    size_t bytes = 0;
+    bool text_only = true;
+    for (int i = 0; i < n_in; ++i) {
+        if (!read_file(in_paths[i], files[i])) return c->fail(GP_ERR_IO, "sort: cannot read %s", in_paths[i]);
+        bytes += files[i].n + 1;
+        text_only = text_only && !(files[i].n >= 8 && std::memcmp(files[i].p.get(), gp::kSurvMagic, 8) == 0);
+    }
+    if (text_only && bytes < kMaxDeviceText) return sort_files(c, files, bytes, out_path);
     std::vector<std::string> texts(n_in);
-    for (int i = 0; i < n_in; ++i)
-        if (!slurp(in_paths[i], texts[i])) return c->fail(GP_ERR_IO, "sort: cannot read %s", in_paths[i]);
+    for (int i = 0; i < n_in; ++i) {
+        texts[i].assign(files[i].p.get(), files[i].n);
+        files[i].p.reset();
+    }
     {
         // all inputs binary survivor files of one job: the records are
         // formatted and sorted on the device
@@ -681,13 +1010,7 @@ static int gp_sort_impl(gp_ctx* c, const char** in_paths, int n_in, const char* 
             g.word_bytes = h0.word_bytes;
             g.rec_bytes = (int)gp::surv_record_bytes(h0);
             for (int a = 0; a < 16; ++a) g.alpha[a] = h0.alpha[a];
-            std::string sorted;
-            int rc = gp_sort_records(c, g, recs, n, sorted);
-            if (rc) return rc;
-            FILE* f = fopen(out_path, "w");
-            if (!f) return c->fail(GP_ERR_IO, "sort: cannot write %s", out_path);
-            fwrite(sorted.data(), 1, sorted.size(), f);
-            return fclose(f) == 0 ? GP_OK : c->fail(GP_ERR_IO, "sort: write failed");
+            return gp_sort_records(c, g, recs, n, out_path);
         }
     }
     std::string all;
@@ -724,6 +1047,119 @@ int gp_sort(gp_ctx* c, const char** in_paths, int n_in, const char* out_path) {
     }
 }
 
+// The match on the device: sorted candidate files (every token no greater than
+// the next line's), so the merge on the first token is an equality join: each
+// a line with the b lines of its token, in file order.  *done = false where
+// the host's parser or merge decides: other characters, lines of blanks or
+// with too few integers, unsorted tokens, more text or pairs than 32 bits.
+static int match_files(gp_ctx* c, int L, int target, const FileText& fa, const FileText& fb, FILE* f, int64_t* n_pairs,
+                       bool* done) {
+    *done = false;
+    if (fa.n + 2 > kMaxDeviceText || fb.n + 2 > kMaxDeviceText) return GP_OK;
+    cudaStream_t s = c->s_comp;
+    const FileText* file[2] = {&fa, &fb};
+    DevBuf* text[2] = {&c->st[kTbText], &c->st[kTbTextB]};
+    DevBuf* start[2] = {&c->st[kTbStart], &c->st[kTbStartB]};
+    DevBuf* len[2] = {&c->st[kTbLen], &c->st[kTbLenB]};
+    DevBuf* tok[2] = {&c->st[kTbTokA], &c->st[kTbTokB]};
+    DevBuf* tlen[2] = {&c->st[kTbTokLenA], &c->st[kTbTokLenB]};
+    DevBuf* seqs[2] = {&c->st[kTbSeqA], &c->st[kTbSeqB]};
+    DevBuf* paf[2] = {&c->st[kTbPafA], &c->st[kTbPafB]};
+    DevBuf& misc = c->st[kTbMisc];
+    const int H = L / 2;
+    Lines ln[2];
+    for (int k = 0; k < 2; ++k) {
+        size_t n = file[k]->n;
+        if (!text[k]->ensure(n + 1 + kTextBlock)) return c->fail(GP_ERR_NOMEM, "match: device allocation");
+        GP_CUDA_TRY(c, cudaMemcpyAsync(text[k]->p, file[k]->p.get(), n, cudaMemcpyHostToDevice, s));
+        if (file[k]->p[n - 1] != '\n') GP_CUDA_TRY(c, cudaMemsetAsync(text[k]->as<char>() + n++, '\n', 1, s));
+        const int rc = find_lines(c, text[k]->as<char>(), n, *start[k], *len[k], ln[k], s);
+        if (rc) return rc;
+        if (ln[k].other) return GP_OK;
+    }
+    int* d_bad = misc.as<int>() + 2;
+    unsigned long long* d_total = misc.as<unsigned long long>() + 2;
+    GP_CUDA_TRY(c, cudaMemsetAsync(misc.p, 0, 64, s));
+    for (int k = 0; k < 2; ++k) {
+        const int64_t n = ln[k].n;
+        if (!tok[k]->ensure(n * 4) || !tlen[k]->ensure(n * 4) || !seqs[k]->ensure((size_t)n * L + 16) ||
+            !paf[k]->ensure((size_t)n * (H + 1) * 4))
+            return c->fail(GP_ERR_NOMEM, "match: device allocation");
+        parse_lines_kernel<<<grid_for(n), 256, 0, s>>>(text[k]->as<char>(), start[k]->as<uint32_t>(),
+                                                       len[k]->as<uint32_t>(), n, L, tok[k]->as<uint32_t>(),
+                                                       tlen[k]->as<uint32_t>(), seqs[k]->as<int8_t>(), d_bad);
+        tokens_sorted_kernel<<<grid_for(n), 256, 0, s>>>(text[k]->as<char>(), tok[k]->as<uint32_t>(),
+                                                         tlen[k]->as<uint32_t>(), n, d_bad);
+        GP_CUDA_TRY(c, cudaGetLastError());
+    }
+    const int64_t na = ln[0].n;
+    DevBuf &db0 = c->st[kTbOutLen], &dnb = c->st[kTbFlag], &dfirst = c->st[kTbOutOff], &dscan = c->st[kTbScan];
+    if (!db0.ensure(na * 4) || !dnb.ensure(na * 4) || !dfirst.ensure(na * 4) || !dscan.ensure(gp::scan_tmp_bytes(na)))
+        return c->fail(GP_ERR_NOMEM, "match: device allocation");
+    token_ranges_kernel<<<grid_for(na), 256, 0, s>>>(text[0]->as<char>(), tok[0]->as<uint32_t>(), tlen[0]->as<uint32_t>(),
+                                                     na, text[1]->as<char>(), tok[1]->as<uint32_t>(),
+                                                     tlen[1]->as<uint32_t>(), ln[1].n, db0.as<uint32_t>(),
+                                                     dnb.as<uint32_t>(), d_total);
+    GP_CUDA_TRY(c, cudaGetLastError());
+    GP_CUDA_TRY(c, gp::exclusive_scan_u32(dnb.as<uint32_t>(), dfirst.as<uint32_t>(), na, dscan.as<uint32_t>(), s));
+    unsigned long long h[8];
+    GP_CUDA_TRY(c, cudaMemcpyAsync(h, misc.p, 64, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    if ((int)(uint32_t)h[1] || h[2] >= (1ull << 31)) return GP_OK;
+    *done = true;
+    const int64_t total = (int64_t)h[2];
+    if (n_pairs) *n_pairs = 0;
+    if (total == 0) return GP_OK;
+    DevBuf &df = c->st[kTbKeys], &dpos = c->st[kTbPos], &dkeep = c->st[kTbOrder], &dia = c->st[kTbIa],
+           &dib = c->st[kTbIb];
+    if (!df.ensure((size_t)total * 4) || !dpos.ensure((size_t)total * 4) || !dkeep.ensure((size_t)total * 4 + 4) ||
+        !dia.ensure((size_t)total * 4) || !dib.ensure((size_t)total * 4) || !dscan.ensure(gp::scan_tmp_bytes(total)))
+        return c->fail(GP_ERR_NOMEM, "match: device allocation");
+    if (H > 0)
+        for (int k = 0; k < 2; ++k)
+            paf_kernel<<<grid_for(ln[k].n), 256, 0, s>>>(seqs[k]->as<int8_t>(), ln[k].n, L, H, paf[k]->as<int>());
+    range_check_kernel<<<grid_for(total), 256, 0, s>>>(dfirst.as<uint32_t>(), db0.as<uint32_t>(), na, (uint32_t)total,
+                                                       paf[0]->as<int>(), paf[1]->as<int>(), H, target,
+                                                       df.as<uint32_t>(), dia.as<uint32_t>(), dib.as<uint32_t>());
+    GP_CUDA_TRY(c, cudaGetLastError());
+    uint32_t* d_cnt = dkeep.as<uint32_t>() + total;
+    GP_CUDA_TRY(c, gp::compact_flags(df.as<uint32_t>(), nullptr, dkeep.as<uint32_t>(), total, dpos.as<uint32_t>(),
+                                     dscan.as<uint32_t>(), d_cnt, s));
+    uint32_t nk = 0;
+    GP_CUDA_TRY(c, cudaMemcpyAsync(&nk, d_cnt, 4, cudaMemcpyDeviceToHost, s));
+    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    // the kept pairs' lines, blocks of them below 2^31 bytes (five a value at most)
+    DevBuf &dbytes = c->st[kTbFlag], &dat = c->st[kTbPos], &dout = c->st[kTbOut];
+    const int64_t step = std::min<int64_t>(nk, (int64_t(1) << 31) / (10 * L + 2));
+    if (nk && (!dbytes.ensure((size_t)step * 4) || !dat.ensure((size_t)step * 4)))
+        return c->fail(GP_ERR_NOMEM, "match: device allocation");
+    for (int64_t k0 = 0; k0 < nk; k0 += step) {
+        const int64_t n = std::min<int64_t>(step, nk - k0);
+        const uint32_t* keep = dkeep.as<uint32_t>() + k0;
+        match_line_bytes_kernel<<<grid_for(n), 256, 0, s>>>(seqs[0]->as<int8_t>(), seqs[1]->as<int8_t>(),
+                                                            dia.as<uint32_t>(), dib.as<uint32_t>(), keep, n, L,
+                                                            dbytes.as<uint32_t>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        GP_CUDA_TRY(c, gp::exclusive_scan_u32(dbytes.as<uint32_t>(), dat.as<uint32_t>(), n, dscan.as<uint32_t>(), s));
+        uint32_t last[2] = {0, 0};
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&last[0], dat.as<uint32_t>() + n - 1, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&last[1], dbytes.as<uint32_t>() + n - 1, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+        const size_t bytes = (size_t)last[0] + last[1];
+        if (!dout.ensure(bytes + 1)) return c->fail(GP_ERR_NOMEM, "match: device allocation");
+        match_lines_kernel<<<(unsigned)std::min<int64_t>((n + 7) / 8, 65535 * 8), 256, 0, s>>>(
+            seqs[0]->as<int8_t>(), seqs[1]->as<int8_t>(), dia.as<uint32_t>(), dib.as<uint32_t>(), keep, n, L,
+            dat.as<uint32_t>(), dout.as<char>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        std::unique_ptr<char[]> out(new char[bytes + 1]);
+        GP_CUDA_TRY(c, cudaMemcpyAsync(out.get(), dout.p, bytes, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+        fwrite(out.get(), 1, bytes, f);
+    }
+    if (n_pairs) *n_pairs = nk;
+    return GP_OK;
+}
+
 static int gp_match_impl(gp_ctx* c, int order, int compress, int paf, const char* path_a, const char* path_b, const char* out_path,
              int append, int64_t* n_pairs) {
     StageRange nvtx_range("gp_match");
@@ -734,14 +1170,24 @@ static int gp_match_impl(gp_ctx* c, int order, int compress, int paf, const char
     // before looking at the inputs (src/main.cpp:97-101)
     FILE* f = fopen(out_path, append ? "a" : "w");
     if (!f) return c->fail(GP_ERR_IO, "match: cannot open %s", out_path);
-    std::string ta, tb, out;
-    const bool okA = slurp(path_a, ta), okB = slurp(path_b, tb);
+    KeepSmall keep{c->st};
+    FileText fa, fb;
+    const bool okA = read_file(path_a, fa), okB = read_file(path_b, fb);
     if (n_pairs) *n_pairs = 0;
-    if (!okA || !okB || ta.empty() || tb.empty()) {
+    if (!okA || !okB || fa.n == 0 || fb.n == 0) {
         fclose(f);
         return GP_EMPTY_INPUT;
     }
-    int rc = gp_match_texts(c, order / compress, compress, paf, ta, tb, out, n_pairs);
+    bool done = false;
+    int rc = match_files(c, order / compress, paf * compress, fa, fb, f, n_pairs, &done);
+    if (done || rc) {
+        fclose(f);
+        return rc;
+    }
+    std::string ta(fa.p.get(), fa.n), tb(fb.p.get(), fb.n), out;
+    fa.p.reset();
+    fb.p.reset();
+    rc = gp_match_texts(c, order / compress, compress, paf, ta, tb, out, n_pairs);
     fwrite(out.data(), 1, out.size(), f);
     fclose(f);
     return rc;

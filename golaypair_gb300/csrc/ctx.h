@@ -77,6 +77,21 @@ struct HostPinned {
     }
 };
 
+// At the end of a stage call: gives back the buffers of an array that are
+// larger than a few calls' allocations are worth (64 MB each).
+struct KeepSmall {
+    DevBuf* b;
+    size_t n;
+    template <size_t N>
+    explicit KeepSmall(DevBuf (&bufs)[N]) : b(bufs), n(N) {}
+    ~KeepSmall() {
+        for (size_t i = 0; i < n; ++i)
+            if (b[i].cap > (size_t(64) << 20)) b[i].release();
+    }
+    KeepSmall(const KeepSmall&) = delete;
+    KeepSmall& operator=(const KeepSmall&) = delete;
+};
+
 // An NVTX range over one stage call, named for the entry point: the stages
 // show on a profiler's timeline (no cost without a tool attached).
 struct StageRange {
@@ -138,7 +153,8 @@ struct gp_ctx {
     // grow-only scratch of the uncompression stage (kept across pairs: a
     // cudaFree per pair would synchronise the device every pair)
     DevBuf ux[66];
-    DevBuf eq[20];  // grow-only scratch of the equivalence filter
+    DevBuf eq[20];  // scratch of the equivalence filter, and of sort and match:
+    DevBuf st[29];  // kept between calls while small (KeepSmall)
     HostPinned hscratch[4];
     // batched generation: one stream per job branch, fork/join events
     static constexpr int kJobStreams = 8;
