@@ -671,7 +671,7 @@ enum EqBuf { kEqText, kEqCount, kEqOffs, kEqScan, kEqVals, kEqInfo, kEqCode, kEq
 int sort_rows(PairSet& ps, const int8_t* rows, int64_t n, uint32_t* idx, uint32_t* flags, cudaStream_t s) {
     gp_ctx* c = ps.c;
     DevBuf &keys = c->eq[kEqKeys], &tmp = c->eq[kEqTmp];
-    if (!keys.ensure((size_t)n * ps.Wk * 4) || !tmp.ensure(gp::radix_sort_tmp_bytes(n)))
+    if (!keys.ensure((size_t)n * ps.Wk * 4) || !tmp.ensure(gp::radix_sort_tmp_bytes(n, ps.Wk)))
         return c->fail(GP_ERR_NOMEM, "equivalence filter: sort buffers");
     pair_keys_kernel<<<grid_of(n * ps.Wk, 256), 256, 0, s>>>(rows, n, ps.W, ps.code, ps.bits, ps.Wk,
                                                              keys.as<uint32_t>());

@@ -673,7 +673,7 @@ int gp_sort_text(gp_ctx* c, const std::string& text, std::string& out) {
     cudaStream_t s = c->s_comp;
     DevBuf dt, ds, dl, dk, di, dtmp, dflag, dpos, dscan, dout;
     if (!dt.ensure(text.size() + 16) || !ds.ensure(n * 8) || !dl.ensure(n * 4) || !dk.ensure((size_t)n * Wk * 4) ||
-        !di.ensure(n * 4) || !dtmp.ensure(gp::radix_sort_tmp_bytes(n)) || !dflag.ensure(n * 4) || !dpos.ensure(n * 4) ||
+        !di.ensure(n * 4) || !dtmp.ensure(gp::radix_sort_tmp_bytes(n, Wk)) || !dflag.ensure(n * 4) || !dpos.ensure(n * 4) ||
         !dscan.ensure(gp::scan_tmp_bytes(n)) || !dout.ensure(n * 4 + 4))
         return c->fail(GP_ERR_NOMEM, "sort: device allocation");
     GP_CUDA_TRY(c, cudaMemcpyAsync(dt.p, text.data(), text.size(), cudaMemcpyHostToDevice, s));
@@ -855,7 +855,7 @@ int sort_device_lines(gp_ctx* c, const char* d_text, const uint32_t* d_start, co
     DevBuf &dk = c->st[kTbKeys], &di = c->st[kTbIdx], &dtmp = c->st[kTbTmp], &dflag = c->st[kTbFlag],
            &dpos = c->st[kTbPos], &dord = c->st[kTbOrder], &dlen2 = c->st[kTbOutLen], &dooff = c->st[kTbOutOff],
            &dout = c->st[kTbOut], &dscan = c->st[kTbScan];
-    if (!dk.ensure((size_t)n * Wk * 4) || !di.ensure(n * 4) || !dtmp.ensure(gp::radix_sort_tmp_bytes(n)) ||
+    if (!dk.ensure((size_t)n * Wk * 4) || !di.ensure(n * 4) || !dtmp.ensure(gp::radix_sort_tmp_bytes(n, Wk)) ||
         !dflag.ensure(n * 4) || !dpos.ensure(n * 4) || !dord.ensure(n * 4 + 4) || !dlen2.ensure(n * 4) ||
         !dooff.ensure(n * 4) || !dscan.ensure(gp::scan_tmp_bytes(n)))
         return c->fail(GP_ERR_NOMEM, "sort: device allocation");

@@ -4,9 +4,13 @@
 // Keys are rows of W 32-bit words, word 0 most significant.  The sort
 // permutes a uint32 index array (keys stay in place and are gathered per
 // pass), 4 or 8 bits per pass (the sort's tuner picks); a pass whose digit
-// is the same for every key is skipped (its histogram has a single non-empty
-// bucket).
+// is the same for every key is skipped.  One kernel counts every digit of every
+// key first, so the passes run without waiting for the host in between, and a
+// pass is two launches (block histograms, scatter) up to kScatterScanBlocks
+// blocks: the scatter sums the blocks before its own.
+#include <algorithm>
 #include <cstdio>
+#include <type_traits>
 #include <vector>
 
 #include "prims.h"
@@ -62,17 +66,55 @@ __global__ void compact_kernel(const uint32_t* flags, const uint32_t* pos, const
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int64_t kScatterScanBlocks = 256;  // 2^19 keys
 
 template <int RB>
 __device__ __forceinline__ uint32_t key_digit(const uint32_t* keys, int W, uint32_t idx, int word, int shift) {
     return (keys[(int64_t)idx * W + word] >> shift) & ((1u << RB) - 1u);
 }
 
-// RB bits per pass: 2^RB buckets (RB <= 8, so one thread per bucket).
+// Every digit's counts over the keys of rows [0, n): total[digit * NB + d]
+// for digit = 0 (the last word's low bits) .. (32 / RB) W - 1.  One block row
+// (blockIdx.y) per word.
 template <int RB>
+__global__ void __launch_bounds__(kSortThreads) radix_totals_kernel(const uint32_t* keys, int W, int sort_words,
+                                                                    int64_t n, uint32_t* total) {
+    constexpr int NB = 1 << RB, ND = 32 / RB;
+    __shared__ uint32_t h[ND * NB];
+    for (int word = blockIdx.y; word < sort_words; word += gridDim.y) {
+        for (int i = threadIdx.x; i < ND * NB; i += kSortThreads) h[i] = 0;
+        __syncthreads();
+        for (int64_t i0 = (int64_t)blockIdx.x * kSortThreads; i0 < n; i0 += (int64_t)gridDim.x * kSortThreads) {
+            const int64_t i = i0 + threadIdx.x;
+            const bool has = i < n;
+            const uint32_t k = has ? keys[i * W + word] : 0u;
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                // most keys share a digit: one addition for a warp that agrees
+                const uint32_t x = has ? (k >> (RB * d)) & (NB - 1u) : 0x100u;
+                int same;
+                __match_all_sync(0xFFFFFFFFu, x, &same);
+                if (same) {
+                    if (has && (threadIdx.x & 31) == 0) atomicAdd(&h[d * NB + x], 32u);
+                } else if (has) {
+                    atomicAdd(&h[d * NB + x], 1u);
+                }
+            }
+        }
+        __syncthreads();
+        const int first = (sort_words - 1 - word) * ND;
+        for (int i = threadIdx.x; i < ND * NB; i += kSortThreads)
+            if (h[i]) atomicAdd(&total[(int64_t)first * NB + i], h[i]);
+        __syncthreads();
+    }
+}
+
+// RB bits per pass: 2^RB buckets (RB <= 8, so one thread per bucket).
+// counts: by block, then bucket (ROWS), or by bucket, then block.
+template <int RB, bool ROWS>
 __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint32_t* keys, int W, const uint32_t* idx,
                                                                    int64_t n, int word, int shift, uint32_t* counts,
-                                                                   int64_t nblocks, uint32_t* total) {
+                                                                   int64_t nblocks) {
     constexpr int NB = 1 << RB;
     __shared__ uint32_t h[NB];
     if (threadIdx.x < NB) h[threadIdx.x] = 0;
@@ -83,22 +125,44 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint32_t
         if (i < n) atomicAdd(&h[key_digit<RB>(keys, W, idx[i], word, shift)], 1u);
     }
     __syncthreads();
-    if (threadIdx.x < NB) {
-        const uint32_t c = h[threadIdx.x];
-        counts[(int64_t)threadIdx.x * nblocks + blockIdx.x] = c;
-        if (c) atomicAdd(&total[threadIdx.x], c);
-    }
+    if (threadIdx.x < NB)
+        counts[ROWS ? (int64_t)blockIdx.x * NB + threadIdx.x : (int64_t)threadIdx.x * nblocks + blockIdx.x] =
+            h[threadIdx.x];
 }
 
-template <int RB>
+// ROWS: the buckets' first places are the digit's totals before them plus the
+// counts of the blocks before this one; otherwise offsets has been scanned.
+template <int RB, bool ROWS>
 __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(const uint32_t* keys, int W, const uint32_t* idx_in,
                                                                       uint32_t* idx_out, int64_t n, int word, int shift,
-                                                                      const uint32_t* offsets, int64_t nblocks) {
+                                                                      const uint32_t* offsets, int64_t nblocks,
+                                                                      const uint32_t* total) {
     constexpr int NB = 1 << RB;
     __shared__ uint32_t base[NB];
     __shared__ uint32_t wh[kSortThreads / 32][NB];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x < NB) base[threadIdx.x] = offsets[(int64_t)threadIdx.x * nblocks + blockIdx.x];
+    if constexpr (ROWS) {
+        uint32_t before = 0;
+        if (threadIdx.x < NB) {
+#pragma unroll 8
+            for (int64_t b = 0; b < (int64_t)blockIdx.x; ++b) before += offsets[b * NB + threadIdx.x];
+        }
+        const uint32_t t = threadIdx.x < NB ? total[threadIdx.x] : 0u;
+        uint32_t x = t;  // inclusive scan of the totals over the block
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wh[0][warp] = x;
+        __syncthreads();
+        uint32_t warps = 0;
+        for (int q = 0; q < warp; ++q) warps += wh[0][q];
+        __syncthreads();
+        if (threadIdx.x < NB) base[threadIdx.x] = warps + x - t + before;
+    } else if (threadIdx.x < NB) {
+        base[threadIdx.x] = offsets[(int64_t)threadIdx.x * nblocks + blockIdx.x];
+    }
     const int64_t tile0 = (int64_t)blockIdx.x * kSortTile;
     for (int k = 0; k < kSortItems; ++k) {
         if (threadIdx.x < NB)
@@ -208,22 +272,23 @@ cudaError_t iota_u32(uint32_t* p, int64_t n, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-size_t radix_sort_tmp_bytes(int64_t n) {
+size_t radix_sort_tmp_bytes(int64_t n, int sort_words) {
     const int64_t nb = (n + kSortTile - 1) / kSortTile;
     return (size_t)n * 4                      // ping-pong index
            + (size_t)nb * 256 * 4 * 2         // counts + offsets
-           + scan_tmp_bytes(nb * 256) + 256 * 4 + 1024;
+           + scan_tmp_bytes(nb * 256) + (size_t)sort_words * 4096 + 1024;
 }
 
 // Sorts idx (a permutation of row numbers) by the keys' first `sort_words`
-// words (of W).  Stable.  tmp: radix_sort_tmp_bytes(n) bytes of device memory.
+// words (of W).  Stable.  tmp: radix_sort_tmp_bytes(n, sort_words) bytes of device memory.
 // radix_bits: 4 or 8 bits per pass.
 cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_t* idx, int64_t n, void* tmp,
                             cudaStream_t st, int radix_bits) {
-    if (n <= 1) return cudaSuccess;
+    if (n <= 1 || sort_words < 1) return cudaSuccess;
     if (radix_bits != 4 && radix_bits != 8) return cudaErrorInvalidValue;
     const int NB = 1 << radix_bits;
     const int per_word = 32 / radix_bits;
+    const int digits = per_word * sort_words;
     const int64_t nb = (n + kSortTile - 1) / kSortTile;
     uint8_t* t = static_cast<uint8_t*>(tmp);
     uint32_t* alt = reinterpret_cast<uint32_t*>(t);
@@ -232,36 +297,49 @@ cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_
     t += (size_t)nb * 256 * 4;
     uint32_t* offs = reinterpret_cast<uint32_t*>(t);
     t += (size_t)nb * 256 * 4;
-    uint32_t* total = reinterpret_cast<uint32_t*>(t);
-    t += 256 * 4;
     t = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(t) + 255) & ~uintptr_t(255));
     uint32_t* stmp = reinterpret_cast<uint32_t*>(t);
+    // every digit's totals (at most 4 KB a word), read back once
+    uint32_t* total = stmp;
+    stmp += (size_t)sort_words * 1024;
+    cudaError_t e = cudaMemsetAsync(total, 0, (size_t)digits * NB * 4, st);
+    if (e != cudaSuccess) return e;
+    const dim3 tg((unsigned)std::min<int64_t>((n + kSortThreads - 1) / kSortThreads, 1216), (unsigned)std::min(sort_words, 65535));
+    if (radix_bits == 8)
+        radix_totals_kernel<8><<<tg, kSortThreads, 0, st>>>(keys, W, sort_words, n, total);
+    else
+        radix_totals_kernel<4><<<tg, kSortThreads, 0, st>>>(keys, W, sort_words, n, total);
+    std::vector<uint32_t> htotal((size_t)digits * NB);
+    e = cudaMemcpyAsync(htotal.data(), total, htotal.size() * 4, cudaMemcpyDeviceToHost, st);
+    if (e != cudaSuccess) return e;
+    e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    const bool rows = nb <= kScatterScanBlocks;
     uint32_t* cur = idx;
     uint32_t* nxt = alt;
-    std::vector<uint32_t> htotal(NB);
-    for (int bi = 0; bi < per_word * sort_words; ++bi) {
+    for (int bi = 0; bi < digits; ++bi) {
+        int nonempty = 0;
+        for (int d = 0; d < NB; ++d) nonempty += htotal[(size_t)bi * NB + d] != 0;
+        if (nonempty <= 1) continue;  // every key has the same digit here
         const int word = sort_words - 1 - bi / per_word;
         const int shift = radix_bits * (bi % per_word);
-        cudaError_t e = cudaMemsetAsync(total, 0, NB * 4, st);
-        if (e != cudaSuccess) return e;
-        if (radix_bits == 8)
-            radix_hist_kernel<8><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb, total);
-        else
-            radix_hist_kernel<4><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb, total);
-        e = cudaMemcpyAsync(htotal.data(), total, NB * 4, cudaMemcpyDeviceToHost, st);
-        if (e != cudaSuccess) return e;
-        e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) return e;
-        int nonempty = 0;
-        for (uint32_t c : htotal) nonempty += c != 0;
-        if (nonempty <= 1) continue;  // every key has the same digit here
-        e = exclusive_scan_u32(counts, offs, nb * NB, stmp, st);
-        if (e != cudaSuccess) return e;
-        if (radix_bits == 8)
-            radix_scatter_kernel<8><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift, offs, nb);
-        else
-            radix_scatter_kernel<4><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift, offs, nb);
-        e = cudaGetLastError();
+        const uint32_t* tot = total + (size_t)bi * NB;
+        auto pass = [&](auto rb) {
+            constexpr int RB = decltype(rb)::value;
+            if (rows) {
+                radix_hist_kernel<RB, true><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb);
+                radix_scatter_kernel<RB, true><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift,
+                                                                                      counts, nb, tot);
+                return cudaGetLastError();
+            }
+            radix_hist_kernel<RB, false><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb);
+            const cudaError_t se = exclusive_scan_u32(counts, offs, nb * NB, stmp, st);
+            if (se != cudaSuccess) return se;
+            radix_scatter_kernel<RB, false><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift,
+                                                                                   offs, nb, tot);
+            return cudaGetLastError();
+        };
+        e = radix_bits == 8 ? pass(std::integral_constant<int, 8>{}) : pass(std::integral_constant<int, 4>{});
         if (e != cudaSuccess) return e;
         uint32_t* sw = cur;
         cur = nxt;

@@ -18,7 +18,7 @@ cudaError_t compact_flags(const uint32_t* flags, const uint32_t* src, uint32_t* 
 cudaError_t mark_unique(const uint32_t* keys, int W, const uint32_t* idx, int64_t n, int cmp_words, uint32_t* flags,
                         cudaStream_t st);
 cudaError_t iota_u32(uint32_t* p, int64_t n, cudaStream_t st);
-size_t radix_sort_tmp_bytes(int64_t n);
+size_t radix_sort_tmp_bytes(int64_t n, int sort_words);
 cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_t* idx, int64_t n, void* tmp,
                             cudaStream_t st, int radix_bits = 8);
 
