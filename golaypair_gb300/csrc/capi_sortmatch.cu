@@ -132,7 +132,7 @@ unsigned grid_for(int64_t n) {
 // A file's bytes go to the device as they are; its lines are found, keyed,
 // compared and written out there.  Offsets are 32 bits: more text than that
 // takes the host's line index (gp_sort_text, gp_match_texts).  Sort and match
-// of the 430,000 lines of a whole order 51: 13.7 ms, 43.3 with the lines, the
+// of the 430,000 lines of a whole order 51: 10.6 ms, 43.3 with the lines, the
 // parse, the merge and the copies on host threads.
 constexpr int kTextThreads = 256;
 constexpr int kTextEach = 16;                            // bytes per thread

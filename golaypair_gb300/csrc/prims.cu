@@ -8,9 +8,14 @@
 // key first, so the passes run without waiting for the host in between, and a
 // pass is two launches (block histograms, scatter) up to kScatterScanBlocks
 // blocks: the scatter sums the blocks before its own.
+// The passes take the leading digits only, as many as hold twice the entropy
+// that n distinct rows need; rows that still agree stand next to each other
+// then and are ranked by whole keys, unless more than kRunMax of them do.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "prims.h"
@@ -67,6 +72,8 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int64_t kScatterScanBlocks = 256;  // 2^19 keys
+constexpr int kRunMax = 32;
+constexpr int kTailPasses = 4;  // about what the two kernels for runs and the wait cost
 
 template <int RB>
 __device__ __forceinline__ uint32_t key_digit(const uint32_t* keys, int W, uint32_t idx, int word, int shift) {
@@ -194,6 +201,51 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(const uint3
     }
 }
 
+// The leading digits of row i and row j agree: words before w, and mask of w.
+__device__ __forceinline__ bool same_lead(const uint32_t* keys, int W, uint32_t i, uint32_t j, int w, uint32_t mask) {
+    const uint32_t *a = keys + (int64_t)i * W, *b = keys + (int64_t)j * W;
+    if ((a[w] ^ b[w]) & mask) return false;
+    for (int k = w - 1; k >= 0; --k)
+        if (a[k] != b[k]) return false;
+    return true;
+}
+
+// first[p]: the p-th row in order starts a run of equal leading digits;
+// *longer: some run has more than kRunMax rows.
+__global__ void run_starts_kernel(const uint32_t* keys, int W, const uint32_t* idx, int64_t n, int w, uint32_t mask,
+                                  uint8_t* first, int* longer) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t i = idx[p];
+        const bool same = p > 0 && same_lead(keys, W, i, idx[p - 1], w, mask);
+        first[p] = same ? 0 : 1;
+        if (same && p >= kRunMax && same_lead(keys, W, i, idx[p - kRunMax], w, mask)) *longer = 1;
+    }
+}
+
+// Each row of a run goes to its place among the run's rows, by the words from
+// w on, equal rows in the order they stand in.
+__global__ void run_rank_kernel(const uint32_t* keys, int W, int sort_words, const uint32_t* idx, int64_t n, int w,
+                                const uint8_t* first, uint32_t* out) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t i = idx[p];
+        int64_t at = p;
+        const uint32_t* a = keys + (int64_t)i * W;
+        for (int64_t q = p; !first[q];) {  // rows before it that are greater
+            const uint32_t* b = keys + (int64_t)idx[--q] * W;
+            int k = w;
+            while (k < sort_words && a[k] == b[k]) ++k;
+            if (k < sort_words && a[k] < b[k]) --at;
+        }
+        for (int64_t q = p + 1; q < n && !first[q]; ++q) {  // rows after it that are less
+            const uint32_t* b = keys + (int64_t)idx[q] * W;
+            int k = w;
+            while (k < sort_words && a[k] == b[k]) ++k;
+            if (k < sort_words && b[k] < a[k]) ++at;
+        }
+        out[at] = i;
+    }
+}
+
 __global__ void iota_kernel(uint32_t* p, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         p[i] = (uint32_t)i;
@@ -300,9 +352,10 @@ cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_
     t = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(t) + 255) & ~uintptr_t(255));
     uint32_t* stmp = reinterpret_cast<uint32_t*>(t);
     // every digit's totals (at most 4 KB a word), read back once
-    uint32_t* total = stmp;
-    stmp += (size_t)sort_words * 1024;
-    cudaError_t e = cudaMemsetAsync(total, 0, (size_t)digits * NB * 4, st);
+    int* longer = reinterpret_cast<int*>(stmp);
+    uint32_t* total = stmp + 16;
+    stmp += 16 + (size_t)sort_words * 1024;
+    cudaError_t e = cudaMemsetAsync(longer, 0, 64 + (size_t)digits * NB * 4, st);
     if (e != cudaSuccess) return e;
     const dim3 tg((unsigned)std::min<int64_t>((n + kSortThreads - 1) / kSortThreads, 1216), (unsigned)std::min(sort_words, 65535));
     if (radix_bits == 8)
@@ -314,36 +367,83 @@ cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_
     if (e != cudaSuccess) return e;
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
+    // Digits that differ, and the leading ones [lead, digits) that the first
+    // passes sort by.  Digits that go together (a candidate's spectrum) hold
+    // less than the sum of their entropies, hence twice log2 n; 43 passes of
+    // an order-51 file of 380,000 lines become 7 (35 us each there).
+    std::vector<char> varies(digits, 0);
+    int lead = 0, below = 0;
+    double entropy = 0.0;
+    for (int bi = digits - 1; bi >= 0; --bi) {
+        double h = 0.0;
+        for (int d = 0; d < NB; ++d) {
+            const uint32_t c = htotal[(size_t)bi * NB + d];
+            if (c == 0 || c == (uint32_t)n) continue;
+            varies[bi] = 1;
+            h -= (double)c / (double)n * std::log2((double)c / (double)n);
+        }
+        if (entropy >= 2.0 * std::log2((double)n)) {
+            below += varies[bi];
+        } else {
+            entropy += h;
+            lead = bi;
+        }
+    }
+    if (below <= kTailPasses) lead = below = 0;
     const bool rows = nb <= kScatterScanBlocks;
     uint32_t* cur = idx;
     uint32_t* nxt = alt;
-    for (int bi = 0; bi < digits; ++bi) {
-        int nonempty = 0;
-        for (int d = 0; d < NB; ++d) nonempty += htotal[(size_t)bi * NB + d] != 0;
-        if (nonempty <= 1) continue;  // every key has the same digit here
-        const int word = sort_words - 1 - bi / per_word;
-        const int shift = radix_bits * (bi % per_word);
-        const uint32_t* tot = total + (size_t)bi * NB;
-        auto pass = [&](auto rb) {
-            constexpr int RB = decltype(rb)::value;
-            if (rows) {
-                radix_hist_kernel<RB, true><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb);
-                radix_scatter_kernel<RB, true><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift,
-                                                                                      counts, nb, tot);
+    auto sort_by = [&](int from) {
+        for (int bi = from; bi < digits; ++bi) {
+            if (!varies[bi]) continue;  // every key has the same digit here
+            const int word = sort_words - 1 - bi / per_word;
+            const int shift = radix_bits * (bi % per_word);
+            const uint32_t* tot = total + (size_t)bi * NB;
+            auto pass = [&](auto rb) {
+                constexpr int RB = decltype(rb)::value;
+                if (rows) {
+                    radix_hist_kernel<RB, true><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb);
+                    radix_scatter_kernel<RB, true><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift,
+                                                                                          counts, nb, tot);
+                    return cudaGetLastError();
+                }
+                radix_hist_kernel<RB, false><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb);
+                const cudaError_t se = exclusive_scan_u32(counts, offs, nb * NB, stmp, st);
+                if (se != cudaSuccess) return se;
+                radix_scatter_kernel<RB, false><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift,
+                                                                                       offs, nb, tot);
                 return cudaGetLastError();
-            }
-            radix_hist_kernel<RB, false><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, n, word, shift, counts, nb);
-            const cudaError_t se = exclusive_scan_u32(counts, offs, nb * NB, stmp, st);
-            if (se != cudaSuccess) return se;
-            radix_scatter_kernel<RB, false><<<(unsigned)nb, kSortThreads, 0, st>>>(keys, W, cur, nxt, n, word, shift,
-                                                                                   offs, nb, tot);
-            return cudaGetLastError();
-        };
-        e = radix_bits == 8 ? pass(std::integral_constant<int, 8>{}) : pass(std::integral_constant<int, 4>{});
+            };
+            const cudaError_t pe =
+                radix_bits == 8 ? pass(std::integral_constant<int, 8>{}) : pass(std::integral_constant<int, 4>{});
+            if (pe != cudaSuccess) return pe;
+            std::swap(cur, nxt);
+        }
+        return cudaSuccess;
+    };
+    e = sort_by(lead);
+    if (e != cudaSuccess) return e;
+    if (below) {
+        const int w = sort_words - 1 - lead / per_word;
+        const uint32_t mask = ~0u << (radix_bits * (lead % per_word));
+        uint8_t* first = reinterpret_cast<uint8_t*>(counts);  // counts and offs: a byte per row at least
+        run_starts_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys, W, cur, n, w, mask, first, longer);
+        e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        uint32_t* sw = cur;
-        cur = nxt;
-        nxt = sw;
+        int hlonger = 0;
+        e = cudaMemcpyAsync(&hlonger, longer, 4, cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) return e;
+        e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return e;
+        if (hlonger) {
+            // rows with equal keys still stand in their first order
+            e = sort_by(0);
+        } else {
+            run_rank_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys, W, sort_words, cur, n, w, first, nxt);
+            e = cudaGetLastError();
+            std::swap(cur, nxt);
+        }
+        if (e != cudaSuccess) return e;
     }
     if (cur != idx) return cudaMemcpyAsync(idx, cur, (size_t)n * 4, cudaMemcpyDeviceToDevice, st);
     return cudaSuccess;

@@ -97,3 +97,26 @@ def test_match_matches_oracle(oracle_lib, tmp_path, name, a, b):
     assert rc == orc == 0 and n.value == m.value
     with open(got, "rb") as f, open(want, "rb") as g:
         assert f.read() == g.read()
+
+
+@pytest.mark.parametrize("rows,run,chars", [
+    (2, 2, "09"), (31, 1, "0123456789"), (4096, 31, "0123456789"), (4096, 32, "0123456789"),
+    (4100, 33, "0123456789"), (4096, 1024, "-0123456789"), (6000, 32, "abcdefghAB"), (20000, 2, " 1"),
+    (2**19 + 5, 1, "0123456789"), (2**19, 2, "0123456789"),
+])
+def test_sort_of_lines_with_equal_starts(oracle_lib, tmp_path, rows, run, chars):
+    """Runs of lines whose first 24 characters agree, a quarter of them whole."""
+    rng = np.random.default_rng(rows + run)
+    c = np.frombuffer(chars.encode(), np.uint8)
+    lead = np.repeat(rng.choice(c, (-(-rows // run), 24)), run, axis=0)[:rows]
+    tail = rng.choice(c, (rows, 17))
+    same = rng.random(rows) < 0.25
+    tail[same] = tail[0]
+    rng.shuffle(text := np.concatenate([lead, tail, np.full((rows, 1), 10, np.uint8)], axis=1))
+    (tmp_path / "in").write_bytes(text.tobytes())
+    arr = (ctypes.c_char_p * 1)(str(tmp_path / "in").encode())
+    got, want = str(tmp_path / "got").encode(), str(tmp_path / "want").encode()
+    with gp.Context(0) as ctx:
+        ctx.check(ctx._lib.gp_sort(ctx.handle, ctypes.cast(arr, ctypes.c_void_p), 1, got), "gp_sort")
+    assert oracle_lib.gpo_sort(ctypes.cast(arr, ctypes.c_void_p), 1, want) == 0
+    assert (tmp_path / "got").read_bytes() == (tmp_path / "want").read_bytes()
