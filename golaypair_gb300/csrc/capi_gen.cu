@@ -377,21 +377,29 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     }
     t_win = since(tb);
     // ---- capacities and the device arena
-    // appends after a job met its soft cap: a lane sees the count at most
-    // 2 kCapCheck steps late, and a step (a block of the words that differ
-    // from a prenecklace in its last two digits: k rows of up to k words)
-    // appends at most one candidate per row and row sum with a role; plus a
-    // warp's queue
-    auto slack_for = [&](const GenPlan& p) {
-        std::vector<int> sums;
-        for (auto& d : p.dec) {
-            sums.push_back(d.first);
-            sums.push_back(d.second);
+    // roles by digit sum: row sum = -c L + 2 * digit sum; and the enumerator's
+    // tables of them
+    std::vector<uint8_t> rtab((size_t)nj * (gp::kMaxDigitSum + 1), 0);
+    std::vector<uint64_t> ctab((size_t)nj * (gp::kMaxDigitSum + 1));
+    std::vector<gp::EnumJob> ej(nj);
+    std::vector<int> per_step(nj);  // candidates of one step, at most
+    for (int ji = 0; ji < nj; ++ji) {
+        const GenPlan& p = jobs[ji].p;
+        uint8_t* r = &rtab[(size_t)ji * (gp::kMaxDigitSum + 1)];
+        for (int ds = 0; ds <= p.L * (p.k - 1) && ds <= gp::kMaxDigitSum; ++ds) {
+            const int rs = -p.compress * p.L + 2 * ds;
+            for (auto& d : p.dec) {
+                if (rs == d.first) r[ds] |= 1;
+                if (rs == d.second) r[ds] |= 2;
+            }
         }
-        std::sort(sums.begin(), sums.end());
-        const int64_t nsums = std::unique(sums.begin(), sums.end()) - sums.begin();
-        const int64_t per_step = std::max<int64_t>(1, (int64_t)p.k * std::min<int64_t>(p.k, nsums));
-        return threads * 2 * gp::kCapCheck * per_step + threads / 32 * gp::kEnumQueue + 4096;
+        ej[ji].t = gp::enum_block(p.k, p.b, p.L, ej[ji].strict);
+        per_step[ji] = gp::enum_cand(p.b, ej[ji].t, r, gp::kMaxDigitSum + 1, &ctab[(size_t)ji * (gp::kMaxDigitSum + 1)]);
+    }
+    // appends after a job met its soft cap: a warp learns of it when it writes
+    // its queue out, and may still hold the rest of its lanes' steps
+    auto slack_for = [&](int ji) {
+        return threads / 32 * (gp::kEnumQueue + 32 * (int64_t)per_step[ji]) + 4096;
     };
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -402,17 +410,19 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     const size_t off_ctr = take(kCounterWords * 8);
     const size_t off_ejobs = take(sizeof(gp::EnumJob) * nj);
     const size_t off_rtab = take((size_t)nj * (gp::kMaxDigitSum + 1));
+    const size_t off_ctab = take(ctab.size() * 8);
     const size_t off_cur = take((size_t)nwin * 16);
     const size_t off_end = take((size_t)nwin * 16);
     const size_t off_wjob = take((size_t)nwin);
-    for (auto& j : jobs) {
+    for (int ji = 0; ji < nj; ++ji) {
+        JobRun& j = jobs[ji];
         const gp::u128 words = range_words(j);
         if (words < (gp::u128)cfg.cand_cap) {
             j.soft = (int64_t)words + 1;  // never met: the job cannot park
             j.hard = j.soft;
         } else {
             j.soft = cfg.cand_cap;
-            j.hard = cfg.cand_cap + slack_for(j.p);
+            j.hard = cfg.cand_cap + slack_for(ji);
         }
         // one iteration adds at most 2 records per candidate (x == y: A and B)
         j.rcap = 2 * j.hard + std::max<int64_t>(j.hard / 2, 4096);
@@ -435,8 +445,6 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     unsigned long long* ctr = reinterpret_cast<unsigned long long*>(A + off_ctr);
     unsigned long long* hctr = hbuf.as<unsigned long long>();
     // ---- job tables
-    std::vector<gp::EnumJob> ej(nj);
-    std::vector<uint8_t> rtab((size_t)nj * (gp::kMaxDigitSum + 1), 0);
     for (int ji = 0; ji < nj; ++ji) {
         JobRun& j = jobs[ji];
         const GenPlan& p = j.p;
@@ -458,15 +466,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
         e.cap = j.hard;
         e.soft_cap = j.soft;
         e.necklaces = ctr + kCumBase + ji * kCumSlots + 0;
-        // roles by digit sum: row sum = -c L + 2 * digit sum
-        for (int ds = 0; ds <= p.L * (p.k - 1) && ds <= gp::kMaxDigitSum; ++ds) {
-            const int rs = -p.compress * p.L + 2 * ds;
-            uint8_t& r = rtab[(size_t)ji * (gp::kMaxDigitSum + 1) + ds];
-            for (auto& d : p.dec) {
-                if (rs == d.first) r |= 1;
-                if (rs == d.second) r |= 2;
-            }
-        }
+        e.cand = reinterpret_cast<const uint64_t*>(A + off_ctab) + (size_t)ji * (gp::kMaxDigitSum + 1);
         // (built before any graph capture: the tables are copied synchronously)
         if (!c->twiddle_image(p.L) || !c->twiddle64(p.L))
             return c->fail(GP_ERR_NOMEM, "batch generation: twiddle tables for length %d", p.L);
@@ -474,6 +474,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     }
     GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_ejobs, ej.data(), sizeof(gp::EnumJob) * nj, cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_rtab, rtab.data(), rtab.size(), cudaMemcpyHostToDevice, s));
+    GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_ctab, ctab.data(), ctab.size() * 8, cudaMemcpyHostToDevice, s));
     if (nwin) {
         GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_cur, cur.data(), (size_t)nwin * 16, cudaMemcpyHostToDevice, s));
         GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_end, end.data(), (size_t)nwin * 16, cudaMemcpyHostToDevice, s));

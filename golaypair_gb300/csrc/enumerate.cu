@@ -13,11 +13,13 @@
 //     a_j = a_{j-(i+1)} for j > i  (period i + 1)
 // until it leaves the window.  Words are packed (see rows.cuh), so the
 // successor is a handful of 64- or 128-bit bit operations.  One step takes a
-// block: the successors that only change the last two digits follow a fixed
-// pattern (rows of Lyndon words, see the kernel), so a block's necklaces are
-// counted row by row without visiting them.  Necklaces whose digit sum
-// matches a decomposition's row sum are appended (warp-aggregated) to a
-// candidate buffer with their A/B role bits.
+// block of up to 64 words: those that share all but their last six bits, t
+// digits.  Which of them are necklaces depends on the word's first t - 1
+// digits only, so it is one table entry, and so are the ones whose digit sum
+// matches a decomposition's row sum, by the sum of the other digits: a
+// step's necklaces are counted and its candidates found without visiting
+// them.  Candidates are appended (warp-aggregated) to a buffer with their A/B
+// role bits.
 //
 // One launch serves several jobs (orders / compressions, each with its own
 // length, alphabet, row-sum table and candidate buffer): every window names
@@ -72,26 +74,13 @@ __device__ __forceinline__ W128 periodic_fill(W128 w, int b, int L, int p) {
     return band(x, low_mask(b * L));
 }
 
-// First prenecklace >= w (w a word of L digits); returns its period.
-__device__ __forceinline__ int first_prenecklace(W128& w, int b, int L) {
-    int p = 1;
-    for (int i = 1; i < L; ++i) {
-        const int d = digit(w, b, L, i), e = digit(w, b, L, i - p);
-        if (d > e) {
-            p = i + 1;
-        } else if (d < e) {
-            w = periodic_fill(w, b, L, p);
-            return p;
-        }
-    }
-    return p;
-}
-
 // The layout of the job a thread is enumerating, held in registers.
 struct JobView {
     int L, b;
     bool narrow;              // b * L <= 64: the word fits its low 64 bits
     uint32_t inv_b;           // floor(x / b) = (x * inv_b) >> 8 for 0 <= x < 128
+    int lead_shift;           // a word's first t - 1 digits: word >> lead_shift
+    uint32_t block;           // a block's words differ in these low bits
     W128 maxpat, full;        // full = low_mask(b * L)
     W128 ones;                // bit 0 of every digit; bit t of every digit = ones << t
     W128 divisors;            // bit p set iff p divides L (the necklace test, no division)
@@ -104,6 +93,8 @@ __device__ __forceinline__ JobView job_view(const EnumJob& j) {
     v.maxpat = w128(j.maxpat);
     v.full = low_mask(j.b * j.L);
     v.ones = w128(j.plane[0]);
+    v.lead_shift = j.b * (j.L - j.t + 1);
+    v.block = (1u << (j.b * j.t)) - 1u;
     v.inv_b = (256u + (uint32_t)j.b - 1u) / (uint32_t)j.b;
     v.narrow = j.b * j.L <= 64;
     v.divisors = {0, 0};
@@ -148,6 +139,40 @@ __device__ __forceinline__ int fkm_next64(uint64_t& w, const JobView& a) {
     return p;
 }
 
+// First prenecklace >= w (w a word of L digits); returns its period.
+__device__ __forceinline__ int first_prenecklace(W128& w, int b, int L) {
+    int p = 1;
+    for (int i = 1; i < L; ++i) {
+        const int d = digit(w, b, L, i), e = digit(w, b, L, i - p);
+        if (d > e) {
+            p = i + 1;
+        } else if (d < e) {
+            w = periodic_fill(w, b, L, p);
+            return p;
+        }
+    }
+    return p;
+}
+
+// The same on words of at most 63 bits.
+__device__ __forceinline__ int first_prenecklace64(uint64_t& w, const JobView& a) {
+    const uint64_t m = (1ull << a.b) - 1ull;
+    int p = 1;
+    for (int i = 1; i < a.L; ++i) {
+        const uint64_t d = (w >> (a.b * (a.L - 1 - i))) & m, e = (w >> (a.b * (a.L - 1 - i + p))) & m;
+        if (d > e) {
+            p = i + 1;
+        } else if (d < e) {
+            const uint64_t full = a.full.lo;
+            uint64_t y = w & (full ^ mask64(a.b * (a.L - p)));
+            for (int len = p; len < a.L; len <<= 1) y |= y >> (a.b * len);
+            w = y & full;
+            return p;
+        }
+    }
+    return p;
+}
+
 __device__ __forceinline__ int digit_sum64(uint64_t w, const JobView& a) {
     int s = 0;
 #pragma unroll
@@ -174,16 +199,21 @@ __device__ __forceinline__ uint4 to_u4(W128 w) {
 __device__ __forceinline__ W128 from_u4(uint4 v) {
     return {((uint64_t)v.y << 32) | v.x, ((uint64_t)v.w << 32) | v.z};
 }
+// Digit sum of a word of a job, for its role.
+__device__ __forceinline__ int word_sum(uint4 v, const EnumJob& j) {
+    const W128 w = from_u4(v), ones = w128(j.plane[0]);
+    int s = 0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        if (t < j.b) {
+            const W128 m = band(w, shl(ones, t));
+            s += (__popcll(m.lo) + __popcll(m.hi)) << t;
+        }
+    }
+    return s;
+}
 __device__ __forceinline__ bool job_full(const EnumJob& j) {
     return (int64_t)*reinterpret_cast<volatile unsigned long long*>(j.count) >= j.soft_cap;
-}
-
-// Bits lo .. lo + n - 1 (n <= 16) of a job's digit-sum bitset, as bits 0 .. n - 1.
-__device__ __forceinline__ uint64_t role_bits(const unsigned long long* tb, int lo, int n) {
-    const int wi = lo >> 6, sh = lo & 63;
-    uint64_t x = tb[wi] >> sh;
-    if (sh) x |= tb[wi + 1] << (64 - sh);
-    return x & ((1ull << n) - 1ull);
 }
 
 // Each thread takes windows from a global counter.  A window whose job
@@ -196,11 +226,16 @@ __device__ __forceinline__ uint64_t role_bits(const unsigned long long* tb, int 
 // Candidates go to a per-warp queue in shared memory first; the warp writes
 // them out when kFlushAt or more are queued, with one counter atomic per
 // job present.  (An atomic per step, whose returned offset the whole warp waits
-// for, made the kernel memory-latency bound.)  A job's soft capacity is
-// checked on a count loaded at the previous check, so the load's latency
-// overlaps the steps in between.
+// for, made the kernel memory-latency bound.)  What the atomic returns tells
+// the warp when a job has met its soft capacity.
+//
+// What bounds it: issue, of the steps where a word has few necklaces behind it
+// and of the queue where many (windows of 2^32 words: order 57 9.4 ms, five
+// orders 48 ms).
+// A block of two digits, its rows taken one by one, needed four times
+// the steps over an alphabet of four and longer ones: 15.1 and 87 ms.
 constexpr int kFlushAt = kEnumQueue - 32;
-constexpr int kQueue = kEnumQueue;  // per warp: < kFlushAt queued + 32 from one step
+constexpr int kQueue = kEnumQueue;  // per warp
 
 // NARROW: every job's words fit 63 bits, so a word and its window end are
 // 64-bit values (the high halves are zero and drop out of the registers).
@@ -208,26 +243,17 @@ template <int MINB, bool NARROW>
 __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
     __shared__ uint8_t role_tab[kMaxEnumJobs][kMaxDigitSum + 1];
     __shared__ EnumJob jobs[kMaxEnumJobs];
-    __shared__ uint4 q_word[8][kQueue];
-    __shared__ uint8_t q_role[8][kQueue];
-    __shared__ uint8_t q_job[8][kQueue];
-    // bit s of tbits[j]: digit sum s has a role in job j (one spare word so
-    // that a 64-bit window starting below bit 1024 stays inside)
-    __shared__ unsigned long long tbits[kMaxEnumJobs][(kMaxDigitSum + 1) / 64 + 1];
-    for (int i = threadIdx.x; i < kMaxEnumJobs * ((kMaxDigitSum + 1) / 64 + 1); i += blockDim.x)
-        (&tbits[0][0])[i] = 0ull;
-    __syncthreads();
-    for (int i = threadIdx.x; i < a.njobs * (kMaxDigitSum + 1); i += blockDim.x) {
-        const int jj = i / (kMaxDigitSum + 1), ds = i % (kMaxDigitSum + 1);
-        role_tab[jj][ds] = a.roles[i];
-        if (a.roles[i]) atomicOr(&tbits[jj][ds >> 6], 1ull << (ds & 63));
-    }
+    __shared__ uint4 q_word[8][kQueue];  // NARROW: the high half holds the job
+    __shared__ uint8_t q_job[NARROW ? 1 : 8][NARROW ? 1 : kQueue];
+    for (int i = threadIdx.x; i < a.njobs * (kMaxDigitSum + 1); i += blockDim.x)
+        role_tab[i / (kMaxDigitSum + 1)][i % (kMaxDigitSum + 1)] = a.roles[i];
     if (threadIdx.x < a.njobs) jobs[threadIdx.x] = a.jobs[threadIdx.x];
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int wq = threadIdx.x >> 5;  // this warp's queue
     const uint32_t lt_mask = (1u << lane) - 1u;
     int qlen = 0;                     // queued candidates (the same in every lane)
+    uint32_t full_jobs = 0;           // jobs whose count this warp has seen at the soft capacity
     // writes the warp's queue out (every lane of the warp calls it)
     auto flush = [&]() {
         __syncwarp();
@@ -235,28 +261,36 @@ __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
             const int e = base + lane;
             const bool has = e < qlen;
             const uint32_t hm = __ballot_sync(0xFFFFFFFFu, has);
+            uint32_t met = 0;
             if (has) {
-                const int jb = q_job[wq][e];
+                uint4 word = q_word[wq][e];
+                int jb;
+                if constexpr (NARROW) {
+                    jb = (int)word.z;
+                    word.z = 0;
+                } else {
+                    jb = q_job[wq][e];
+                }
                 const uint32_t grp = __match_any_sync(hm, jb);
                 const int leader = __ffs(grp) - 1;
                 const EnumJob& J = jobs[jb];
                 unsigned long long pos0 = 0;
                 if (lane == leader) pos0 = atomicAdd(J.count, (unsigned long long)__popc(grp));
                 pos0 = __shfl_sync(grp, pos0, leader);
+                if ((int64_t)pos0 + __popc(grp) >= J.soft_cap) met = 1u << jb;
                 const unsigned long long pos = pos0 + __popc(grp & lt_mask);
                 if ((int64_t)pos < J.cap) {
-                    J.words[pos] = q_word[wq][e];
-                    J.out_roles[pos] = q_role[wq][e];
+                    J.words[pos] = word;
+                    J.out_roles[pos] = role_tab[jb][word_sum(word, J)];
                 } else {
                     atomicCAS(a.status, 0, GP_KSTATUS_OVERFLOW);
                 }
             }
+            full_jobs |= __reduce_or_sync(0xFFFFFFFFu, met);
         }
         qlen = 0;
         __syncwarp();
     };
-    unsigned long long seen_count = 0;  // count of job seen_job, loaded at the previous check
-    int seen_job = -1;
     // windows are handed out dynamically: a thread takes the next unvisited
     // one from a global counter when it needs work (long windows do not
     // hold up a statically assigned share)
@@ -277,7 +311,7 @@ __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
     bool have = false;  // w is a valid prenecklace to process
     bool parked_any = false;
     unsigned long long necklaces = 0;  // of job `job`, flushed when the job changes
-    for (int step = 1;; ++step) {
+    for (;;) {
         // (re)load a window when idle; skip windows whose job is full
         while (active && !have) {
             const int nj = a.win_job[win];
@@ -297,7 +331,10 @@ __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
                 }
                 jv = job_view(jobs[job]);
                 if (lt(w, end)) {
-                    p = first_prenecklace(w, jv.b, jv.L);
+                    if constexpr (NARROW)
+                        p = first_prenecklace64(w.lo, jv);
+                    else
+                        p = first_prenecklace(w, jv.b, jv.L);
                     have = lt(w, end);
                 }
                 if (have && pref < 0) pref = (int64_t)atomicAdd(a.next_win, 1ull);
@@ -309,116 +346,83 @@ __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
             }
         }
         if (!__any_sync(0xFFFFFFFFu, active)) break;
-        // One step takes a block of words that differ from the prenecklace w
-        // only in the last two digits (v, d), in FKM order:
-        //  * the rest of w's row: FKM's successor of a word whose last digit
-        //    is below the maximum K is the word with that digit raised by
-        //    one, with period L (a Lyndon word, so a necklace);
-        //  * when the last digit reaches K and the second-to-last v is below
-        //    K: the successor raises v and sets the last digit to the first
-        //    digit a_0 (period L - 1), then raises the last digit again
-        //    (period L) up to K; and so on up to v = K (L >= 3, so a_0 is not
-        //    the raised digit, and k^2 <= 64 for the candidate mask);
-        // up to the window's end.  The block's necklaces are counted without
-        // visiting them one by one, its candidates are the words whose digit
-        // sum has a role, and one successor follows the whole block.
+        // One step takes the prenecklace w and the words after it that differ
+        // from it in the last t digits only, x (t as the job's table has it,
+        // L >= 2 t or t = 1).  Let a_0 a_1 .. be w's first digits.
+        //  * A word with a larger x is a prenecklace iff no tail of x that is
+        //    shorter than x is less than the a_0 a_1 .. of its length: tails
+        //    that begin before x hold because w is one.
+        //  * Its period is L, and it is a necklace, iff no such tail equals
+        //    a_0 a_1 ..; else its period L - m, m < t the tail's length, does
+        //    not divide L, as L > 2 m.
+        //  * w itself is a necklace iff its period p divides L.
+        // After the block comes FKM's successor of the word with the largest x,
+        // every digit the maximum, which is a prenecklace too.
         W128 w0 = w;
-        uint64_t cmask = 0;  // bit (v - v0) * k + d: that word is a candidate
-        int spre = 0, v0 = 0, kk = 1;
+        uint64_t cmask = 0;  // bit x: that word is a candidate
         if (active) {
-            const int b = jv.b;
-            const uint64_t dmask = (1ull << b) - 1ull;
-            const int K = (int)(jv.maxpat.lo & dmask);
-            kk = K + 1;
-            const int d0 = (int)(w.lo & dmask);
-            v0 = (int)((w.lo >> b) & dmask);
-            const bool two = jv.L >= 3 && kk * kk <= 64;
-            const int vmax = two ? K : v0;
-            // words at or past the window's end are cut: x = (v << b) | d below xend
-            uint32_t xend = 0xFFFFFFFFu;
-            const uint64_t m2 = (1ull << (2 * b)) - 1ull;
-            if ((NARROW || end.hi == w.hi) && (end.lo & ~m2) == (w.lo & ~m2)) xend = (uint32_t)(end.lo & m2);
-            const int a0 = (NARROW || jv.narrow) ? (int)((w.lo >> (b * (jv.L - 1))) & dmask) : digit(w, b, jv.L, 0);
-            const int s0 = (NARROW || jv.narrow) ? digit_sum64(w.lo, jv) : digit_sum(w, jv);
-            spre = s0 - v0 - d0;
-            const bool neck_first = divides_L(jv, p), neck_row = divides_L(jv, jv.L - 1);
-            int lastv = v0, lastd = d0;
-            for (int v = v0; v <= vmax; ++v) {
-                // row v: words (v, dlo .. dhi); every one a necklace but
-                // perhaps the first; candidates: the digit sums with a role
-                const int dlo = v == v0 ? d0 : a0;
-                int dhi = K;
-                bool cut = false;
-                const int64_t lim = (int64_t)xend - ((int64_t)v << b) - 1;  // xend = 2^32 - 1: no cut
-                if (lim < (int64_t)dhi) {
-                    dhi = (int)lim;
-                    cut = true;
+            const EnumJob& J = jobs[job];
+            const uint32_t x0 = (uint32_t)w.lo & jv.block;
+            w0.lo = w.lo & ~(uint64_t)jv.block;
+            const uint32_t a0 = (uint32_t)(NARROW ? w.lo >> jv.lead_shift : shr(w, jv.lead_shift).lo);
+            uint64_t in = J.strict[a0] & (~1ull << x0);
+            bool done = false;
+            if ((NARROW || end.hi == w.hi) && ((end.lo ^ w.lo) & ~(uint64_t)jv.block) == 0) {
+                in &= (1ull << ((uint32_t)end.lo & jv.block)) - 1ull;  // the window ends here
+                done = true;
+            }
+            if (divides_L(jv, p)) in |= 1ull << x0;
+            necklaces += (unsigned long long)__popcll(in);
+            const int sum = (NARROW || jv.narrow) ? digit_sum64(w0.lo, jv) : digit_sum(w0, jv);
+            cmask = in & __ldg(J.cand + sum);
+            if (!done) {
+                w.lo = w0.lo | (jv.maxpat.lo & jv.block);
+                if (NARROW || jv.narrow) {
+                    uint64_t wl = w.lo;
+                    p = fkm_next64(wl, jv);
+                    w.lo = wl;
+                } else {
+                    p = fkm_next(w, jv);
                 }
-                if (dhi < dlo) break;
-                const int n = dhi - dlo + 1;
-                const bool first_neck = v == v0 ? neck_first : neck_row;
-                necklaces += (unsigned long long)(n - (first_neck ? 0 : 1));
-                uint64_t rm = role_bits(tbits[job], spre + v + dlo, n);
-                if (!first_neck) rm &= ~1ull;
-                cmask |= rm << ((v - v0) * kk + dlo);
-                lastv = v;
-                lastd = dhi;
-                if (cut) break;
+                done = p == 0 || !(NARROW ? w.lo < end.lo : lt(w, end));
             }
-            // the block's last word, then its successor
-            w.lo = (w.lo & ~m2) | ((uint64_t)lastv << b) | (uint64_t)lastd;
-            int np;
-            if (NARROW || jv.narrow) {
-                uint64_t wl = w.lo;
-                np = fkm_next64(wl, jv);
-                w.lo = wl;
-            } else {
-                np = fkm_next(w, jv);
-            }
-            if (np == 0 || !(NARROW ? w.lo < end.lo : lt(w, end))) {
-                have = false;
-                a.cur[win] = a.end[win];
-                win = take();
-                active = win < a.nwin;
-            } else {
-                p = np;
-            }
+            if (done) a.cur[win] = a.end[win];
+            have = !done;
         }
-        // queue the block's candidates, one per lane per round; write the
-        // queue out from kFlushAt
+        // the block's candidates into the queue, each lane's behind those of
+        // the lanes before it; written out from kFlushAt on
         while (__any_sync(0xFFFFFFFFu, cmask != 0)) {
-            const bool has = cmask != 0;
-            const int t = has ? __ffsll((long long)cmask) - 1 : 0;
-            cmask &= cmask - 1ull;
-            const uint32_t want = __ballot_sync(0xFFFFFFFFu, has);
-            if (has) {
-                const int slot = qlen + __popc(want & lt_mask);
-                const int v = v0 + t / kk, d = t % kk;
-                W128 cand = w0;
-                const int b = jv.b;
-                const uint64_t m2 = (1ull << (2 * b)) - 1ull;
-                cand.lo = (cand.lo & ~m2) | ((uint64_t)v << b) | (uint64_t)d;
-                q_word[wq][slot] = to_u4(cand);
-                q_role[wq][slot] = role_tab[job][spre + v + d];
-                q_job[wq][slot] = (uint8_t)job;
+            const int n = __popcll(cmask);
+            int to = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xFFFFFFFFu, to, o);
+                if (lane >= o) to += y;
             }
-            qlen += __popc(want);
+            const int total = __shfl_sync(0xFFFFFFFFu, to, 31);
+            for (int slot = qlen + to - n; cmask && slot < kQueue; ++slot) {
+                W128 cand = w0;
+                cand.lo |= (uint64_t)(__ffsll((long long)cmask) - 1);
+                cmask &= cmask - 1ull;
+                if constexpr (NARROW) {
+                    cand.hi = (uint64_t)job;
+                } else {
+                    q_job[wq][slot] = (uint8_t)job;
+                }
+                q_word[wq][slot] = to_u4(cand);
+            }
+            qlen = qlen + total < kQueue ? qlen + total : kQueue;
             if (qlen >= kFlushAt) flush();
         }
-        // every kCapCheck steps: leave a window whose job reached its soft
-        // capacity (by the count loaded kCapCheck steps ago), then load the
-        // count afresh
-        if ((step & (kCapCheck - 1)) == 0 && active && have) {
-            if (seen_job == job && (int64_t)seen_count >= jobs[job].soft_cap) {
-                a.cur[win] = to_u4(w);
-                have = false;
-                parked_any = true;
-                win = take();
-                active = win < a.nwin;
-            } else {
-                seen_count = *reinterpret_cast<volatile unsigned long long*>(jobs[job].count);
-                seen_job = job;
-            }
+        // leave a window whose job has met its soft capacity
+        if (active && have && ((full_jobs >> job) & 1u)) {
+            a.cur[win] = to_u4(w);
+            have = false;
+            parked_any = true;
+        }
+        if (active && !have) {
+            win = take();
+            active = win < a.nwin;
         }
     }
     flush();

@@ -14,9 +14,6 @@ namespace gp {
 
 constexpr int kMaxDigitSum = 1023;
 constexpr int kMaxEnumJobs = 8;
-// Steps between a lane's checks of its job's candidate count against the
-// soft capacity (a step is a block of up to k^2 words; see enumerate.cu).
-constexpr int kCapCheck = 2;
 constexpr int kEnumQueue = 264;  // candidates a warp queues in shared memory (written out from 232; static shared memory stays under 48 KB)
 
 struct U128p {
@@ -34,7 +31,49 @@ struct EnumJob {
     int64_t cap;               // hard capacity of words / out_roles
     int64_t soft_cap;          // stop when count reaches this
     unsigned long long* necklaces;  // out: necklaces visited
+    // Blocks of words that differ in their last t digits x (b t <= 6 bits):
+    int t;
+    uint64_t strict[32];       // [first t - 1 digits]: x whose shorter tails all exceed them
+    const uint64_t* cand;      // device, [sum of the other digits]: x with a digit sum that has a role
 };
+
+// t, and fills strict.
+inline int enum_block(int k, int b, int L, uint64_t strict[32]) {
+    const int t = L >= 2 * (6 / b) ? 6 / b : 1;
+    for (uint32_t a = 0; a < 32; ++a) {
+        strict[a] = 0;
+        if (a >> (b * (t - 1))) continue;
+        for (uint32_t x = 0; x < (1u << (b * t)); ++x) {
+            bool in = true;
+            for (int i = 0; i < t; ++i) in = in && (int)((x >> (b * i)) & ((1u << b) - 1u)) < k;
+            for (int n = 1; n < t; ++n)  // tails of n digits
+                in = in && (x & ((1u << (b * n)) - 1u)) > (a >> (b * (t - 1 - n)));
+            if (in) strict[a] |= 1ull << x;
+        }
+    }
+    return t;
+}
+
+// cand[s], s = 0 .. n - 1: bit x where s + the digit sum of x has a role
+// (roles of digit sums 0 .. n - 1; none beyond); the largest number of bits set
+// in one entry.
+inline int enum_cand(int b, int t, const uint8_t* roles, int n, uint64_t* cand) {
+    int most = 0;
+    for (int s = 0; s < n; ++s) {
+        cand[s] = 0;
+        int bits = 0;
+        for (uint32_t x = 0; x < (1u << (b * t)); ++x) {
+            int d = s;
+            for (int i = 0; i < t; ++i) d += (int)((x >> (b * i)) & ((1u << b) - 1u));
+            if (d < n && roles[d]) {
+                cand[s] |= 1ull << x;
+                ++bits;
+            }
+        }
+        most = bits > most ? bits : most;
+    }
+    return most;
+}
 
 struct EnumArgs {
     const EnumJob* jobs;       // device array of njobs jobs
