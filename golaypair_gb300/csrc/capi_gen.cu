@@ -497,6 +497,9 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     gp::EnumArgs ea_wide = ea;
     ea.nwin = nwin_narrow;
     ea.narrow = 1;
+    ea.win_jobs = ea_wide.win_jobs = 0;
+    for (int ji = 0; ji < nj; ++ji)
+        if (range_words(jobs[ji]) != 0) (narrow_job(ji) ? ea : ea_wide).win_jobs |= 1u << ji;
     ea_wide.cur += nwin_narrow;
     ea_wide.end += nwin_narrow;
     ea_wide.win_job += nwin_narrow;

@@ -25,6 +25,8 @@
 // length, alphabet, row-sum table and candidate buffer): every window names
 // its job.  A window whose job's buffer has met its soft capacity is left
 // with its position saved; the host drains the buffers and relaunches.
+#include <type_traits>
+
 #include "gp_device.cuh"
 #include "enumerate.h"
 
@@ -74,7 +76,7 @@ __device__ __forceinline__ W128 periodic_fill(W128 w, int b, int L, int p) {
     return band(x, low_mask(b * L));
 }
 
-// The layout of the job a thread is enumerating, held in registers.
+// The layout of a job's words, derived once per block (in shared memory).
 struct JobView {
     int L, b;
     bool narrow;              // b * L <= 64: the word fits its low 64 bits
@@ -199,153 +201,208 @@ __device__ __forceinline__ uint4 to_u4(W128 w) {
 __device__ __forceinline__ W128 from_u4(uint4 v) {
     return {((uint64_t)v.y << 32) | v.x, ((uint64_t)v.w << 32) | v.z};
 }
-// Digit sum of a word of a job, for its role.
-__device__ __forceinline__ int word_sum(uint4 v, const EnumJob& j) {
-    const W128 w = from_u4(v), ones = w128(j.plane[0]);
-    int s = 0;
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-        if (t < j.b) {
-            const W128 m = band(w, shl(ones, t));
-            s += (__popcll(m.lo) + __popcll(m.hi)) << t;
-        }
-    }
-    return s;
-}
 __device__ __forceinline__ bool job_full(const EnumJob& j) {
     return (int64_t)*reinterpret_cast<volatile unsigned long long*>(j.count) >= j.soft_cap;
 }
 
-// Each thread takes windows from a global counter.  A window whose job
-// has reached its soft capacity is left (position saved) and the thread goes
-// on with its next window, so one full job does not idle the others.
-// MINB = 3: 72 registers, no spills (3 CTAs of 256 per SM);
-// MINB = 4: at most 64 registers (4 CTAs of 256 per SM); MINB = 8: capped
-// at 32 registers for full occupancy (some spills).  The tuner picks.
+// A warp takes windows from a global counter, up to 32 at a time: it loads
+// them, drops finished ones and finds their first prenecklaces together, and
+// hands them to its lanes as these run out of work.  A window whose job has
+// reached its soft capacity is left (position saved), so one full job does not
+// idle the others.
 //
 // Candidates go to a per-warp queue in shared memory first; the warp writes
 // them out when kFlushAt or more are queued, with one counter atomic per
-// job present.  (An atomic per step, whose returned offset the whole warp waits
-// for, made the kernel memory-latency bound.)  What the atomic returns tells
-// the warp when a job has met its soft capacity.
+// job present.  What the atomic returns tells the warp when a job has met its
+// soft capacity; warps that find few candidates look at the count every
+// kCapCheck steps, on a load whose latency overlaps the steps in between.
 //
-// What bounds it: issue, of the steps where a word has few necklaces behind it
-// and of the queue where many (windows of 2^32 words: order 57 9.4 ms, five
-// orders 48 ms).
-// A block of two digits, its rows taken one by one, needed four times
-// the steps over an alphabet of four and longer ones: 15.1 and 87 ms.
-constexpr int kFlushAt = kEnumQueue - 32;
-constexpr int kQueue = kEnumQueue;  // per warp
-
+// What bounds it: issue (67 %) once every lane has a dense window, the last
+// windows' serial steps at the end.  An order-57 window of 2^32 words (2.3 G
+// necklaces, 208 M candidates): 2.6 ms of kernel time, 9.4 when each lane took,
+// loaded and checked its own windows and every 32 candidates took an atomic,
+// 15.1 with blocks of two digits taken a row at a time; five orders: 27, 48 and
+// 87 ms.  Blocks per SM 4, 5, 6: 2.56, 2.53, 2.70 and 27.0, 27.2, 30.4 ms.
+//
 // NARROW: every job's words fit 63 bits, so a word and its window end are
 // 64-bit values (the high halves are zero and drop out of the registers).
+constexpr int kQueue = kEnumQueue;  // per warp
+constexpr int kFlushAt = kEnumQueue - 32;
+constexpr int kCapCheck = 4;
+
+template <bool NARROW>
+struct EnumShared {
+    using Word = typename std::conditional<NARROW, uint64_t, W128>::type;
+    EnumJob jobs[kMaxEnumJobs];
+    JobView views[kMaxEnumJobs];
+    unsigned long long visited[kMaxEnumJobs];  // necklaces, by job
+    Word q_word[8][kQueue];                    // per warp: queued candidates and their jobs
+    Word pool_w[8][32], pool_end[8][32];       // per warp: windows taken and not begun
+    int64_t pool_win[8][32];
+    uint8_t q_job[8][kQueue], pool_p[8][32], pool_job[8][32];
+};
+
 template <int MINB, bool NARROW>
 __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
-    __shared__ uint8_t role_tab[kMaxEnumJobs][kMaxDigitSum + 1];
-    __shared__ EnumJob jobs[kMaxEnumJobs];
-    __shared__ uint4 q_word[8][kQueue];  // NARROW: the high half holds the job
-    __shared__ uint8_t q_job[NARROW ? 1 : 8][NARROW ? 1 : kQueue];
-    for (int i = threadIdx.x; i < a.njobs * (kMaxDigitSum + 1); i += blockDim.x)
-        role_tab[i / (kMaxDigitSum + 1)][i % (kMaxDigitSum + 1)] = a.roles[i];
-    if (threadIdx.x < a.njobs) jobs[threadIdx.x] = a.jobs[threadIdx.x];
+    __shared__ EnumShared<NARROW> sh;
+    if (threadIdx.x < a.njobs) {
+        sh.jobs[threadIdx.x] = a.jobs[threadIdx.x];
+        sh.views[threadIdx.x] = job_view(sh.jobs[threadIdx.x]);
+    }
+    if (threadIdx.x < kMaxEnumJobs) sh.visited[threadIdx.x] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int wq = threadIdx.x >> 5;  // this warp's queue
+    const int wq = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    int qlen = 0;                     // queued candidates (the same in every lane)
-    uint32_t full_jobs = 0;           // jobs whose count this warp has seen at the soft capacity
-    // writes the warp's queue out (every lane of the warp calls it)
+    // the same in every lane of the warp:
+    int qlen = 0;             // queued candidates
+    uint32_t full_jobs = 0;   // jobs seen at their soft capacity
+    int pool = 0;             // windows in the pool
+    bool open = true;         // windows may be left at the counter
+    bool parked = false;      // (per lane) a window was left
+    auto put = [](W128 v) {
+        if constexpr (NARROW)
+            return v.lo;
+        else
+            return v;
+    };
+    auto get = [](auto v) {
+        if constexpr (NARROW)
+            return W128{v, 0};
+        else
+            return v;
+    };
+    auto before = [](W128 x, W128 y) { return NARROW ? x.lo < y.lo : lt(x, y); };
+
+    // writes the warp's queue out
     auto flush = [&]() {
         __syncwarp();
-        for (int base = 0; base < qlen; base += 32) {
-            const int e = base + lane;
-            const bool has = e < qlen;
-            const uint32_t hm = __ballot_sync(0xFFFFFFFFu, has);
-            uint32_t met = 0;
-            if (has) {
-                uint4 word = q_word[wq][e];
-                int jb;
-                if constexpr (NARROW) {
-                    jb = (int)word.z;
-                    word.z = 0;
-                } else {
-                    jb = q_job[wq][e];
-                }
-                const uint32_t grp = __match_any_sync(hm, jb);
-                const int leader = __ffs(grp) - 1;
-                const EnumJob& J = jobs[jb];
-                unsigned long long pos0 = 0;
-                if (lane == leader) pos0 = atomicAdd(J.count, (unsigned long long)__popc(grp));
-                pos0 = __shfl_sync(grp, pos0, leader);
-                if ((int64_t)pos0 + __popc(grp) >= J.soft_cap) met = 1u << jb;
-                const unsigned long long pos = pos0 + __popc(grp & lt_mask);
-                if ((int64_t)pos < J.cap) {
-                    J.words[pos] = word;
-                    J.out_roles[pos] = role_tab[jb][word_sum(word, J)];
+        uint32_t present = 0;  // jobs in the queue, one nearly always
+        for (int e = lane; e < qlen; e += 32) present |= 1u << sh.q_job[wq][e];
+        present = __reduce_or_sync(0xFFFFFFFFu, present);
+        while (present) {
+            const int jb = __ffs(present) - 1;
+            present &= present - 1u;
+            const EnumJob& J = sh.jobs[jb];
+            unsigned mine = 0;
+            for (int e = lane; e < qlen; e += 32) mine += sh.q_job[wq][e] == jb;
+            const unsigned count = __reduce_add_sync(0xFFFFFFFFu, mine);
+            unsigned long long pos = 0;
+            if (lane == 0) pos = atomicAdd(J.count, (unsigned long long)count);
+            pos = __shfl_sync(0xFFFFFFFFu, pos, 0);
+            if ((int64_t)(pos + count) >= J.soft_cap) full_jobs |= 1u << jb;
+            for (int base = 0; base < qlen; base += 32) {
+                const int e = base + lane;
+                const bool has = e < qlen && sh.q_job[wq][e] == jb;
+                const uint32_t hm = __ballot_sync(0xFFFFFFFFu, has);
+                const unsigned long long at = pos + __popc(hm & lt_mask);
+                pos += __popc(hm);
+                if (!has) continue;
+                if ((int64_t)at < J.cap) {
+                    const W128 word = get(sh.q_word[wq][e]);
+                    J.words[at] = to_u4(word);
+                    const int sum = NARROW ? digit_sum64(word.lo, sh.views[jb]) : digit_sum(word, sh.views[jb]);
+                    J.out_roles[at] = __ldg(a.roles + jb * (kMaxDigitSum + 1) + sum);
                 } else {
                     atomicCAS(a.status, 0, GP_KSTATUS_OVERFLOW);
                 }
             }
-            full_jobs |= __reduce_or_sync(0xFFFFFFFFu, met);
         }
         qlen = 0;
         __syncwarp();
     };
-    // windows are handed out dynamically: a thread takes the next unvisited
-    // one from a global counter when it needs work (long windows do not
-    // hold up a statically assigned share)
-    // The index of the window after the current one is fetched when the
-    // current one starts, so the atomic's latency is hidden by its steps.
-    int64_t pref = -1;
-    auto take = [&]() -> int64_t {
-        const int64_t w0 = pref >= 0 ? pref : (int64_t)atomicAdd(a.next_win, 1ull);
-        pref = -1;
-        return w0;
-    };
-    int64_t win = take();  // current window
-    bool active = win < a.nwin;
-    W128 w = {0, 0}, end = {0, 0};
-    JobView jv{};
-    int job = 0;
-    int p = 0;
-    bool have = false;  // w is a valid prenecklace to process
-    bool parked_any = false;
-    unsigned long long necklaces = 0;  // of job `job`, flushed when the job changes
-    for (;;) {
-        // (re)load a window when idle; skip windows whose job is full
-        while (active && !have) {
-            const int nj = a.win_job[win];
-            if (nj != job && necklaces) {
-                atomicAdd(jobs[job].necklaces, necklaces);
-                necklaces = 0;
+
+    // takes windows into the (empty) pool: about as many as leave some for the
+    // other warps
+    int64_t taken = 0;  // of the counter's windows, as last seen
+    auto refill = [&]() {
+        if (full_jobs == a.win_jobs) {  // nothing more to visit this time
+            parked = true;
+            open = false;
+            return;
+        }
+        int64_t n = (a.nwin - taken) / ((int64_t)gridDim.x * 8);
+        n = n < 1 ? 1 : n > 32 ? 32 : n;
+        long long w0 = 0;
+        if (lane == 0) w0 = (long long)atomicAdd(a.next_win, (unsigned long long)n);
+        w0 = __shfl_sync(0xFFFFFFFFu, w0, 0);
+        taken = w0 + n;
+        open = taken < a.nwin;
+        const int64_t win = w0 + lane;
+        bool ok = lane < n && win < a.nwin, full = false;
+        int job = 0, p = 0;
+        W128 w{}, end{};
+        if (ok) {
+            const uint4 c4 = a.cur[win], e4 = a.end[win];
+            job = a.win_job[win];
+            w = from_u4(c4);
+            end = from_u4(e4);
+            ok = lt(w, end);  // else finished
+            full = ok && (((full_jobs >> job) & 1u) || job_full(sh.jobs[job]));
+            if (full) {
+                parked = true;  // untouched: it keeps its position
+                ok = false;
             }
-            job = nj;
-            if (job_full(jobs[job])) {
-                parked_any = true;  // window untouched: it keeps its position
-            } else {
-                w = from_u4(a.cur[win]);
-                end = from_u4(a.end[win]);
-                if constexpr (NARROW) {
-                    w.hi = 0;
-                    end.hi = 0;
-                }
-                jv = job_view(jobs[job]);
-                if (lt(w, end)) {
-                    if constexpr (NARROW)
-                        p = first_prenecklace64(w.lo, jv);
-                    else
-                        p = first_prenecklace(w, jv.b, jv.L);
-                    have = lt(w, end);
-                }
-                if (have && pref < 0) pref = (int64_t)atomicAdd(a.next_win, 1ull);
-                if (!have) a.cur[win] = a.end[win];  // window finished
-            }
-            if (!have) {
-                win = take();
-                active = win < a.nwin;
+            if (ok) {
+                const JobView& v = sh.views[job];
+                if constexpr (NARROW)
+                    p = first_prenecklace64(w.lo, v);
+                else
+                    p = first_prenecklace(w, v.b, v.L);
+                ok = before(w, end);
+                if (!ok) a.cur[win] = e4;  // no prenecklace in it
             }
         }
-        if (!__any_sync(0xFFFFFFFFu, active)) break;
+        // (a warp that went on through windows it may not begin, on its own,
+        // would hold up the launch by milliseconds)
+        full_jobs |= __reduce_or_sync(0xFFFFFFFFu, full ? 1u << job : 0u);
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
+        if (ok) {
+            const int e = __popc(m & lt_mask);
+            sh.pool_w[wq][e] = put(w);
+            sh.pool_end[wq][e] = put(end);
+            sh.pool_win[wq][e] = win;
+            sh.pool_p[wq][e] = (uint8_t)p;
+            sh.pool_job[wq][e] = (uint8_t)job;
+        }
+        pool = __popc(m);
+        __syncwarp();
+    };
+
+    W128 w = {0, 0}, end = {0, 0};
+    int64_t win = 0;
+    int job = 0, p = 0;
+    bool have = false;                 // w is a prenecklace to process, of window win
+    unsigned long long necklaces = 0;  // of job `job`
+    unsigned long long seen = 0;       // a count of the lane's job
+    int seen_job = -1;
+    for (int step = 1;; ++step) {
+        // windows for idle lanes
+        for (uint32_t idle; (idle = __ballot_sync(0xFFFFFFFFu, !have)) != 0 && (pool || open);) {
+            if (!pool) refill();
+            const int r = __popc(idle & lt_mask);
+            if (!have && r < pool) {
+                const int e = pool - 1 - r;
+                const int nj = sh.pool_job[wq][e];
+                if ((full_jobs >> nj) & 1u) {
+                    parked = true;
+                } else {
+                    if (nj != job && necklaces) {
+                        atomicAdd(&sh.visited[job], necklaces);
+                        necklaces = 0;
+                    }
+                    job = nj;
+                    w = get(sh.pool_w[wq][e]);
+                    end = get(sh.pool_end[wq][e]);
+                    win = sh.pool_win[wq][e];
+                    p = sh.pool_p[wq][e];
+                    have = true;
+                }
+            }
+            pool = pool > __popc(idle) ? pool - __popc(idle) : 0;
+            __syncwarp();
+        }
+        if (!__any_sync(0xFFFFFFFFu, have)) break;
         // One step takes the prenecklace w and the words after it that differ
         // from it in the last t digits only, x (t as the job's table has it,
         // L >= 2 t or t = 1).  Let a_0 a_1 .. be w's first digits.
@@ -360,31 +417,32 @@ __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
         // every digit the maximum, which is a prenecklace too.
         W128 w0 = w;
         uint64_t cmask = 0;  // bit x: that word is a candidate
-        if (active) {
-            const EnumJob& J = jobs[job];
-            const uint32_t x0 = (uint32_t)w.lo & jv.block;
-            w0.lo = w.lo & ~(uint64_t)jv.block;
-            const uint32_t a0 = (uint32_t)(NARROW ? w.lo >> jv.lead_shift : shr(w, jv.lead_shift).lo);
+        if (have) {
+            const EnumJob& J = sh.jobs[job];
+            const JobView& v = sh.views[job];
+            const uint32_t x0 = (uint32_t)w.lo & v.block;
+            w0.lo = w.lo & ~(uint64_t)v.block;
+            const uint32_t a0 = (uint32_t)(NARROW ? w.lo >> v.lead_shift : shr(w, v.lead_shift).lo);
             uint64_t in = J.strict[a0] & (~1ull << x0);
             bool done = false;
-            if ((NARROW || end.hi == w.hi) && ((end.lo ^ w.lo) & ~(uint64_t)jv.block) == 0) {
-                in &= (1ull << ((uint32_t)end.lo & jv.block)) - 1ull;  // the window ends here
+            if ((NARROW || end.hi == w.hi) && ((end.lo ^ w.lo) & ~(uint64_t)v.block) == 0) {
+                in &= (1ull << ((uint32_t)end.lo & v.block)) - 1ull;  // the window ends here
                 done = true;
             }
-            if (divides_L(jv, p)) in |= 1ull << x0;
+            if (divides_L(v, p)) in |= 1ull << x0;
             necklaces += (unsigned long long)__popcll(in);
-            const int sum = (NARROW || jv.narrow) ? digit_sum64(w0.lo, jv) : digit_sum(w0, jv);
+            const int sum = (NARROW || v.narrow) ? digit_sum64(w0.lo, v) : digit_sum(w0, v);
             cmask = in & __ldg(J.cand + sum);
             if (!done) {
-                w.lo = w0.lo | (jv.maxpat.lo & jv.block);
-                if (NARROW || jv.narrow) {
+                w.lo = w0.lo | (v.maxpat.lo & v.block);
+                if (NARROW || v.narrow) {
                     uint64_t wl = w.lo;
-                    p = fkm_next64(wl, jv);
+                    p = fkm_next64(wl, v);
                     w.lo = wl;
                 } else {
-                    p = fkm_next(w, jv);
+                    p = fkm_next(w, v);
                 }
-                done = p == 0 || !(NARROW ? w.lo < end.lo : lt(w, end));
+                done = p == 0 || !before(w, end);
             }
             if (done) a.cur[win] = a.end[win];
             have = !done;
@@ -404,30 +462,36 @@ __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
                 W128 cand = w0;
                 cand.lo |= (uint64_t)(__ffsll((long long)cmask) - 1);
                 cmask &= cmask - 1ull;
-                if constexpr (NARROW) {
-                    cand.hi = (uint64_t)job;
-                } else {
-                    q_job[wq][slot] = (uint8_t)job;
-                }
-                q_word[wq][slot] = to_u4(cand);
+                sh.q_word[wq][slot] = put(cand);
+                sh.q_job[wq][slot] = (uint8_t)job;
             }
             qlen = qlen + total < kQueue ? qlen + total : kQueue;
             if (qlen >= kFlushAt) flush();
         }
+        if ((step & (kCapCheck - 1)) == 0) {
+            const bool met = have && seen_job == job && (int64_t)seen >= sh.jobs[job].soft_cap;
+            full_jobs |= __reduce_or_sync(0xFFFFFFFFu, met ? 1u << job : 0u);
+            if (have) {
+                seen = *reinterpret_cast<volatile unsigned long long*>(sh.jobs[job].count);
+                seen_job = job;
+            }
+        }
         // leave a window whose job has met its soft capacity
-        if (active && have && ((full_jobs >> job) & 1u)) {
+        if (have && ((full_jobs >> job) & 1u)) {
             a.cur[win] = to_u4(w);
             have = false;
-            parked_any = true;
-        }
-        if (active && !have) {
-            win = take();
-            active = win < a.nwin;
+            parked = true;
         }
     }
     flush();
-    if (parked_any) *a.incomplete = 1;
-    if (necklaces) atomicAdd(jobs[job].necklaces, necklaces);
+    if (parked) *a.incomplete = 1;
+    for (int j = 0; j < a.njobs; ++j) {
+        unsigned long long v = job == j ? necklaces : 0ull;
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+        if (lane == 0 && v) atomicAdd(&sh.visited[j], v);
+    }
+    __syncthreads();
+    if (threadIdx.x < a.njobs && sh.visited[threadIdx.x]) atomicAdd(sh.jobs[threadIdx.x].necklaces, sh.visited[threadIdx.x]);
 }
 
 template <bool NARROW>
@@ -437,8 +501,8 @@ cudaError_t launch_enumerate_t(const EnumArgs& a, int num_sms, cudaStream_t st, 
     const int vi = variant == 1 ? 1 : variant == 2 ? 2 : 0;
     int& per_sm = resident[vi];
     if (per_sm == 0) {
-        cudaError_t e = vi == 1   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enumerate_kernel<8, NARROW>, 256, 0)
-                        : vi == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enumerate_kernel<3, NARROW>, 256, 0)
+        cudaError_t e = vi == 1   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enumerate_kernel<6, NARROW>, 256, 0)
+                        : vi == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enumerate_kernel<5, NARROW>, 256, 0)
                                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enumerate_kernel<4, NARROW>, 256, 0);
         if (e != cudaSuccess || per_sm < 1) per_sm = 1;
     }
@@ -446,9 +510,9 @@ cudaError_t launch_enumerate_t(const EnumArgs& a, int num_sms, cudaStream_t st, 
     const int64_t maxb = (int64_t)num_sms * per_sm;
     if (blocks > maxb) blocks = maxb;
     if (vi == 1)
-        enumerate_kernel<8, NARROW><<<(unsigned)blocks, 256, 0, st>>>(a);
+        enumerate_kernel<6, NARROW><<<(unsigned)blocks, 256, 0, st>>>(a);
     else if (vi == 2)
-        enumerate_kernel<3, NARROW><<<(unsigned)blocks, 256, 0, st>>>(a);
+        enumerate_kernel<5, NARROW><<<(unsigned)blocks, 256, 0, st>>>(a);
     else
         enumerate_kernel<4, NARROW><<<(unsigned)blocks, 256, 0, st>>>(a);
     return cudaGetLastError();

@@ -14,7 +14,7 @@ namespace gp {
 
 constexpr int kMaxDigitSum = 1023;
 constexpr int kMaxEnumJobs = 8;
-constexpr int kEnumQueue = 264;  // candidates a warp queues in shared memory (written out from 232; static shared memory stays under 48 KB)
+constexpr int kEnumQueue = 192;  // candidates a warp queues in shared memory (written out from 160)
 
 struct U128p {
     uint64_t lo, hi;
@@ -82,6 +82,7 @@ struct EnumArgs {
     uint4* cur;                // per window: next word to visit (updated on exit)
     const uint4* end;          // per window: first word past the window
     const uint8_t* win_job;    // per window: its job
+    uint32_t win_jobs;         // the jobs that have windows here, a bit each
     int64_t nwin;
     unsigned long long* next_win;  // window handout counter (zero before the launch)
     int* incomplete;           // out: 1 if some window is unfinished
@@ -89,7 +90,7 @@ struct EnumArgs {
     int narrow;                // 1: every job's word fits 63 bits (b * L <= 63): the 64-bit kernel
 };
 
-// variant 0: unrestricted registers; 1: 32 registers, full occupancy
+// variant: 256-thread blocks per SM, 0: 4 (64 registers), 1: 6 (40), 2: 5 (48)
 cudaError_t launch_enumerate(const EnumArgs& a, int num_sms, cudaStream_t st, int variant = 0);
 
 }  // namespace gp
