@@ -7,8 +7,10 @@
 //   psd_tc_kernel      guarded FP32 tensor-core PSD filter (rows near the bound stay)
 //   mask_to_list       surviving rows
 //   finalize_kernel    exact FP64 PSD, canonical check, signature records
-// The host then orders each role's records by word (the reference's FKM
-// order) and writes the candidate files.
+// The device then sorts each role's records by word (the reference's FKM
+// order) and formats their lines (gen_text.cu), and the host writes the
+// candidate files.  Records that were drained to the host meanwhile, or go to
+// binary files, are ordered and formatted by host threads.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -24,6 +26,7 @@
 #include "ctx.h"
 #include "enumerate.h"
 #include "finalize.h"
+#include "gen_text.h"
 #include "host_math.h"
 #include "survivors.h"
 
@@ -224,6 +227,8 @@ struct JobRun {
     size_t off_words = 0, off_roles = 0, off_mask = 0, off_idx = 0, off_rec = 0, off_units = 0;
     std::vector<int16_t> units;
     RecordSet ra, rb;
+    bool want_text = false;  // the call writes text files next
+    gp::GenText text;        // made instead of ra and rb where it can be
     gp_gen_stats st{};
     // set when the engine stopped early: the word ranks still to search
     std::vector<std::pair<gp::u128, gp::u128>> remaining;
@@ -707,7 +712,16 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     GP_CUDA_TRY(c, cudaStreamSynchronize(s));
     for (int ji = 0; ji < nj; ++ji) {
         JobRun& j = jobs[ji];
-        const int rc = drain_records(c, j, A, (int64_t)hctr[kCumBase + ji * kCumSlots + 1]);
+        const int64_t nrec = (int64_t)hctr[kCumBase + ji * kCumSlots + 1];
+        int rc = GP_OK;
+        if (j.want_text && !(stop && stop->stopped) && j.ra.size() + j.rb.size() == 0) {
+            const gp::FinalizeArgs fa = finalize_args(ji);
+            gp::GenRecords r{fa.rec_words, fa.rec_role, fa.rec_sig, nrec, j.p.L, j.p.b, {}};
+            for (int i = 0; i < j.p.k; ++i) r.alpha[i] = j.p.alpha[i];
+            rc = gp::records_to_text(c, r, j.text, s);
+            if (rc) return rc;
+        }
+        if (!j.text.p) rc = drain_records(c, j, A, nrec);
         if (rc) return rc;
         j.st.necklaces += (int64_t)hctr[kCumBase + ji * kCumSlots + 0];
         j.st.psd_pass += (int64_t)hctr[kCumBase + ji * kCumSlots + 2];
@@ -837,16 +851,26 @@ int plan_for(gp_ctx* c, int order, int compress, int paf, GenPlan& p) {
     return GP_OK;
 }
 
-int finish(gp_ctx* c, const GenPlan& p, const RecordSet& ra, const RecordSet& rb, const char* path_a,
-           const char* path_b, gp_gen_stats* st) {
+int write_lines(gp_ctx* c, const char* text, size_t bytes, const char* path) {
+    FILE* f = fopen(path, "w");
+    if (!f) return c->fail(GP_ERR_IO, "cannot open %s for writing", path);
+    const bool ok = fwrite(text, 1, bytes, f) == bytes;
+    return fclose(f) == 0 && ok ? GP_OK : c->fail(GP_ERR_IO, "write failed: %s", path);
+}
+
+int finish(gp_ctx* c, const JobRun& j, const char* path_a, const char* path_b, gp_gen_stats* st) {
+    const gp::GenText& t = j.text;
     int rc_a = GP_OK;
-    std::thread ta([&] { rc_a = write_records(c, p, ra, 0, path_a); });  // A and B files side by side
-    const int rc_b = write_records(c, p, rb, 1, path_b);
+    std::thread ta([&] {  // A and B files side by side
+        rc_a = t.p ? write_lines(c, t.p.get(), t.bytes_a, path_a) : write_records(c, j.p, j.ra, 0, path_a);
+    });
+    const int rc_b = t.p ? write_lines(c, t.p.get() + t.bytes_a, t.bytes - t.bytes_a, path_b)
+                         : write_records(c, j.p, j.rb, 1, path_b);
     ta.join();
     if (rc_a) return rc_a;
     if (rc_b) return rc_b;
-    st->written_a = (int64_t)ra.size();
-    st->written_b = (int64_t)rb.size();
+    st->written_a = t.p ? t.n_a : (int64_t)j.ra.size();
+    st->written_b = t.p ? t.n - t.n_a : (int64_t)j.rb.size();
     return GP_OK;
 }
 
@@ -989,6 +1013,7 @@ int generate_resumable(gp_ctx* c, const GenPlan& p, const std::string& spec,
     std::vector<JobRun> jobs(1);
     JobRun& j = jobs[0];
     j.p = p;
+    j.want_text = c->out_format == GP_FORMAT_TEXT;
     FILE* probe = fopen(ckpt, "rb");
     if (probe) {
         fclose(probe);
@@ -1012,7 +1037,7 @@ int generate_resumable(gp_ctx* c, const GenPlan& p, const std::string& spec,
         if (rc) return rc;
         if (done) *done = 0;
     } else {
-        rc = finish(c, p, j.ra, j.rb, path_a, path_b, &st);
+        rc = finish(c, j, path_a, path_b, &st);
         if (rc) return rc;
         remove(ckpt);
         if (done) *done = 1;
@@ -1073,12 +1098,13 @@ int gp_generate(gp_ctx* c, int order, int compress, int paf, int proc_id, int pr
     std::vector<std::pair<gp::u128, gp::u128>> ranges = shard_ranges(p, proc_id, proc_num);
     std::vector<JobRun> jobs(1);
     jobs[0].p = p;
+    jobs[0].want_text = c->out_format == GP_FORMAT_TEXT;
     jobs[0].ranges = std::move(ranges);
     rc = run_batch(c, jobs, single_job_cfg(), nullptr);
     if (rc) return rc;
     st = jobs[0].st;
     const auto tf = std::chrono::steady_clock::now();
-    rc = finish(c, p, jobs[0].ra, jobs[0].rb, path_a, path_b, &st);
+    rc = finish(c, jobs[0], path_a, path_b, &st);
     if (rc) return rc;
     if (getenv("GP_GEN_TIMING")) fprintf(stderr, "[gen] files %.4f s\n", since(tf));
     st.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1104,11 +1130,12 @@ int gp_generate_window(gp_ctx* c, int order, int compress, int paf, uint64_t beg
     if (hi > space) hi = space;
     std::vector<JobRun> jobs(1);
     jobs[0].p = p;
+    jobs[0].want_text = c->out_format == GP_FORMAT_TEXT;
     if (lo < hi) jobs[0].ranges.emplace_back(lo, hi);
     rc = run_batch(c, jobs, single_job_cfg(), nullptr);
     if (rc) return rc;
     st = jobs[0].st;
-    rc = finish(c, p, jobs[0].ra, jobs[0].rb, path_a, path_b, &st);
+    rc = finish(c, jobs[0], path_a, path_b, &st);
     if (rc) return rc;
     st.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (stats) *stats = st;
@@ -1156,6 +1183,7 @@ extern "C" int gp_generate_batch(gp_ctx* c, const gp_gen_job* jobs, int njobs, i
         }
     }
     int iters = 0;
+    for (auto& j : run) j.want_text = c->out_format == GP_FORMAT_TEXT;
     int rc = run_batch(c, run, bc, &iters);
     if (rc) return rc;
     const auto tf = std::chrono::steady_clock::now();
@@ -1165,7 +1193,7 @@ extern "C" int gp_generate_batch(gp_ctx* c, const gp_gen_job* jobs, int njobs, i
         std::vector<std::thread> th;
         for (int i = 0; i < njobs; ++i)
             th.emplace_back([&, i] {
-                rcs[i] = finish(c, run[i].p, run[i].ra, run[i].rb, jobs[i].path_a, jobs[i].path_b, &run[i].st);
+                rcs[i] = finish(c, run[i], jobs[i].path_a, jobs[i].path_b, &run[i].st);
             });
         for (auto& t : th) t.join();
         for (int i = 0; i < njobs; ++i)

@@ -299,6 +299,7 @@ int gp_ctx_destroy(gp_ctx* c) {
     for (auto& b : c->ux) b.release();
     for (auto& b : c->eq) b.release();
     for (auto& b : c->st) b.release();
+    for (auto& b : c->gt) b.release();
     for (auto& b : c->hscratch) b.release();
     if (c->s_comp) cudaStreamDestroy(c->s_comp);
     if (c->s_copy) cudaStreamDestroy(c->s_copy);

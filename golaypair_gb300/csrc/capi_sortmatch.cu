@@ -725,15 +725,6 @@ struct SurvGeom {
     int alpha[16];
 };
 
-__device__ __forceinline__ int ndigits_u(unsigned v) {
-    int n = 1;
-    while (v >= 10) {
-        v /= 10;
-        ++n;
-    }
-    return n;
-}
-
 __device__ __forceinline__ void rec_word(const uint8_t* r, int word_bytes, uint64_t& lo, uint64_t& hi) {
     lo = hi = 0;
     for (int i = 0; i < word_bytes; ++i) {
@@ -770,7 +761,7 @@ __global__ void surv_len_kernel(const uint8_t* recs, int64_t n, SurvGeom g, uint
         const int used = g.bits * g.L;
         const bool high = used < 64 ? (lo >> used) != 0 || hi != 0 : (used < 128 && (hi >> (used - 64)) != 0);
         uint32_t l = 3 + 1 + 1;  // "PSD", the space after the signature, the newline
-        for (int k = 0; k < g.L - 1; ++k) l += (uint32_t)ndigits_u(rec_sig(r, g, k));
+        for (int k = 0; k < g.L - 1; ++k) l += (uint32_t)gp::dec_digits(rec_sig(r, g, k));
         bool ok = !high;
         for (int j = 0; j < g.L; ++j) {
             const int d = rec_digit(lo, hi, g.bits, g.L, j);
@@ -779,23 +770,12 @@ __global__ void surv_len_kernel(const uint8_t* recs, int64_t n, SurvGeom g, uint
                 break;
             }
             const int v = g.alpha[d];
-            l += (uint32_t)(ndigits_u((unsigned)(v < 0 ? -v : v)) + (v < 0) + 1);
+            l += (uint32_t)(gp::dec_digits((unsigned)(v < 0 ? -v : v)) + (v < 0) + 1);
         }
         if (!ok) atomicExch(bad, 1);
         len[i] = l;
         atomicMax(maxlen, l - 1);
     }
-}
-
-__device__ __forceinline__ char* put_dec(char* o, unsigned v) {
-    char tmp[10];
-    int n = 0;
-    do {
-        tmp[n++] = (char)('0' + v % 10);
-        v /= 10;
-    } while (v);
-    while (n) *o++ = tmp[--n];
-    return o;
 }
 
 // each record's line (src/utils/io.cpp:14-36) at its offset
@@ -810,12 +790,12 @@ __global__ void surv_format_kernel(const uint8_t* recs, int64_t n, SurvGeom g, c
         *o++ = 'P';
         *o++ = 'S';
         *o++ = 'D';
-        for (int k = 0; k < g.L - 1; ++k) o = put_dec(o, rec_sig(r, g, k));
+        for (int k = 0; k < g.L - 1; ++k) o = gp::put_dec(o, rec_sig(r, g, k));
         *o++ = ' ';
         for (int j = 0; j < g.L; ++j) {
             const int v = g.alpha[rec_digit(lo, hi, g.bits, g.L, j)];
             if (v < 0) *o++ = '-';
-            o = put_dec(o, (unsigned)(v < 0 ? -v : v));
+            o = gp::put_dec(o, (unsigned)(v < 0 ? -v : v));
             *o++ = ' ';
         }
         *o = '\n';

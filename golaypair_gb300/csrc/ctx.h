@@ -155,6 +155,7 @@ struct gp_ctx {
     DevBuf ux[66];
     DevBuf eq[20];  // scratch of the equivalence filter, and of sort and match:
     DevBuf st[29];  // kept between calls while small (KeepSmall)
+    DevBuf gt[8];   // the same for the generation stage's text
     HostPinned hscratch[4];
     // batched generation: one stream per job branch, fork/join events
     static constexpr int kJobStreams = 8;

@@ -1,9 +1,30 @@
-// pair_text.cuh -- pair lines on the device: "%d " per entry of a, " ", "%d "
-// per entry of b, newline (src/utils/io.cpp:75-95).
+// pair_text.cuh -- numbers and lines as text on the device.  Pair lines: "%d "
+// per entry of a, " ", "%d " per entry of b, newline (src/utils/io.cpp:75-95).
 #pragma once
 #include <cstdint>
 
 namespace gp {
+
+__device__ __forceinline__ int dec_digits(unsigned v) {
+    int n = 1;
+    while (v >= 10) {
+        v /= 10;
+        ++n;
+    }
+    return n;
+}
+
+// Writes v in decimal; returns the end.
+__device__ __forceinline__ char* put_dec(char* o, unsigned v) {
+    char tmp[10];
+    int n = 0;
+    do {
+        tmp[n++] = (char)('0' + v % 10);
+        v /= 10;
+    } while (v);
+    while (n) *o++ = tmp[--n];
+    return o;
+}
 
 // Bytes of "%d ".
 __device__ __forceinline__ int value_bytes(int v) {
