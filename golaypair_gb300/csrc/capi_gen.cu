@@ -12,7 +12,6 @@
 // candidate files.  Records that were drained to the host meanwhile, or go to
 // binary files, are ordered and formatted by host threads.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -260,10 +259,6 @@ gp::u128 range_words(const JobRun& j) {
     return t;
 }
 
-uint4 to_u4(gp::u128 w) {
-    return make_uint4((uint32_t)w, (uint32_t)(w >> 32), (uint32_t)(w >> 64), (uint32_t)(w >> 96));
-}
-
 // Copies job j's records to the host and appends them to its A/B lists.
 int drain_records(gp_ctx* c, JobRun& j, uint8_t* arena, int64_t nrec) {
     if (nrec <= 0) return GP_OK;
@@ -305,24 +300,19 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     if (nj < 1 || nj > gp::kMaxEnumJobs) return c->fail(GP_ERR_ARG, "batch of %d jobs (1..%d)", nj, gp::kMaxEnumJobs);
     cudaStream_t s = c->s_comp;
     if (!c->ensure_job_streams()) return c->fail(GP_ERR_CUDA, "cannot create job streams");
-    // ---- rank windows, shared out over the jobs by words in range
+    // ---- rank windows: as many for every job, because the jobs meet their
+    // capacities or end at different times and the others' windows have to
+    // keep all threads busy then (five jobs: 22.7 + 6.6 ms of enumeration with
+    // one such share for all, 14.5 + 3.2 with one each)
     const int64_t threads = (int64_t)c->num_sms * 8 * 256;
     const int64_t target = threads * std::max(1, cfg.windows_per_thread);
-    double total_words = 0;
-    for (auto& j : jobs) total_words += (double)range_words(j);
     // Each range is cut into windows of wsize words (the last one shorter);
-    // the windows are laid out job by job, range by range, and built by
-    // host threads over chunks of consecutive windows (each chunk steps its
-    // own rank counter from its first window).
-    struct Chunk {
-        int ji;
-        gp::u128 r0, r1, wsize;  // the range and the job's window size
-        int64_t w0, nw;          // first window of the chunk (in its range), count
-        int64_t out;             // index of its first window in cur / end / wjob
-    };
-    std::vector<Chunk> chunks;
+    // the windows are laid out job by job, range by range.  The device makes
+    // their first words (launch_windows).
+    std::vector<gp::WinRange> wranges;
+    gp::WinJobs wjobs{};
     int64_t nwin = 0, nwin_narrow = 0;
-    constexpr int64_t kChunkWindows = 8192;
+    auto to_p = [](gp::u128 v) { return gp::U128p{(uint64_t)v, (uint64_t)(v >> 64)}; };
     // the windows of jobs whose words fit 63 bits first: they go to the
     // enumerator's 64-bit instantiation, the others to a second launch
     auto narrow_job = [&](int ji) { return jobs[ji].p.b * jobs[ji].p.L <= 63; };
@@ -330,55 +320,18 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     for (int ji = 0; ji < nj; ++ji) {
         if (narrow_job(ji) != (pass == 0)) continue;
         JobRun& j = jobs[ji];
+        const gp::u128 space = gp::upow(j.p.k, j.p.L);
+        wjobs.job[ji] = {j.p.k, j.p.b, j.p.L, to_p(space), to_p(gp::rank_to_word(space - 1, j.p.k, j.p.b, j.p.L) + 1)};
         const gp::u128 words = range_words(j);
         if (words == 0) continue;
-        int64_t nw = (int64_t)((double)target * ((double)words / total_words));
-        if (nw < 256) nw = 256;
-        gp::u128 wsize = words / (gp::u128)nw;
+        gp::u128 wsize = words / (gp::u128)target;
         if (wsize < 1) wsize = 1;
         for (auto& r : j.ranges) {
             if (r.first >= r.second) continue;
-            const int64_t n = (int64_t)((r.second - r.first + wsize - 1) / wsize);
-            for (int64_t w0 = 0; w0 < n; w0 += kChunkWindows) {
-                chunks.push_back({ji, r.first, r.second, wsize, w0, std::min(kChunkWindows, n - w0), nwin});
-                nwin += std::min(kChunkWindows, n - w0);
-            }
+            wranges.push_back({to_p(r.first), to_p(r.second), to_p(wsize), nwin, ji});
+            nwin += (int64_t)((r.second - r.first + wsize - 1) / wsize);
         }
         if (pass == 0) nwin_narrow = nwin;
-    }
-    std::vector<uint4> cur(nwin), end(nwin);
-    std::vector<uint8_t> wjob(nwin);
-    {
-        std::atomic<size_t> next{0};
-        auto work = [&]() {
-            for (size_t ci = next++; ci < chunks.size(); ci = next++) {
-                const Chunk& ch = chunks[ci];
-                const GenPlan& p = jobs[ch.ji].p;
-                const gp::u128 space = gp::upow(p.k, p.L);
-                const gp::u128 maxw = gp::rank_to_word(space - 1, p.k, p.b, p.L);
-                gp::u128 lo = ch.r0 + (gp::u128)ch.w0 * ch.wsize;
-                gp::RankStepper step(lo, ch.wsize < space ? ch.wsize : space, p.k, p.b, p.L);
-                for (int64_t i = 0; i < ch.nw; ++i, lo += ch.wsize) {
-                    const bool whole = lo + ch.wsize <= ch.r1;  // the window ends wsize words on
-                    const gp::u128 hi = whole ? lo + ch.wsize : ch.r1;
-                    const int64_t o = ch.out + i;
-                    cur[o] = to_u4(step.word());
-                    step.advance();
-                    if (hi >= space)
-                        end[o] = to_u4(maxw + 1);
-                    else if (whole)
-                        end[o] = to_u4(step.word());
-                    else
-                        end[o] = to_u4(gp::rank_to_word(hi, p.k, p.b, p.L));
-                    wjob[o] = (uint8_t)ch.ji;
-                }
-            }
-        };
-        const unsigned nt = (unsigned)std::min<size_t>(chunks.size(), std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
-        std::vector<std::thread> th;
-        for (unsigned t = 1; t < nt; ++t) th.emplace_back(work);
-        work();
-        for (auto& t : th) t.join();
     }
     t_win = since(tb);
     // ---- capacities and the device arena
@@ -419,6 +372,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     const size_t off_cur = take((size_t)nwin * 16);
     const size_t off_end = take((size_t)nwin * 16);
     const size_t off_wjob = take((size_t)nwin);
+    const size_t off_wranges = take(wranges.size() * sizeof(gp::WinRange));
     for (int ji = 0; ji < nj; ++ji) {
         JobRun& j = jobs[ji];
         const gp::u128 words = range_words(j);
@@ -481,9 +435,11 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_rtab, rtab.data(), rtab.size(), cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_ctab, ctab.data(), ctab.size() * 8, cudaMemcpyHostToDevice, s));
     if (nwin) {
-        GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_cur, cur.data(), (size_t)nwin * 16, cudaMemcpyHostToDevice, s));
-        GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_end, end.data(), (size_t)nwin * 16, cudaMemcpyHostToDevice, s));
-        GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_wjob, wjob.data(), (size_t)nwin, cudaMemcpyHostToDevice, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(A + off_wranges, wranges.data(), wranges.size() * sizeof(gp::WinRange),
+                                       cudaMemcpyHostToDevice, s));
+        GP_CUDA_TRY(c, gp::launch_windows(wjobs, reinterpret_cast<const gp::WinRange*>(A + off_wranges),
+                                          (int64_t)wranges.size(), nwin, reinterpret_cast<uint4*>(A + off_cur),
+                                          reinterpret_cast<uint4*>(A + off_end), A + off_wjob, s));
     }
     GP_CUDA_TRY(c, cudaMemsetAsync(ctr, 0, kCounterWords * 8, s));
     gp::EnumArgs ea;
@@ -691,8 +647,11 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
                                                                              stop->start).count() >= stop->max_seconds))) {
             // unfinished windows hold the next word to visit (a finished
             // window holds its end): [rank(cur), rank(end)) is still to do
-            std::vector<uint4> hcur(nwin);
+            std::vector<uint4> hcur(nwin), end(nwin);
+            std::vector<uint8_t> wjob(nwin);
             GP_CUDA_TRY(c, cudaMemcpy(hcur.data(), A + off_cur, (size_t)nwin * 16, cudaMemcpyDeviceToHost));
+            GP_CUDA_TRY(c, cudaMemcpy(end.data(), A + off_end, (size_t)nwin * 16, cudaMemcpyDeviceToHost));
+            GP_CUDA_TRY(c, cudaMemcpy(wjob.data(), A + off_wjob, (size_t)nwin, cudaMemcpyDeviceToHost));
             auto from_u4 = [](uint4 v) {
                 return ((gp::u128)v.w << 96) | ((gp::u128)v.z << 64) | ((gp::u128)v.y << 32) | v.x;
             };

@@ -221,8 +221,9 @@ __device__ __forceinline__ bool job_full(const EnumJob& j) {
 // windows' serial steps at the end.  An order-57 window of 2^32 words (2.3 G
 // necklaces, 208 M candidates): 2.6 ms of kernel time, 9.4 when each lane took,
 // loaded and checked its own windows and every 32 candidates took an atomic,
-// 15.1 with blocks of two digits taken a row at a time; five orders: 27, 48 and
-// 87 ms.  Blocks per SM 4, 5, 6: 2.56, 2.53, 2.70 and 27.0, 27.2, 30.4 ms.
+// 15.1 with blocks of two digits taken a row at a time; five orders: 18, 48 and
+// 87 ms (27 with as many windows for all five as for one).  Blocks per SM
+// 4, 5, 6: 2.56, 2.53, 2.70 and 27.0, 27.2, 30.4 ms.
 //
 // NARROW: every job's words fit 63 bits, so a word and its window end are
 // 64-bit values (the high halves are zero and drop out of the registers).
@@ -494,6 +495,62 @@ __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
     if (threadIdx.x < a.njobs && sh.visited[threadIdx.x]) atomicAdd(sh.jobs[threadIdx.x].necklaces, sh.visited[threadIdx.x]);
 }
 
+using u128d = unsigned __int128;
+
+__device__ __forceinline__ u128d u128_of(U128p v) { return ((u128d)v.hi << 64) | v.lo; }
+
+// Packed word of the word with rank r: the rank's base-k digits, by 32-bit
+// pieces while it is longer than 64 bits.
+__device__ __forceinline__ W128 word_of_rank(u128d r, const WinJobs::Job& j) {
+    W128 w = {0, 0};
+    const uint64_t k = (uint64_t)j.k;
+    uint64_t lo = (uint64_t)r, hi = (uint64_t)(r >> 64);
+    for (int q = 0; q < j.L; ++q) {
+        uint64_t d;
+        if (hi) {
+            uint64_t piece[4] = {hi >> 32, hi & 0xFFFFFFFFull, lo >> 32, lo & 0xFFFFFFFFull};
+            d = 0;
+            for (int i = 0; i < 4; ++i) {
+                const uint64_t x = (d << 32) | piece[i];
+                piece[i] = x / k;
+                d = x - piece[i] * k;
+            }
+            hi = (piece[0] << 32) | piece[1];
+            lo = (piece[2] << 32) | piece[3];
+        } else {
+            const uint64_t x = lo / k;
+            d = lo - x * k;
+            lo = x;
+        }
+        w = bor(w, shl({d, 0}, j.b * q));
+    }
+    return w;
+}
+
+// A thread per window: two rank conversions, 33 us for 311,000 windows
+// (2.5 to 3.5 ms on host threads, and their copy).
+__global__ void window_words_kernel(WinJobs jobs, const WinRange* ranges, int64_t nranges, int64_t nwin, uint4* cur,
+                                    uint4* end, uint8_t* win_job) {
+    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nwin; w += (int64_t)gridDim.x * blockDim.x) {
+        int64_t a = 0, z = nranges;  // the last range whose first window is w or before
+        while (z - a > 1) {
+            const int64_t m = (a + z) / 2;
+            if (ranges[m].first <= w)
+                a = m;
+            else
+                z = m;
+        }
+        const WinRange& r = ranges[a];
+        const WinJobs::Job& j = jobs.job[r.job];
+        const u128d size = u128_of(r.wsize), last = u128_of(r.r1);
+        const u128d lo = u128_of(r.r0) + (u128d)(w - r.first) * size;
+        const u128d hi = last - lo > size ? lo + size : last;
+        cur[w] = to_u4(word_of_rank(lo, j));
+        end[w] = hi >= u128_of(j.space) ? to_u4(w128(j.past)) : to_u4(word_of_rank(hi, j));
+        win_job[w] = (uint8_t)r.job;
+    }
+}
+
 template <bool NARROW>
 cudaError_t launch_enumerate_t(const EnumArgs& a, int num_sms, cudaStream_t st, int variant) {
     // one wave of resident blocks: windows are handed out dynamically
@@ -519,6 +576,15 @@ cudaError_t launch_enumerate_t(const EnumArgs& a, int num_sms, cudaStream_t st, 
 }
 
 }  // namespace
+
+cudaError_t launch_windows(const WinJobs& jobs, const WinRange* ranges, int64_t nranges, int64_t nwin, uint4* cur,
+                           uint4* end, uint8_t* win_job, cudaStream_t st) {
+    if (nwin <= 0 || nranges <= 0) return cudaSuccess;
+    const int64_t blocks = (nwin + 255) / 256;
+    window_words_kernel<<<(unsigned)(blocks < 65536 ? blocks : 65536), 256, 0, st>>>(jobs, ranges, nranges, nwin, cur,
+                                                                                     end, win_job);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_enumerate(const EnumArgs& a, int num_sms, cudaStream_t st, int variant) {
     if (a.nwin <= 0) return cudaSuccess;

@@ -90,6 +90,25 @@ struct EnumArgs {
     int narrow;                // 1: every job's word fits 63 bits (b * L <= 63): the 64-bit kernel
 };
 
+// The windows of a range of word ranks [r0, r1): wsize words each, the last
+// one shorter; windows first, first + 1, ...
+struct WinRange {
+    U128p r0, r1, wsize;
+    int64_t first;
+    int64_t job;
+};
+
+struct WinJobs {
+    struct Job {
+        int k, b, L;
+        U128p space, past;  // k^L; the number after the last word
+    } job[kMaxEnumJobs];
+};
+
+// cur, end, win_job of windows 0 .. nwin - 1 (ranges: device, by first).
+cudaError_t launch_windows(const WinJobs& jobs, const WinRange* ranges, int64_t nranges, int64_t nwin, uint4* cur,
+                           uint4* end, uint8_t* win_job, cudaStream_t st);
+
 // variant: 256-thread blocks per SM, 0: 4 (64 registers), 1: 6 (40), 2: 5 (48)
 cudaError_t launch_enumerate(const EnumArgs& a, int num_sms, cudaStream_t st, int variant = 0);
 
