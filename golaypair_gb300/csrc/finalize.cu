@@ -1,7 +1,7 @@
 // finalize.cu -- exact per-survivor work after the tensor-core filter.
 //
-// For every candidate whose mask bit survived the guarded filter, one warp:
-//   * computes all L PSD bins in FP64 (src/utils/fourier.cpp:25-43) and
+// For every candidate whose mask bit survived the guarded filter, a warp:
+//   * computes the PSD bins 0..L/2 in FP64 (src/utils/fourier.cpp:25-43) and
 //     re-applies the exact filter (fourier.cpp:45-52);
 //   * for each role (A / B) of the candidate, optionally checks that the
 //     sequence is the lexicographic minimum of its orbit, as isCanonical
@@ -11,6 +11,8 @@
 //   * writes a record: the word, the role and the signature
 //     rint(psd[k]) (or bound - rint(psd[k]) for inverted roles), k = 1..L-1
 //     (src/utils/io.cpp:14-36).
+#include <algorithm>
+
 #include "gp_device.cuh"
 #include "finalize.h"
 #include "rows.cuh"
@@ -56,103 +58,159 @@ __global__ void mask_to_list_multi_kernel(ListMultiArgs a) {
     list_bits(j.mask, j.n, j.n_dev, j.out, j.count, j.cap, a.status);
 }
 
+// Rows a warp computes the spectra of at once: 32 lanes over the lanes that a
+// row's L/2 + 1 bins take, to the next power of two.  The spectra are bound by
+// the FP64 pipe (two DFMA per cycle and SM on GB300), as in psd_fp64.cu: x is
+// real, so bins above L/2 repeat those below and a bin needs only the folded
+// sums x_j + x_{L-j} and x_j - x_{L-j} (exact integers, made once per row):
+// a quarter of the DFMAs of L bins of L terms by 32 lanes.  1.4 M survivors of
+// five orders: 7.3 ms, 10.0 with the direct sums.
+__host__ __device__ __forceinline__ int rows_at_once(int L) {
+    int r = 8;
+    while (r > 1 && 32 / r < L / 2 + 1) r /= 2;
+    return r;
+}
+
+// shared memory: the twiddles, then per warp its rows' folded sums, spectra
+// and values
+struct FinalizeLayout {
+    size_t fold, psd, x, per_warp;
+};
+__host__ __device__ __forceinline__ FinalizeLayout finalize_layout(int L) {
+    const size_t R = (size_t)rows_at_once(L), H = (size_t)L / 2;
+    FinalizeLayout s;
+    s.fold = 0;
+    s.psd = R * (H + 1) * sizeof(double2);
+    s.x = s.psd + R * (H + 1) * sizeof(double);
+    s.per_warp = (s.x + R * L + 15) & ~size_t(15);
+    return s;
+}
+
 __device__ __forceinline__ void finalize_rows(const FinalizeArgs& a, double2* sh_tw) {
-    const int L = a.src.L;
-    double* psd_all = reinterpret_cast<double*>(sh_tw + L);
-    int8_t* xs_all = reinterpret_cast<int8_t*>(psd_all + kWarps * L);
+    const int L = a.src.L, H = L / 2, J = (L - 1) / 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* psd = psd_all + warp * L;
-    int8_t* xs = xs_all + warp * kMaxLen;
+    const int R = rows_at_once(L), G = 32 / R;  // G lanes to a row
+    const FinalizeLayout lay = finalize_layout(L);
+    uint8_t* mine = reinterpret_cast<uint8_t*>(sh_tw + L) + (size_t)warp * lay.per_warp;
+    double2* fold_all = reinterpret_cast<double2*>(mine + lay.fold);
+    double* psd_all = reinterpret_cast<double*>(mine + lay.psd);
+    int8_t* xs_all = reinterpret_cast<int8_t*>(mine + lay.x);
     for (int m = threadIdx.x; m < L; m += blockDim.x) sh_tw[m] = make_double2(a.tw[2 * m], a.tw[2 * m + 1]);
     __syncthreads();
     int64_t cnt = (int64_t)*a.n_idx;
     if (cnt > a.idx_cap) cnt = a.idx_cap;
-    const int H = L / 2;
-    for (int64_t i = (int64_t)blockIdx.x * kWarps + warp; i < cnt; i += (int64_t)gridDim.x * kWarps) {
-        const uint32_t row = a.idx[i];
-        if (lane == 0) decode_row(a.src, row, xs);
+    unsigned passed = 0;  // lane 0: rows that pass
+    for (int64_t i0 = ((int64_t)blockIdx.x * kWarps + warp) * R; i0 < cnt; i0 += (int64_t)gridDim.x * kWarps * R) {
+        const int n = (int)(cnt - i0 < R ? cnt - i0 : R);
+        const int g = lane / G, gl = lane % G;  // this lane's row and place in it
+        const bool in = g < n;
+        const uint32_t my_row = in ? a.idx[i0 + g] : 0u;
+        int8_t* xg = xs_all + g * L;
+        double2* fold = fold_all + g * (H + 1);
+        double* pg = psd_all + g * (H + 1);
+        if (in) {
+            if (a.src.seqs) {
+                for (int j = gl; j < L; j += G) xg[j] = a.src.seqs[(int64_t)my_row * L + j];
+            } else {
+                const uint4 w = a.src.words[my_row];
+                const uint64_t lo = ((uint64_t)w.y << 32) | w.x, hi = ((uint64_t)w.w << 32) | w.z;
+                for (int j = gl; j < L; j += G)
+                    xg[j] = (int8_t)(2 * word_digit(lo, hi, a.src.pack_bits, L, j) - a.src.alpha_c);
+            }
+        }
+        __syncwarp();
+        if (in)
+            for (int j = 1 + gl; j <= J; j += G)
+                fold[j] = make_double2((double)(xg[j] + xg[L - j]), (double)(xg[j] - xg[L - j]));
         __syncwarp();
         bool fail = false;
-        for (int k = lane; k < L; k += 32) {
-            double re = 0.0, im = 0.0;
-            int m = 0;
-            for (int j = 0; j < L; ++j) {
-                const double v = (double)xs[j];
-                const double2 w = sh_tw[m];
-                re = fma(v, w.x, re);
-                im = fma(-v, w.y, im);
-                m += k;
-                if (m >= L) m -= L;
-            }
-            const double p = re * re + im * im;
-            psd[k] = p;
-            if (k >= 1 && k <= H && p > a.thr) fail = true;
-        }
-        fail = __any_sync(0xFFFFFFFFu, fail);
-        __syncwarp();
-        if (fail) continue;
-        if (lane == 0) atomicAdd(a.psd_pass, 1ull);
-        if (a.prune_tab) {
-            // p(L/2) is the square of the alternating sum and p(L/3) the norm
-            // of an Eisenstein integer: both exact integers here
-            bool keep = true;
-            if (L % 2 == 0) {
-                const int m = a.bound - __double2int_rn(psd[L / 2]);
-                keep = m >= 0 && m <= a.bound && (a.prune_tab[m] & 1);
-            }
-            if (keep && L % 3 == 0) {
-                const int m = a.bound - __double2int_rn(psd[L / 3]);
-                keep = m >= 0 && m <= a.bound && (a.prune_tab[m] & 2);
-            }
-            if (!keep) continue;
-        }
-        const uint8_t roles = a.roles ? a.roles[row] : a.fixed_role;
-        for (int r = 0; r < 2; ++r) {
-            if (!((roles >> r) & 1)) continue;
-            bool canonical = true;
-            if (a.check_canonical) {
-                // r = 0: affine maps (constructGenerators(0, L)); r = 1: dihedral
-                const int nmul = r == 0 ? a.n_units : (L > 2 ? 2 : 1);
-                const int64_t G = (int64_t)nmul * L;
-                bool less = false;
-                for (int64_t g = lane; g < G && !less; g += 32) {
-                    const int mi = (int)(g / L);
-                    const int u = r == 0 ? a.units[mi] : (mi == 0 ? 1 : L - 1);
-                    const int t = (int)(g % L);
-                    int idx = t;
-                    for (int q = 0; q < L; ++q) {
-                        const int v = xs[idx], x = xs[q];
-                        if (v != x) {
-                            less = v < x;
-                            break;
-                        }
-                        idx += u;
-                        if (idx >= L) idx -= L;
-                    }
+        if (in) {
+            const double x0 = (double)xg[0], xh = L % 2 == 0 ? (double)xg[H] : 0.0;
+            for (int k = gl; k <= H; k += G) {
+                double re = k % 2 ? x0 - xh : x0 + xh, im = 0.0;
+                int m = k;
+                for (int j = 1; j <= J; ++j) {
+                    const double2 w = sh_tw[m], f = fold[j];
+                    re = fma(f.x, w.x, re);
+                    im = fma(f.y, w.y, im);
+                    m += k;
+                    if (m >= L) m -= L;
                 }
-                canonical = !__any_sync(0xFFFFFFFFu, less);
+                const double p = re * re + im * im;
+                pg[k] = p;
+                if (k >= 1 && p > a.thr) fail = true;
             }
-            if (!canonical) continue;
-            unsigned long long pos = 0;
-            if (lane == 0) pos = atomicAdd(a.rec_count, 1ull);
-            pos = __shfl_sync(0xFFFFFFFFu, pos, 0);
-            if ((int64_t)pos >= a.rec_cap) {
-                if (lane == 0) atomicCAS(a.status, 0, GP_KSTATUS_OVERFLOW);
-                continue;
+        }
+        const uint32_t failed = __ballot_sync(0xFFFFFFFFu, fail);
+        __syncwarp();
+        for (int q = 0; q < n; ++q) {  // its rows one by one, by the whole warp
+            if ((failed >> (q * G)) & (G == 32 ? 0xFFFFFFFFu : (1u << G) - 1u)) continue;
+            ++passed;
+            const uint32_t row = __shfl_sync(0xFFFFFFFFu, my_row, q * G);
+            const int8_t* xs = xs_all + q * L;
+            const double* psd = psd_all + q * (H + 1);
+            if (a.prune_tab) {
+                // p(L/2) is the square of the alternating sum and p(L/3) the norm
+                // of an Eisenstein integer: both exact integers here
+                bool keep = true;
+                if (L % 2 == 0) {
+                    const int m = a.bound - __double2int_rn(psd[L / 2]);
+                    keep = m >= 0 && m <= a.bound && (a.prune_tab[m] & 1);
+                }
+                if (keep && L % 3 == 0) {
+                    const int m = a.bound - __double2int_rn(psd[L / 3]);
+                    keep = m >= 0 && m <= a.bound && (a.prune_tab[m] & 2);
+                }
+                if (!keep) continue;
             }
-            const bool inv = (a.invert_roles >> r) & 1;
-            for (int k = 1 + lane; k < L; k += 32) {
-                const int s = __double2int_rn(psd[k]);
-                a.rec_sig[pos * (L - 1) + (k - 1)] = (uint16_t)(inv ? a.bound - s : s);
-            }
-            if (lane == 0) {
-                a.rec_words[pos] = a.src.words ? a.src.words[row] : make_uint4(row, 0, 0, 0);
-                if (a.rec_role) a.rec_role[pos] = (uint8_t)(1 << r);
-                if (a.rec_src) a.rec_src[pos] = row;
+            const uint8_t roles = a.roles ? a.roles[row] : a.fixed_role;
+            for (int r = 0; r < 2; ++r) {
+                if (!((roles >> r) & 1)) continue;
+                bool canonical = true;
+                if (a.check_canonical) {
+                    // r = 0: affine maps (constructGenerators(0, L)); r = 1: dihedral
+                    const int nmul = r == 0 ? a.n_units : (L > 2 ? 2 : 1);
+                    const int maps = nmul * L;
+                    bool less = false;
+                    for (int e = lane; e < maps && !less; e += 32) {
+                        const int mi = e / L;
+                        const int u = r == 0 ? a.units[mi] : (mi == 0 ? 1 : L - 1);
+                        int idx = e - mi * L;
+                        for (int d = 0; d < L; ++d) {
+                            const int v = xs[idx], x = xs[d];
+                            if (v != x) {
+                                less = v < x;
+                                break;
+                            }
+                            idx += u;
+                            if (idx >= L) idx -= L;
+                        }
+                    }
+                    canonical = !__any_sync(0xFFFFFFFFu, less);
+                }
+                if (!canonical) continue;
+                unsigned long long pos = 0;
+                if (lane == 0) pos = atomicAdd(a.rec_count, 1ull);
+                pos = __shfl_sync(0xFFFFFFFFu, pos, 0);
+                if ((int64_t)pos >= a.rec_cap) {
+                    if (lane == 0) atomicCAS(a.status, 0, GP_KSTATUS_OVERFLOW);
+                    continue;
+                }
+                const bool inv = (a.invert_roles >> r) & 1;
+                for (int k = 1 + lane; k < L; k += 32) {
+                    const int s = __double2int_rn(psd[k <= H ? k : L - k]);
+                    a.rec_sig[pos * (L - 1) + (k - 1)] = (uint16_t)(inv ? a.bound - s : s);
+                }
+                if (lane == 0) {
+                    a.rec_words[pos] = a.src.words ? a.src.words[row] : make_uint4(row, 0, 0, 0);
+                    if (a.rec_role) a.rec_role[pos] = (uint8_t)(1 << r);
+                    if (a.rec_src) a.rec_src[pos] = row;
+                }
             }
         }
         __syncwarp();
     }
+    if (lane == 0 && passed) atomicAdd(a.psd_pass, (unsigned long long)passed);
 }
 
 __global__ void __launch_bounds__(kWarps * 32) finalize_kernel(FinalizeArgs a) {
@@ -166,9 +224,7 @@ __global__ void __launch_bounds__(kWarps * 32) finalize_multi_kernel(FinalizeMul
     finalize_rows(m.job[blockIdx.y], sh_tw);
 }
 
-size_t finalize_smem(int L) {
-    return sizeof(double2) * L + sizeof(double) * kWarps * L + (size_t)kWarps * kMaxLen;
-}
+size_t finalize_smem(int L) { return sizeof(double2) * L + kWarps * finalize_layout(L).per_warp; }
 
 }  // namespace
 
@@ -210,17 +266,16 @@ cudaError_t launch_finalize_multi(const FinalizeMultiArgs& a, const int64_t* max
                                   cudaStream_t st) {
     if (a.njobs <= 0 || a.njobs > kMaxMultiJobs) return a.njobs == 0 ? cudaSuccess : cudaErrorInvalidValue;
     int64_t rows = 0;
-    int maxL = 1;
+    size_t smem = 0;
     for (int j = 0; j < a.njobs; ++j) {
         rows = max_rows[j] > rows ? max_rows[j] : rows;
-        maxL = a.job[j].src.L > maxL ? a.job[j].src.L : maxL;
+        smem = std::max(smem, finalize_smem(a.job[j].src.L));
     }
     if (rows <= 0) return cudaSuccess;
     int64_t blocks = (rows + kWarps - 1) / kWarps;
     // per job as many blocks as its own launch would take: blocks of a job
     // with fewer rows end at once
     if (blocks > (int64_t)num_sms * 16) blocks = (int64_t)num_sms * 16;
-    const size_t smem = finalize_smem(maxL);
     cudaError_t e =
         cudaFuncSetAttribute(finalize_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
