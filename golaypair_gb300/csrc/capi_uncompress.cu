@@ -39,11 +39,12 @@
 //    vectors and buckets the survivors by (pair, hash bits), one entry per
 //    pair and role that uses the survivor's side;
 //    ux_join_kernel matches each bucket in a shared-memory hash table and
-//    verifies the PAF sums exactly.  No signature is computed on the device.
-// 5. Host: the few matched pairs get their FP64 signatures; a pair is kept
-//    when the two signature strings are equal (the reference's join key),
-//    and the pairs of each input pair are written in the order of the
-//    reference's sorted files (a line, then b line), input pairs in order.
+//    verifies the PAF sums exactly.
+// 5. ux_lines_kernel expands the few matched pairs, computes their FP64
+//    signatures and keeps a pair when the two signature strings are equal
+//    (the reference's join key); the pairs are sorted by input pair and in the
+//    order of the reference's sorted files (a line, then b line), and written
+//    as text, on the device.
 #include <algorithm>
 #include <stdexcept>
 #include <array>
@@ -60,6 +61,7 @@
 
 #include "ctx.h"
 #include "host_math.h"
+#include "pair_text.cuh"
 #include "prims.h"
 
 namespace {
@@ -733,6 +735,176 @@ __global__ void __launch_bounds__(256) ux_join_kernel(JoinArgs a) {
     }
 }
 
+// The matched pairs of a batch: a warp per match.
+//  * its two expansions and their signatures (io.cpp:14-36; x is real: the
+//    bins up to Lnew / 2 of its folded sums, as in psd_fp64.cu);
+//  * whether the signature strings are equal (a carries bound - rint(p));
+//  * its sort key: the input pair, the a-line's characters after "PSD", the
+//    b-sequence's (b-lines are compared where the a-lines are equal, so their
+//    signatures are), 4 bits each; matches that are not kept sort last.
+// Sizes are small (a few thousand matches), so it is bound by its latency: 50 us
+// of a call of 200 order-39 pairs that takes 1.35 ms, and took 3.1 with the
+// matches expanded, formatted and sorted on host threads.
+constexpr int kLineWarps = 4;
+constexpr int kMaxTokenCodes = (kMaxLnew - 1) * 11;  // characters of an int
+constexpr int kMaxLineCodes = kMaxTokenCodes + 2 + 2 * kMaxLnew * 5;  // and "-128 "
+
+struct LineArgs {
+    LevelDev lv;
+    const uint8_t* rows;      // of the batch's sides
+    const uint64_t* matches;  // words of a and b
+    uint64_t n;
+    const double2* tw;        // cos, sin of 2 pi m / Lnew
+    int bound;
+    int W;                    // words of a key
+    int8_t* seqs;             // [n][2 Lnew]
+    uint32_t* keys;           // [n][W]
+    unsigned* kept;
+};
+
+// Codes of v in decimal: '-' 2, digits 3 .. 12 (' ' is 1, nothing 0: the order
+// of the bytes).  Returns how many.
+__device__ __forceinline__ int put_codes(int v, uint8_t* o) {
+    unsigned u = (unsigned)(v < 0 ? -v : v);
+    int n = gp::dec_digits(u) + (v < 0 ? 1 : 0);
+    if (o) {
+        if (v < 0) o[0] = 2;
+        for (int i = n - 1; i >= (v < 0 ? 1 : 0); --i) {
+            o[i] = (uint8_t)(3 + u % 10);
+            u /= 10;
+        }
+    }
+    return n;
+}
+
+// The numbers val(0) .. val(n - 1), a blank after each where blanks, as codes at
+// out, by the whole warp; returns how many codes.
+template <class Val>
+__device__ __forceinline__ int put_numbers(int n, bool blanks, Val val, uint8_t* out) {
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        const int v = k < n ? val(k) : 0;
+        const int mine = k < n ? put_codes(v, nullptr) + (blanks ? 1 : 0) : 0;
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (k < n) {
+            uint8_t* q = out + at + incl - mine;
+            q += put_codes(v, q);
+            if (blanks) *q = 1;
+        }
+        at += __shfl_sync(0xFFFFFFFFu, incl, 31);
+    }
+    __syncwarp();
+    return at;
+}
+
+__global__ void __launch_bounds__(kLineWarps * 32) ux_lines_kernel(LineArgs a) {
+    __shared__ double2 s_tw[kMaxLnew], s_fold[kLineWarps][kMaxLnew / 2];
+    __shared__ int8_t s_x[kLineWarps][2 * kMaxLnew];
+    __shared__ uint8_t s_d[kLineWarps][kMaxL];
+    __shared__ int s_sig[kLineWarps][2][kMaxLnew];
+    __shared__ uint8_t s_code[kLineWarps][kMaxLineCodes], s_tok[kLineWarps][kMaxTokenCodes];
+    const LevelDev& lv = a.lv;
+    const int N = lv.Lnew, H = N / 2, J = (N - 1) / 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int m = threadIdx.x; m < N; m += blockDim.x) s_tw[m] = a.tw[m];
+    __syncthreads();
+    double2* fold = s_fold[warp];
+    uint8_t *code = s_code[warp], *tok = s_tok[warp];
+    for (uint64_t e = (uint64_t)blockIdx.x * kLineWarps + warp; e < a.n; e += (uint64_t)gridDim.x * kLineWarps) {
+        for (int h = 0; h < 2; ++h) {
+            const uint64_t word = a.matches[2 * e + h];
+            const uint8_t* r = a.rows + (word >> kRankBits) * (uint64_t)lv.L;
+            int8_t* x = s_x[warp] + h * N;
+            if (lane == 0) decode_rank(word & kRankMask, r, lv.cnt, lv.L, s_d[warp]);
+            __syncwarp();
+            for (int j = lane; j < N; j += 32) {
+                const int i = j % lv.L, q = j / lv.L;
+                x[j] = lv.vals[((size_t)r[i] * lv.dmax + s_d[warp][i]) * lv.r + q];
+                a.seqs[(2 * e + h) * (uint64_t)N + j] = x[j];
+            }
+            __syncwarp();
+            for (int j = 1 + lane; j <= J; j += 32)
+                fold[j] = make_double2((double)(x[j] + x[N - j]), (double)(x[j] - x[N - j]));
+            __syncwarp();
+            int* sig = s_sig[warp][h];
+            for (int k = 1 + lane; k <= H; k += 32) {
+                double re = (double)(N % 2 ? x[0] : k % 2 ? x[0] - x[H] : x[0] + x[H]), im = 0.0;
+                int m = k;
+                for (int j = 1; j <= J; ++j) {
+                    re = fma(fold[j].x, s_tw[m].x, re);
+                    im = fma(fold[j].y, s_tw[m].y, im);
+                    m += k;
+                    if (m >= N) m -= N;
+                }
+                const int p = __double2int_rn(re * re + im * im);
+                sig[k - 1] = sig[N - k - 1] = h ? p : a.bound - p;
+            }
+            __syncwarp();
+        }
+        const int *sa = s_sig[warp][0], *sb = s_sig[warp][1];
+        const int8_t* x = s_x[warp];
+        int n = put_numbers(N - 1, false, [&](int k) { return sa[k]; }, code);
+        const int nt = put_numbers(N - 1, false, [&](int k) { return sb[k]; }, tok);
+        bool same = n == nt;
+        for (int i = lane; i < n && same; i += 32) same = code[i] == tok[i];
+        const bool keep = __all_sync(0xFFFFFFFFu, same);
+        if (lane == 0) code[n] = 1;
+        n += 1;
+        n += put_numbers(N, true, [&](int k) { return (int)x[k]; }, code + n);
+        if (lane == 0) code[n] = 0;  // an a-line's end sorts below its continuations
+        n += 1;
+        n += put_numbers(N, true, [&](int k) { return (int)x[N + k]; }, code + n);
+        __syncwarp();
+        uint32_t* key = a.keys + e * (uint64_t)a.W;
+        for (int w = lane; w < a.W; w += 32) {
+            uint32_t v = 0;
+            if (w == 0) {
+                v = keep ? (uint32_t)(a.matches[2 * e] >> kRankBits) >> 1 : 0xFFFFFFFFu;
+            } else {
+                for (int i = 0; i < 8; ++i) {
+                    const int c = (w - 1) * 8 + i;
+                    v = (v << 4) | (c < n ? code[c] : 0u);
+                }
+            }
+            key[w] = v;
+        }
+        if (lane == 0 && keep) atomicAdd(a.kept, 1u);
+        __syncwarp();
+    }
+}
+
+// bytes of the lines k0 .. k0 + n - 1 in order, none past the kept ones; and
+// bytes[n] = 0, so that a scan of n + 1 entries gives the total
+__global__ void ux_line_bytes_kernel(const int8_t* seqs, int N, const uint32_t* order, uint64_t k0, uint64_t n,
+                                     const unsigned* kept, uint32_t* bytes) {
+    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k <= n; k += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t b = 0;
+        if (k < n && k0 + k < *kept) {
+            const int8_t* x = seqs + (uint64_t)order[k0 + k] * 2 * N;
+            b = (uint32_t)gp::pair_line_bytes(x, x + N, N);
+        }
+        bytes[k] = b;
+    }
+}
+
+// a warp per line
+__global__ void ux_text_kernel(const int8_t* seqs, int N, const uint32_t* order, uint64_t n, const uint32_t* off,
+                               char* text) {
+    const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t k = w0; k < n; k += nw) {
+        const int8_t* x = seqs + (uint64_t)order[k] * 2 * N;
+        gp::put_pair_line(x, x + N, N, text + off[k]);
+    }
+}
+
 // ------------------------------------------------------------ side planning
 // uncompression.cpp:107-142, one thread per side of a compressed pair:
 //  * the rotation: the first distinct letter (ascending value) with the most
@@ -1144,63 +1316,6 @@ int plan_sides(gp_ctx* c, const Level& lv, const std::vector<uint8_t>& seqs, std
     return GP_OK;
 }
 
-void put_uint(std::string& s, unsigned v) {
-    char tmp[12];
-    int n = 0;
-    do {
-        tmp[n++] = (char)('0' + v % 10);
-        v /= 10;
-    } while (v);
-    while (n) s.push_back(tmp[--n]);
-}
-
-void put_int(std::string& s, int v) {
-    if (v < 0) {
-        s.push_back('-');
-        put_uint(s, (unsigned)(-v));
-    } else {
-        put_uint(s, (unsigned)v);
-    }
-}
-
-// The expansion of a survivor word, on the host.
-void host_expand(const Level& lv, const Side& sd, uint64_t rank, std::vector<int>& x) {
-    std::vector<int> d(lv.L, 0);
-    for (int i = lv.L - 1; i >= 0; --i) {
-        const uint64_t c = lv.rowparts[sd.rows[i]].size();
-        d[i] = (int)(rank % c);
-        rank /= c;
-    }
-    x.assign(lv.Lnew, 0);
-    for (int i = 0; i < lv.L; ++i)
-        for (int q = 0; q < lv.r; ++q) x[i + lv.L * q] = lv.rowparts[sd.rows[i]][d[i]][q];
-}
-
-// "PSD" + signature + " " + sequence (src/utils/io.cpp:14-36; the a-side
-// writes bound - rint(psd)), the line the reference's scratch files hold.
-void candidate_line(const Level& lv, const std::vector<int>& x, bool invert, std::string& line, std::string& seq) {
-    const int N = lv.Lnew, bound = 2 * lv.order - lv.paf;
-    line = "PSD";
-    for (int k = 1; k < N; ++k) {
-        double re = 0, im = 0;
-        for (int j = 0, m = 0; j < N; ++j, m += k, m -= m >= N ? N : 0) {
-            re += x[j] * lv.cs[m];
-            im -= x[j] * lv.sn[m];
-        }
-        const int p = (int)std::nearbyint(re * re + im * im);
-        put_int(line, invert ? bound - p : p);
-    }
-    seq.clear();
-    for (int v : x) {
-        put_int(seq, v);
-        seq.push_back(' ');
-    }
-    line.push_back(' ');
-    line += seq;
-}
-
-std::string signature_token(const std::string& line) { return line.substr(0, line.find(' ')); }
-
 bool slurp(const char* path, std::string& out) {
     FILE* f = fopen(path, "rb");
     if (!f) return false;
@@ -1239,13 +1354,6 @@ unsigned grid_for(uint64_t n, unsigned cap) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g, cap));
 }
 
-// A matched pair of expansions: its two candidate lines (the reference's
-// sorted scratch files' order), the output line and the two sequences.
-struct Match {
-    std::string la, lb, line;
-    std::vector<int> xa, xb;
-};
-
 // The engine over consecutive pairs [p0, p1): device scratch in ux[4..].
 struct Batcher {
     gp_ctx* c;
@@ -1257,8 +1365,11 @@ struct Batcher {
     ScanKernel scan;
     int scan_blocks = 0;
     size_t smem = 0;
-    // the matched pairs of each pair of the batch, in output order
-    std::vector<std::vector<Match>> out;
+    bool want_rows;  // the chain goes on: keep the matched pairs' values
+    // the matched pairs of the batch in output order: lines, and values (2 L'
+    // per pair)
+    std::string text;
+    std::vector<int8_t> out_rows;
 
     // Runs the batch; on overflow of a device list returns GP_ERR_OVERFLOW
     // with *overflowed set, so the caller can halve the batch.
@@ -1308,7 +1419,8 @@ int Batcher::run(int64_t p0, int64_t p1, bool* overflowed) {
         }
     }
     ubeg[nu] = units;
-    out.assign(np_, {});
+    text.clear();
+    out_rows.clear();
     if (units == 0) return GP_OK;
     // capacities: every expansion could pass at small sizes; at large ones
     // a pass rate of 1/8 (order 57: under 1 %), at most 2^30 survivors (8 GB;
@@ -1465,42 +1577,72 @@ int Batcher::run(int64_t p0, int64_t p1, bool* overflowed) {
     if (rc) return rc;
     const uint64_t nm = hc[2];
     if (nm == 0) return GP_OK;
-    std::vector<uint64_t> hm(nm * 2);
-    GP_CUDA_TRY(c, cudaMemcpy(hm.data(), dm.p, nm * 16, cudaMemcpyDeviceToHost));
-    // signatures of the matched expansions; the reference joins on the
-    // signature string, which the PAF condition implies up to FP64 rounding
-    std::vector<Match> items(nm);
-    std::vector<char> keep(nm, 0);
-    std::vector<int64_t> pair_of(nm);
-    auto work = [&](uint64_t lo, uint64_t hi) {
-        std::vector<int> xa, xb;
-        std::string la, sa_, lb, sb_;
-        for (uint64_t m = lo; m < hi; ++m) {
-            const uint64_t va = hm[2 * m], vb = hm[2 * m + 1];
-            const int64_t side_a = (int64_t)(va >> kRankBits), side_b = (int64_t)(vb >> kRankBits);
-            host_expand(lv, sides[2 * p0 + side_a], va & kRankMask, xa);
-            host_expand(lv, sides[2 * p0 + side_b], vb & kRankMask, xb);
-            candidate_line(lv, xa, true, la, sa_);
-            candidate_line(lv, xb, false, lb, sb_);
-            pair_of[m] = side_a >> 1;
-            if (signature_token(la) != signature_token(lb)) continue;
-            keep[m] = 1;
-            items[m] = Match{la, lb, sa_ + " " + sb_ + "\n", xa, xb};
-        }
-    };
-    const unsigned nt = (unsigned)std::min<uint64_t>(16, (nm + 63) / 64);
-    if (nt <= 1) {
-        work(0, nm);
-    } else {
-        std::vector<std::thread> th;
-        for (unsigned t = 0; t < nt; ++t) th.emplace_back(work, nm * t / nt, nm * (t + 1) / nt);
-        for (auto& t : th) t.join();
+    const int N = lv.Lnew, bound = 2 * lv.order - lv.paf;
+    const int digits = (int)std::to_string(std::abs((long long)bound)).size() + 1;
+    const int W = 1 + ((N - 1) * digits + 2 + 2 * N * 5 + 7) / 8;
+    const uint64_t chunk = std::min<uint64_t>(nm, (uint64_t(1) << 31) / (uint64_t)(10 * N + 2));  // lines at once
+    DevBuf &dseqs = c->ux[36], &dkey = c->ux[37], &dord = c->ux[38], &dtmp = c->ux[39], &dbytes = c->ux[40],
+           &doff = c->ux[41], &dtext = c->ux[42], &dkept = c->ux[43];
+    if (nm > INT32_MAX || !dseqs.ensure(nm * 2 * N) || !dkey.ensure(nm * W * 4) || !dord.ensure(nm * 4) ||
+        !dtmp.ensure(std::max(gp::radix_sort_tmp_bytes((int64_t)nm, W), gp::scan_tmp_bytes((int64_t)chunk + 1))) ||
+        !dbytes.ensure((chunk + 1) * 4) || !doff.ensure((chunk + 1) * 4) || !dkept.ensure(4)) {
+        *overflowed = true;
+        return GP_ERR_OVERFLOW;
     }
-    for (uint64_t m = 0; m < nm; ++m)
-        if (keep[m]) out[pair_of[m]].push_back(std::move(items[m]));
-    for (auto& v : out)
-        std::sort(v.begin(), v.end(),
-                  [](const Match& p, const Match& q) { return p.la != q.la ? p.la < q.la : p.lb < q.lb; });
+    LineArgs la{};
+    la.lv = d;
+    la.rows = c->ux[24].as<uint8_t>() + (size_t)(2 * p0) * L;
+    la.matches = dm.as<uint64_t>();
+    la.n = nm;
+    la.tw = c->ux[27].as<double2>();
+    la.bound = bound;
+    la.W = W;
+    la.seqs = dseqs.as<int8_t>();
+    la.keys = dkey.as<uint32_t>();
+    la.kept = dkept.as<unsigned>();
+    uint32_t* ord = dord.as<uint32_t>();
+    GP_CUDA_TRY(c, cudaMemsetAsync(dkept.p, 0, 4, s));
+    ux_lines_kernel<<<(unsigned)std::min<uint64_t>((nm + kLineWarps - 1) / kLineWarps, (uint64_t)c->num_sms * 8),
+                      kLineWarps * 32, 0, s>>>(la);
+    GP_CUDA_TRY(c, cudaGetLastError());
+    GP_CUDA_TRY(c, gp::iota_u32(ord, (int64_t)nm, s));
+    GP_CUDA_TRY(c, gp::radix_sort_keys(la.keys, W, W, ord, (int64_t)nm, dtmp.p, s, 8));
+    unsigned kept = 0;
+    for (uint64_t k0 = 0; k0 < nm; k0 += chunk) {
+        const uint64_t n = std::min(chunk, nm - k0);
+        ux_line_bytes_kernel<<<grid_for(n + 1, (unsigned)c->num_sms * 8), 256, 0, s>>>(la.seqs, N, ord, k0, n, la.kept,
+                                                                                      dbytes.as<uint32_t>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        GP_CUDA_TRY(c, gp::exclusive_scan_u32(dbytes.as<uint32_t>(), doff.as<uint32_t>(), (int64_t)n + 1,
+                                              dtmp.as<uint32_t>(), s));
+        uint32_t bytes = 0;
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&bytes, doff.as<uint32_t>() + n, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&kept, la.kept, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+        if (kept <= k0) break;
+        if (!dtext.ensure(bytes)) {
+            *overflowed = true;
+            return GP_ERR_OVERFLOW;
+        }
+        const uint64_t lines = std::min<uint64_t>(n, kept - k0);
+        ux_text_kernel<<<grid_for(lines * 32, (unsigned)c->num_sms * 8), 256, 0, s>>>(
+            la.seqs, N, ord + k0, lines, doff.as<uint32_t>(), dtext.as<char>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        const size_t at = text.size();
+        text.resize(at + bytes);
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&text[at], dtext.p, bytes, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    }
+    if (want_rows && kept) {
+        std::vector<int8_t> rows2(nm * 2 * N);
+        std::vector<uint32_t> order(kept);
+        GP_CUDA_TRY(c, cudaMemcpyAsync(rows2.data(), dseqs.p, rows2.size(), cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(order.data(), ord, (size_t)kept * 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+        out_rows.resize((size_t)kept * 2 * N);
+        for (unsigned k = 0; k < kept; ++k)
+            memcpy(&out_rows[(size_t)k * 2 * N], &rows2[(size_t)order[k] * 2 * N], 2 * N);
+    }
     return GP_OK;
 }
 
@@ -1567,7 +1709,7 @@ int run_level(gp_ctx* c, const Level& lv, const std::vector<uint8_t>& seqs, FILE
     LevelDev ld{};
     rc = upload_level(c, lv, ld, s);
     if (rc) return rc;
-    Batcher bt{c, lv, ld, sides, seqs, s, scan_kernel_for(lv.np), 0, 0, {}};
+    Batcher bt{c, lv, ld, sides, seqs, s, scan_kernel_for(lv.np), 0, 0, next != nullptr, {}, {}};
     {
         // shared memory of the scan: the largest suffix table and term table
         // any side of this call needs (a few tens of KB: several CTAs per SM)
@@ -1602,7 +1744,6 @@ int run_level(gp_ctx* c, const Level& lv, const std::vector<uint8_t>& seqs, FILE
         p = q;
     }
     std::reverse(todo.begin(), todo.end());
-    std::string buf;
     while (!todo.empty()) {
         const auto [p0, p1] = todo.back();
         todo.pop_back();
@@ -1616,16 +1757,8 @@ int run_level(gp_ctx* c, const Level& lv, const std::vector<uint8_t>& seqs, FILE
         }
         if (rc == GP_ERR_OVERFLOW && over) return c->fail(GP_ERR_OVERFLOW, "uncompress: one pair overflows the device lists");
         if (rc) return rc;
-        buf.clear();
-        for (auto& v : bt.out)
-            for (auto& m : v) {
-                buf += m.line;
-                if (next) {
-                    for (int x : m.xa) next->push_back((int8_t)x);
-                    for (int x : m.xb) next->push_back((int8_t)x);
-                }
-            }
-        if (!buf.empty() && fwrite(buf.data(), 1, buf.size(), out) != buf.size())
+        if (next) next->insert(next->end(), bt.out_rows.begin(), bt.out_rows.end());
+        if (!bt.text.empty() && fwrite(bt.text.data(), 1, bt.text.size(), out) != bt.text.size())
             return c->fail(GP_ERR_IO, "uncompress: write failed");
     }
     return GP_OK;
