@@ -237,19 +237,63 @@ __device__ __forceinline__ int compare_halves(const Half& H1, int s1, const Half
 // shift, and the shifts that fix a and b, and then compare the 4 phi(L) (x 8)
 // combinations of two halves.  (Every combination on its own takes each
 // half's shifts four times; a CTA of 128 threads per pair left most of them
-// idle in its second round at length 57: 7.50 ms for 30,000 pairs, now 1.88.)
+// idle in its second round at length 57: 7.50 ms for 30,000 pairs, 1.88 by
+// halves.)
+// Entries +-1 of up to 64 per half are words of one bit each, first entry
+// highest: x[m i + s] over all s are the rotations of the decimated word, a
+// sign pattern flips fixed bits, and the order of images is the order of the
+// numbers (the call goes from 4.24 to 2.72 ms).
 constexpr int kCanonWarps = 4;
 struct HalfShift {
     uint8_t s, fix_a, fix_b;
 };
 
+// A warp's shared memory: the pair, its halves' least words (lengths up to 64),
+// their least shifts.
+struct CanonLayout {
+    size_t words, tab, per_warp;
+};
+__host__ __device__ __forceinline__ CanonLayout canon_layout(int L, int nhalf) {
+    CanonLayout s;
+    s.words = (2 * (size_t)L + 7) & ~size_t(7);
+    s.tab = s.words + (L <= 64 ? sizeof(uint64_t) * nhalf : 0);
+    s.per_warp = (s.tab + sizeof(HalfShift) * nhalf + 7) & ~size_t(7);
+    return s;
+}
+
+// The least rotation of the word of x's decimation by m, bits flipped by sign,
+// and how many rotations equal wa and wb.
+__device__ __forceinline__ uint64_t least_rotation(uint64_t x, int L, int m, uint64_t sign, uint64_t wa, uint64_t wb,
+                                                   int& fix_a, int& fix_b) {
+    uint64_t y = 0;
+    for (int i = 0, j = 0; i < L; ++i) {
+        y = (y << 1) | ((x >> (L - 1 - j)) & 1ull);
+        j += m;
+        j -= j >= L ? L : 0;
+    }
+    const uint64_t all = ~0ull >> (64 - L);
+    uint64_t best = ~0ull;
+    fix_a = fix_b = 0;
+    for (int t = 0; t < L; ++t) {
+        const uint64_t v = y ^ sign;
+        best = v < best ? v : best;
+        fix_a += v == wa;
+        fix_b += v == wb;
+        y = ((y << 1) & all) | (y >> (L - 1));
+    }
+    return best;
+}
+
 __global__ void __launch_bounds__(32 * kCanonWarps) canon_kernel(CanonArgs a) {
-    extern __shared__ uint8_t sh[];
+    extern __shared__ __align__(8) uint8_t sh[];
     const int L = a.L, W = 2 * L, npat = a.alt ? 4 : 1, nhalf = 2 * npat * a.nu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // per warp: the pair, then the halves' least shifts
-    int8_t* x = reinterpret_cast<int8_t*>(sh) + (size_t)warp * (W + sizeof(HalfShift) * nhalf);
-    HalfShift* tab = reinterpret_cast<HalfShift*>(x + W);
+    const CanonLayout lay = canon_layout(L, nhalf);
+    uint8_t* mine = sh + (size_t)warp * lay.per_warp;
+    int8_t* x = reinterpret_cast<int8_t*>(mine);
+    uint64_t* least = reinterpret_cast<uint64_t*>(mine + lay.words);
+    HalfShift* tab = reinterpret_cast<HalfShift*>(mine + lay.tab);
     const int ncombo = 4 * a.nu * (a.alt ? 8 : 1);
     // half t: source half t & 1, sign pattern, unit index
     auto half_of = [&](int src, int pat, int ui) { return (ui * npat + pat) * 2 + src; };
@@ -273,9 +317,31 @@ __global__ void __launch_bounds__(32 * kCanonWarps) canon_kernel(CanonArgs a) {
         __syncwarp();
         for (int o = lane; o < W; o += 32) x[o] = a.pairs[pr * W + o];
         __syncwarp();
+        bool bits = L <= 64;  // the pair's entries are +-1
+        uint64_t word[2] = {0, 0};
+        if (bits) {
+            bool unit = true;
+            for (int h = 0; h < 2; ++h) {
+                const int v0 = lane < L ? x[h * L + lane] : 1, v1 = lane + 32 < L ? x[h * L + lane + 32] : 1;
+                unit = unit && (v0 == 1 || v0 == -1) && (v1 == 1 || v1 == -1);
+                const uint64_t w = __ballot_sync(0xFFFFFFFFu, v0 > 0) |
+                                   (uint64_t)__ballot_sync(0xFFFFFFFFu, v1 > 0) << 32;
+                word[h] = __brevll(w) >> (64 - L);
+            }
+            bits = __all_sync(0xFFFFFFFFu, unit);
+        }
         for (int t = lane; t < nhalf; t += 32) {
-            int s, fa, fb;
-            least_shift(half(t), s, fa, fb);
+            int s = 0, fa, fb;
+            if (bits) {
+                const int pat = (t >> 1) % npat;
+                // negated entries: the odd ones (pattern bit 0), all the others (bit 1)
+                uint64_t sign = 0;
+                if (pat & 1) sign = (0x5555555555555555ull << (L & 1)) & (~0ull >> (64 - L));
+                if (pat & 2) sign ^= ~0ull >> (64 - L);
+                least[t] = least_rotation(word[t & 1], L, a.units[(t >> 1) / npat], sign, word[0], word[1], fa, fb);
+            } else {
+                least_shift(half(t), s, fa, fb);
+            }
             tab[t] = HalfShift{(uint8_t)s, (uint8_t)fa, (uint8_t)fb};
         }
         __syncwarp();
@@ -283,6 +349,10 @@ __global__ void __launch_bounds__(32 * kCanonWarps) canon_kernel(CanonArgs a) {
             int a1, b1, a2, b2;
             halves(c1, a1, b1);
             halves(c2, a2, b2);
+            if (bits) {
+                if (least[a1] != least[a2]) return least[a1] < least[a2] ? -1 : 1;
+                return least[b1] == least[b2] ? 0 : least[b1] < least[b2] ? -1 : 1;
+            }
             const int d = a1 == a2 ? 0 : compare_halves(half(a1), tab[a1].s, half(a2), tab[a2].s);
             return d || b1 == b2 ? d : compare_halves(half(b1), tab[b1].s, half(b2), tab[b2].s);
         };
@@ -306,7 +376,10 @@ __global__ void __launch_bounds__(32 * kCanonWarps) canon_kernel(CanonArgs a) {
         for (int o = lane; o < W; o += 32) {
             const Half& H = o < L ? A : B;
             const int i = o < L ? o : o - L;
-            a.canon[pr * W + o] = (int8_t)(sign_of(H.pat, i) * x[H.h + (H.m * i + tab[o < L ? ta : tb].s) % L]);
+            if (bits)
+                a.canon[pr * W + o] = (least[o < L ? ta : tb] >> (L - 1 - i)) & 1ull ? 1 : -1;
+            else
+                a.canon[pr * W + o] = (int8_t)(sign_of(H.pat, i) * x[H.h + (H.m * i + tab[o < L ? ta : tb].s) % L]);
         }
         if (lane == 0) a.fixers[pr] = fix;
     }
@@ -792,7 +865,7 @@ int canonical_classes(PairSet& ps, int L, int compress, std::vector<unsigned lon
     ca.alt = !(compress > 1 || L % 2 == 1) ? 1 : 0;  // filter.cpp:83-87
     ca.canon = dc.as<int8_t>();
     ca.fixers = df.as<uint32_t>();
-    const size_t smem = (size_t)kCanonWarps * (W + sizeof(HalfShift) * 2 * (ca.alt ? 4 : 1) * ca.nu);
+    const size_t smem = kCanonWarps * canon_layout(L, 2 * (ca.alt ? 4 : 1) * ca.nu).per_warp;
     const int64_t grid = std::min<int64_t>((np + kCanonWarps - 1) / kCanonWarps, (int64_t)c->num_sms * 16);
     canon_kernel<<<(unsigned)grid, 32 * kCanonWarps, smem, s>>>(ca);
     GP_CUDA_TRY(c, cudaGetLastError());
