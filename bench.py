@@ -365,7 +365,7 @@ def run_gpu(args):
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "fp16 x fp16 -> fp32 (tcgen05) + f64 recheck; int8 input",
             "data": "synthetic (seeded, generated on device)", "config": WORKLOAD,
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": args.steps,  # one psd_tc_kernel per step, its FP64 recheck included
             "verdicts_exact_vs_fp64_kernel": verdicts_equal and e2e_equal,
             "unsure_per_step": int(st.n_unsure), "pass_per_step": int(st.n_pass),
             "fp64_comparator": {"value": fp64_value, "unit": UNIT, "ms_per_step": fms / f_steps,
