@@ -314,5 +314,5 @@ class Context:
 
 
 def unpack_mask(mask, n):
-    bits = np.unpackbits(mask.view(np.uint8), bitorder="little")
-    return bits[:n].astype(bool)
+    # the unpacked bytes are 0 and 1: bools without a second pass over them
+    return np.unpackbits(mask.view(np.uint8), count=n, bitorder="little").view(np.bool_)
