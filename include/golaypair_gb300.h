@@ -250,7 +250,7 @@ typedef struct gp_gen_job {
 typedef struct gp_batch_config {
     int enum_variant;        /* enumerator kernel: 0 = 4 CTAs per SM (64 registers), 1 = 6 (40),
                                 2 = 5 (48) */
-    int windows_per_thread;  /* rank windows per enumerator thread (0: 1) */
+    int windows_per_thread;  /* rank windows per enumerator thread and job (0: 1) */
     int64_t cand_cap;        /* candidates per job per pipeline iteration (0: 2^22) */
     int tc_ctas_per_sm;      /* tensor-core filter CTAs per SM (0: as many as fit) */
     int no_graph;            /* 1: launch each iteration's kernels directly instead of replaying a CUDA graph */
