@@ -398,7 +398,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
     }
     DevBuf& arena = c->scratch[7];
     HostPinned& hbuf = c->hscratch[3];
-    if (!arena.ensure(off) || !hbuf.ensure(kCounterWords * 8))
+    if (!arena.ensure(off) || !hbuf.ensure((kCounterWords + 1) * 8))
         return c->fail(GP_ERR_NOMEM, "batch generation: cannot allocate %zu bytes of device memory", off);
     uint8_t* A = arena.as<uint8_t>();
     unsigned long long* ctr = reinterpret_cast<unsigned long long*>(A + off_ctr);
@@ -536,6 +536,14 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
         GP_CUDA_TRY(c, gp::launch_finalize_multi(fm, cap, c->num_sms, s));
         return GP_OK;
     };
+    // the counters, and the kernels' status word behind them (a read of its own
+    // after every iteration would be one more wait)
+    int* hstatus = reinterpret_cast<int*>(hctr + kCounterWords);
+    auto copy_counters = [&]() -> int {
+        GP_CUDA_TRY(c, cudaMemcpyAsync(hctr, ctr, kCounterWords * 8, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(hstatus, c->status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        return GP_OK;
+    };
     auto enqueue_iteration = [&]() -> int {
         GP_CUDA_TRY(c, cudaMemsetAsync(ctr, 0, kIterWords * 8, s));
         if (ea.nwin > 0 && ea_wide.nwin > 0) {
@@ -556,8 +564,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
         if (multi) {
             const int rc = enqueue_multi();
             if (rc) return rc;
-            GP_CUDA_TRY(c, cudaMemcpyAsync(hctr, ctr, kCounterWords * 8, cudaMemcpyDeviceToHost, s));
-            return GP_OK;
+            return copy_counters();
         }
         // branches per job
         GP_CUDA_TRY(c, cudaEventRecord(c->ev_fork, s));
@@ -579,8 +586,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
             GP_CUDA_TRY(c, cudaEventRecord(c->ev_join[ji], sj));
             GP_CUDA_TRY(c, cudaStreamWaitEvent(s, c->ev_join[ji], 0));
         }
-        GP_CUDA_TRY(c, cudaMemcpyAsync(hctr, ctr, kCounterWords * 8, cudaMemcpyDeviceToHost, s));
-        return GP_OK;
+        return copy_counters();
     };
     t_setup = since(tb) - t_win;
     // ---- capture it once
@@ -619,7 +625,7 @@ int run_batch(gp_ctx* c, std::vector<JobRun>& jobs, const BatchCfg& cfg, int* it
             if (rc) return rc;
         }
         GP_CUDA_TRY(c, cudaStreamSynchronize(s));
-        int rc = c->check_status("batch generation");
+        int rc = *hstatus ? c->check_status("batch generation") : GP_OK;
         if (rc) return rc;
         ++iters;
         int64_t added = 0;
