@@ -87,6 +87,7 @@ struct LevelDev {
     int target;                           // paf * c'
     const int* cnt;                       // [nrows] choices per row
     const int8_t* vals;                   // [nrows][dmax][r] values of each choice
+    const uint64_t* words;                // one_bit: [nrows][dmax] the choice's 1s at bits 0, L, 2 L, ..
     const float4* ctab;                   // [L][nrows][dmax][np]: (re 2p, re 2p+1, im 2p, im 2p+1)
     const double2* ctab64;                // [L][nrows][dmax][2 np]
     const uint8_t* side_rows;             // [sides][L] row of each position
@@ -515,21 +516,45 @@ __device__ __forceinline__ void expand_values(const LevelDev& lv, uint64_t val, 
     }
 }
 
+// one_bit: the expansion's 1s, entry j at bit j.
+__device__ __forceinline__ uint64_t expansion_word(const LevelDev& lv, uint64_t val) {
+    const uint8_t* rows = lv.side_rows + (size_t)(val >> kRankBits) * lv.L;
+    uint64_t rank = val & kRankMask, w = 0;
+    for (int i = lv.L - 1; i >= 0; --i) {
+        const uint32_t row = rows[i], c = (uint32_t)lv.cnt[row];
+        uint32_t d = 0;
+        if (c > 1) {
+            if (rank >> 32) {
+                d = (uint32_t)(rank % c);
+                rank /= c;
+            } else {
+                const uint32_t q = (uint32_t)rank / c;
+                d = (uint32_t)rank - q * c;
+                rank = q;
+            }
+        }
+        w |= lv.words[row * (uint32_t)lv.dmax + d] << i;
+    }
+    return w;
+}
+
+// Periodic autocorrelation of a one_bit expansion at shift s.
+__device__ __forceinline__ int word_paf(uint64_t w, int N, int s) {
+    const uint64_t mask = N == 64 ? ~0ull : ((1ull << N) - 1ull);
+    const uint64_t rot = ((w >> s) | (w << (N - s))) & mask;  // bit j = bit j + s of w
+    return N - 2 * __popcll(w ^ rot);
+}
+
 // PAF(s), s = 1 .. H, of an expansion (src/utils/golay.cpp:27-33).
 __device__ __forceinline__ void expansion_paf(const LevelDev& lv, uint64_t val, int* paf) {
-    int8_t x[kMaxLnew];
-    expand_values(lv, val, x);
     const int N = lv.Lnew;
     if (lv.one_bit) {
-        uint64_t w = 0;
-        for (int j = 0; j < N; ++j) w |= (uint64_t)(x[j] > 0) << j;
-        const uint64_t mask = N == 64 ? ~0ull : ((1ull << N) - 1ull);
-        for (int s = 1; s <= lv.H; ++s) {
-            const uint64_t rot = ((w >> s) | (w << (N - s))) & mask;  // bit j = bit j + s of w
-            paf[s - 1] = N - 2 * __popcll(w ^ rot);
-        }
+        const uint64_t w = expansion_word(lv, val);
+        for (int s = 1; s <= lv.H; ++s) paf[s - 1] = word_paf(w, N, s);
         return;
     }
+    int8_t x[kMaxLnew];
+    expand_values(lv, val, x);
     for (int s = 1; s <= lv.H; ++s) {
         int acc = 0, j2 = s;
         for (int j = 0; j < N; ++j) {
@@ -552,10 +577,11 @@ __device__ __forceinline__ uint64_t mix64(uint64_t h) {
 // join key of a survivor's PAF vector in its role: as the a-side of a pair
 // it hashes paf*c' - PAF_a(s), as the b-side PAF_b(s); complementary pairs
 // have equal keys
-__device__ __forceinline__ uint64_t join_key(const LevelDev& lv, const int* paf, bool is_a) {
+template <class Paf>
+__device__ __forceinline__ uint64_t join_key(const LevelDev& lv, Paf paf, bool is_a) {
     uint64_t h = 0x243f6a8885a308d3ull;
     for (int s = 0; s < lv.H; ++s) {
-        const int v = is_a ? lv.target - paf[s] : paf[s];
+        const int p = paf(s), v = is_a ? lv.target - p : p;
         h = (h ^ (uint64_t)(uint32_t)v) * 0x100000001b3ull;
     }
     return mix64(h);
@@ -619,8 +645,14 @@ __global__ void ux_key_kernel(KeyArgs a) {
             a.bucket[i] = 0xFFFFFFFFu;
             continue;
         }
+        // +-1 expansions as a word, their vector made as it is hashed (with both in
+        // local memory 4,000 order-57 pairs took 2.7 ms more of 139)
         int paf[kMaxLnew / 2];
-        expansion_paf(a.lv, v, paf);
+        uint64_t word = 0;
+        if (a.lv.one_bit)
+            word = expansion_word(a.lv, v);
+        else
+            expansion_paf(a.lv, v, paf);
         uint64_t e = i;
         for (uint32_t j = j0; j < j1; ++j) {
             const uint32_t code = a.uses[j], pair = code >> 1, role = code & 1u;
@@ -630,7 +662,9 @@ __global__ void ux_key_kernel(KeyArgs a) {
                 flag_overflow(a.status);
                 break;
             }
-            const uint64_t h = join_key(a.lv, paf, role == 0);
+            const uint64_t h = a.lv.one_bit
+                                   ? join_key(a.lv, [&](int s) { return word_paf(word, a.lv.Lnew, s + 1); }, role == 0)
+                                   : join_key(a.lv, [&](int s) { return paf[s]; }, role == 0);
             const uint32_t b = a.pair_base[pair] + (lg ? (uint32_t)(h >> (64 - lg)) : 0u);
             a.keys[e] = h;
             a.bucket[e] = b;
@@ -1188,15 +1222,21 @@ __global__ void __launch_bounds__(256) ux_tables_kernel(TablesArgs a) {
     }
 }
 
-// A level's tables on the device (context scratch ux[0..3] and ux[34..36]).
+// A level's tables on the device (context scratch ux[0..3], ux[34], ux[35] and ux[44]).
 int upload_level(gp_ctx* c, const Level& lv, LevelDev& d, cudaStream_t s) {
     const int np = lv.np, NB = 2 * np;
     std::vector<int> cnt(lv.nrows);
     std::vector<int8_t> vals((size_t)lv.nrows * lv.dmax * lv.r, 0);
+    const bool one_bit = lv.cn == 1 && lv.Lnew <= 64;
+    std::vector<uint64_t> words(one_bit ? (size_t)lv.nrows * lv.dmax : 0, 0);
     for (int row = 0; row < lv.nrows; ++row) {
         cnt[row] = (int)lv.rowparts[row].size();
         for (int d = 0; d < cnt[row]; ++d)
-            for (int q = 0; q < lv.r; ++q) vals[((size_t)row * lv.dmax + d) * lv.r + q] = (int8_t)lv.rowparts[row][d][q];
+            for (int q = 0; q < lv.r; ++q) {
+                const int v = lv.rowparts[row][d][q];
+                vals[((size_t)row * lv.dmax + d) * lv.r + q] = (int8_t)v;
+                if (one_bit && v > 0) words[(size_t)row * lv.dmax + d] |= uint64_t(1) << (lv.L * q);
+            }
     }
     std::vector<double2> tw(2 * (size_t)lv.Lnew);  // cosines, then sines, as (hi, lo)
     for (int m = 0; m < lv.Lnew; ++m) {
@@ -1209,12 +1249,14 @@ int upload_level(gp_ctx* c, const Level& lv, LevelDev& d, cudaStream_t s) {
     }
     const size_t terms = (size_t)lv.L * lv.nrows * lv.dmax;
     DevBuf &dcnt = c->ux[0], &dvals = c->ux[1], &dct = c->ux[2], &dct64 = c->ux[3], &dbins = c->ux[34],
-           &dtw = c->ux[35];
-    if (!dcnt.ensure(cnt.size() * 4) || !dvals.ensure(vals.size() + 16) || !dct.ensure(terms * np * 16) ||
+           &dtw = c->ux[35], &dwords = c->ux[44];
+    if (!dwords.ensure(words.size() * 8 + 8) || !dcnt.ensure(cnt.size() * 4) || !dvals.ensure(vals.size() + 16) || !dct.ensure(terms * np * 16) ||
         !dct64.ensure(terms * NB * 16) || !dbins.ensure((size_t)lv.nb * 4 + 4) || !dtw.ensure(tw.size() * 16))
         return c->fail(GP_ERR_NOMEM, "uncompress: level tables");
     GP_CUDA_TRY(c, cudaMemcpyAsync(dcnt.p, cnt.data(), cnt.size() * 4, cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(dvals.p, vals.data(), vals.size(), cudaMemcpyHostToDevice, s));
+    if (one_bit)
+        GP_CUDA_TRY(c, cudaMemcpyAsync(dwords.p, words.data(), words.size() * 8, cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(dbins.p, lv.bins.data(), lv.bins.size() * 4, cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(dtw.p, tw.data(), tw.size() * 16, cudaMemcpyHostToDevice, s));
     TablesArgs ta{lv.L, lv.r, lv.Lnew, lv.nrows, lv.dmax, lv.nb, np, dcnt.as<int>(), dvals.as<int8_t>(),
@@ -1232,7 +1274,8 @@ int upload_level(gp_ctx* c, const Level& lv, LevelDev& d, cudaStream_t s) {
     d.dmax = lv.dmax;
     d.np = np;
     d.nb = lv.nb;
-    d.one_bit = lv.cn == 1 && lv.Lnew <= 64;
+    d.one_bit = one_bit;
+    d.words = dwords.as<uint64_t>();
     d.target = lv.paf * lv.cn;
     d.cnt = dcnt.as<int>();
     d.vals = dvals.as<int8_t>();
