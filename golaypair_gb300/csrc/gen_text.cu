@@ -9,6 +9,9 @@
 // What bounds it: the copy and the files.  A generation call over an order-57
 // window of 2^32 words with 40 MB of lines: 17.5 ms, 46 with the records
 // copied, sorted and formatted by host threads.
+#include <algorithm>
+#include <new>
+
 #include "ctx.h"
 #include "gen_text.h"
 #include "pair_text.cuh"
@@ -120,7 +123,8 @@ int records_to_text(gp_ctx* c, const GenRecords& r, GenText& out, cudaStream_t s
     record_lines_kernel<<<grid, 256, 0, s>>>(r, idx, off, b[kGtText].as<char>());
     GP_CUDA_TRY(c, cudaGetLastError());
     uint32_t bytes_a = (uint32_t)bytes;
-    std::shared_ptr<char[]> text(new char[bytes]);
+    std::shared_ptr<char[]> text(new (std::nothrow) char[bytes]);
+    if (!text) return GP_OK;
     if ((int64_t)n_a < n) GP_CUDA_TRY(c, cudaMemcpyAsync(&bytes_a, off + n_a, 4, cudaMemcpyDeviceToHost, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(text.get(), b[kGtText].p, bytes, cudaMemcpyDeviceToHost, s));
     GP_CUDA_TRY(c, cudaStreamSynchronize(s));
