@@ -219,21 +219,20 @@ __device__ __forceinline__ bool job_full(const EnumJob& j) {
 //
 // What bounds it: issue (67 %) once every lane has a dense window, the last
 // windows' serial steps at the end.  An order-57 window of 2^32 words (2.3 G
-// necklaces, 208 M candidates): 2.6 ms of kernel time, 9.4 when each lane took,
+// necklaces, 208 M candidates): 2.4 ms of kernel time, 9.4 when each lane took,
 // loaded and checked its own windows and every 32 candidates took an atomic,
-// 15.1 with blocks of two digits taken a row at a time; five orders: 18, 48 and
-// 87 ms (27 with as many windows for all five as for one).  Blocks per SM
-// 4, 5, 6: 2.56, 2.53, 2.70 and 27.0, 27.2, 30.4 ms.
+// 15.1 with blocks of two digits taken a row at a time; five orders: 16, 48 and
+// 87 ms (27 with as many windows for all five as for one).  With that and
+// queues of 192, blocks per SM 4, 5, 6: 2.56, 2.53, 2.70 and 27.0, 27.2, 30.4 ms.
 //
 // NARROW: every job's words fit 63 bits, so a word and its window end are
 // 64-bit values (the high halves are zero and drop out of the registers).
-constexpr int kQueue = kEnumQueue;  // per warp
-constexpr int kFlushAt = kEnumQueue - 32;
 constexpr int kCapCheck = 4;
 
 template <bool NARROW>
 struct EnumShared {
     using Word = typename std::conditional<NARROW, uint64_t, W128>::type;
+    static constexpr int kQueue = NARROW ? kEnumQueue : kEnumQueueWide;
     EnumJob jobs[kMaxEnumJobs];
     JobView views[kMaxEnumJobs];
     unsigned long long visited[kMaxEnumJobs];  // necklaces, by job
@@ -246,6 +245,7 @@ struct EnumShared {
 template <int MINB, bool NARROW>
 __global__ void __launch_bounds__(256, MINB) enumerate_kernel(EnumArgs a) {
     __shared__ EnumShared<NARROW> sh;
+    constexpr int kQueue = EnumShared<NARROW>::kQueue, kFlushAt = kQueue - 32;
     if (threadIdx.x < a.njobs) {
         sh.jobs[threadIdx.x] = a.jobs[threadIdx.x];
         sh.views[threadIdx.x] = job_view(sh.jobs[threadIdx.x]);
