@@ -1031,11 +1031,12 @@ int gp_sort(gp_ctx* c, const char** in_paths, int n_in, const char* out_path) {
 // the next line's), so the merge on the first token is an equality join: each
 // a line with the b lines of its token, in file order.  *done = false where
 // the host's parser or merge decides: other characters, lines of blanks or
-// with too few integers, unsorted tokens, more text or pairs than 32 bits.
+// with too few integers, unsorted tokens, more text or pairs than 32 bits,
+// sequences without entries (an order of 0).
 static int match_files(gp_ctx* c, int L, int target, const FileText& fa, const FileText& fb, FILE* f, int64_t* n_pairs,
                        bool* done) {
     *done = false;
-    if (fa.n + 2 > kMaxDeviceText || fb.n + 2 > kMaxDeviceText) return GP_OK;
+    if (L < 1 || fa.n + 2 > kMaxDeviceText || fb.n + 2 > kMaxDeviceText) return GP_OK;
     cudaStream_t s = c->s_comp;
     const FileText* file[2] = {&fa, &fb};
     DevBuf* text[2] = {&c->st[kTbText], &c->st[kTbTextB]};
