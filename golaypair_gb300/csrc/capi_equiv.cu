@@ -761,7 +761,7 @@ int sort_rows(PairSet& ps, const int8_t* rows, int64_t n, uint32_t* idx, uint32_
 // `text` holds n bytes and a terminating zero.
 int load_pairs(PairSet& ps, const char* text, size_t n, cudaStream_t s) {
     gp_ctx* c = ps.c;
-    if (n == 0) return GP_OK;
+    if (n == 0 || ps.W < 1) return GP_OK;  // no values, or none to a pair
     const bool huge = n >> 32;  // more text than the device's 32-bit offsets reach
     const int64_t blocks = huge ? 1 : (int64_t)((n + kParseBlock - 1) / kParseBlock);
     DevBuf &dt = c->eq[kEqText], &dcnt = c->eq[kEqCount], &doff = c->eq[kEqOffs], &dscan = c->eq[kEqScan],

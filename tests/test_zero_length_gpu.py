@@ -22,3 +22,14 @@ def test_match_of_sequences_without_entries(tmp_path, lines):
                                str(tmp_path / "out").encode(), 0, ctypes.byref(n))
     assert rc == 0 and n.value == lines
     assert (tmp_path / "out").read_text() == " \n" * lines
+
+
+@pytest.mark.parametrize("order", [0, -4])
+@pytest.mark.parametrize("values", ["", "1 -1 1 -1 \n", "1 1  -1 1 \n" * 300])
+def test_equivalence_of_pairs_without_entries(tmp_path, order, values):
+    (tmp_path / "in").write_text(values)
+    (tmp_path / "out").write_text("an older file")
+    with gp.Context(0) as ctx:
+        rc = ctx._lib.gp_equiv_filter(ctx.handle, order, 1, str(tmp_path / "in").encode(), str(tmp_path / "out").encode())
+    assert rc == 0
+    assert (tmp_path / "out").read_bytes() == b""  # no pair to write
