@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -329,7 +330,8 @@ __global__ void __launch_bounds__(256) match_lines_kernel(const int8_t* a, const
         gp::put_pair_line(a + (int64_t)ia[keep[k]] * L, b + (int64_t)ib[keep[k]] * L, L, text + at[k]);
 }
 
-// A file's bytes, unset until read: pieces read by host threads.
+// A file's bytes, unset until read: pieces read by host threads.  A directory
+// is an error, not a file of no bytes.
 struct FileText {
     std::unique_ptr<char[]> p;
     size_t n = 0;
@@ -337,8 +339,14 @@ struct FileText {
 bool read_file(const char* path, FileText& t) {
     const int fd = open(path, O_RDONLY);
     if (fd < 0) return false;
+    struct Closer {
+        int fd;
+        ~Closer() { close(fd); }
+    } closer{fd};
     struct stat sb;
-    const size_t size = fstat(fd, &sb) == 0 && S_ISREG(sb.st_mode) && sb.st_size > 0 ? (size_t)sb.st_size : 0;
+    const bool known = fstat(fd, &sb) == 0;
+    if (known && S_ISDIR(sb.st_mode)) throw std::runtime_error(std::string(path) + " is a directory");
+    const size_t size = known && S_ISREG(sb.st_mode) && sb.st_size > 0 ? (size_t)sb.st_size : 0;
     t.p.reset(new char[size + 1]);
     constexpr size_t kPiece = size_t(2) << 20;
     const size_t pieces = (size + kPiece - 1) / kPiece;
@@ -353,7 +361,6 @@ bool read_file(const char* path, FileText& t) {
         }
         got[k] = at - lo;
     });
-    close(fd);
     t.n = 0;
     for (size_t k = 0; k < pieces; ++k) {  // a file cut short meanwhile ends at its first short piece
         t.n += got[k];
