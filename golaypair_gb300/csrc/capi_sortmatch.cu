@@ -370,16 +370,40 @@ bool read_file(const char* path, FileText& t) {
     return true;
 }
 
-// Device text to a new file of the sort (an input may have the same name:
-// it has been read by now).
+// A stage's output file: closed on every way out, and whole only if every
+// write and the close say so (a large write goes past the stream's buffer, so
+// on a full disk the close alone can succeed).
+struct OutFile {
+    FILE* f;
+    bool whole = true;
+    OutFile(const char* path, const char* mode) : f(fopen(path, mode)) {}
+    ~OutFile() {
+        if (f) fclose(f);
+    }
+    OutFile(const OutFile&) = delete;
+    OutFile& operator=(const OutFile&) = delete;
+    void put(const char* p, size_t n) { whole = fwrite(p, 1, n, f) == n && whole; }
+    bool close() {
+        whole = fclose(f) == 0 && whole;
+        f = nullptr;
+        return whole;
+    }
+};
+
+// The sort's output (an input may have the same name: it has been read by now).
+int write_file(gp_ctx* c, const char* p, size_t n, const char* path) {
+    OutFile f(path, "w");
+    if (!f.f) return c->fail(GP_ERR_IO, "sort: cannot write %s", path);
+    f.put(p, n);
+    return f.close() ? GP_OK : c->fail(GP_ERR_IO, "sort: write failed: %s", path);
+}
+
+// The same from device text.
 int write_text(gp_ctx* c, const char* d_text, size_t n, const char* path, cudaStream_t s) {
     std::unique_ptr<char[]> h(new char[n + 1]);
     GP_CUDA_TRY(c, cudaMemcpyAsync(h.get(), d_text, n, cudaMemcpyDeviceToHost, s));
     GP_CUDA_TRY(c, cudaStreamSynchronize(s));
-    FILE* f = fopen(path, "w");
-    if (!f) return c->fail(GP_ERR_IO, "sort: cannot write %s", path);
-    fwrite(h.get(), 1, n, f);
-    return fclose(f) == 0 ? GP_OK : c->fail(GP_ERR_IO, "sort: write failed");
+    return write_file(c, h.get(), n, path);
 }
 
 // The context's sort and match buffers, one use each.
@@ -1019,10 +1043,7 @@ static int gp_sort_impl(gp_ctx* c, const char** in_paths, int n_in, const char* 
     std::string sorted;
     int rc = gp_sort_text(c, all, sorted);
     if (rc) return rc;
-    FILE* f = fopen(out_path, "w");
-    if (!f) return c->fail(GP_ERR_IO, "sort: cannot write %s", out_path);
-    fwrite(sorted.data(), 1, sorted.size(), f);
-    return fclose(f) == 0 ? GP_OK : c->fail(GP_ERR_IO, "sort: write failed");
+    return write_file(c, sorted.data(), sorted.size(), out_path);
 }
 
 // No C++ exception (an allocation failure on a huge input) crosses the C ABI.
@@ -1040,8 +1061,8 @@ int gp_sort(gp_ctx* c, const char** in_paths, int n_in, const char* out_path) {
 // the host's parser or merge decides: other characters, lines of blanks or
 // with too few integers, unsorted tokens, more text or pairs than 32 bits,
 // sequences without entries (an order of 0).
-static int match_files(gp_ctx* c, int L, int target, const FileText& fa, const FileText& fb, FILE* f, int64_t* n_pairs,
-                       bool* done) {
+static int match_files(gp_ctx* c, int L, int target, const FileText& fa, const FileText& fb, OutFile& f,
+                       int64_t* n_pairs, bool* done) {
     *done = false;
     if (L < 1 || fa.n + 2 > kMaxDeviceText || fb.n + 2 > kMaxDeviceText) return GP_OK;
     cudaStream_t s = c->s_comp;
@@ -1142,7 +1163,7 @@ static int match_files(gp_ctx* c, int L, int target, const FileText& fa, const F
         std::unique_ptr<char[]> out(new char[bytes + 1]);
         GP_CUDA_TRY(c, cudaMemcpyAsync(out.get(), dout.p, bytes, cudaMemcpyDeviceToHost, s));
         GP_CUDA_TRY(c, cudaStreamSynchronize(s));
-        fwrite(out.get(), 1, bytes, f);
+        f.put(out.get(), bytes);
     }
     if (n_pairs) *n_pairs = nk;
     return GP_OK;
@@ -1156,29 +1177,25 @@ static int gp_match_impl(gp_ctx* c, int order, int compress, int paf, const char
     cudaSetDevice(c->device);
     // the reference opens the pair writer (truncating unless appending)
     // before looking at the inputs (src/main.cpp:97-101)
-    FILE* f = fopen(out_path, append ? "a" : "w");
-    if (!f) return c->fail(GP_ERR_IO, "match: cannot open %s", out_path);
+    OutFile f(out_path, append ? "a" : "w");
+    if (!f.f) return c->fail(GP_ERR_IO, "match: cannot open %s", out_path);
     KeepSmall keep{c->st};
     FileText fa, fb;
     const bool okA = read_file(path_a, fa), okB = read_file(path_b, fb);
     if (n_pairs) *n_pairs = 0;
-    if (!okA || !okB || fa.n == 0 || fb.n == 0) {
-        fclose(f);
-        return GP_EMPTY_INPUT;
-    }
+    if (!okA || !okB || fa.n == 0 || fb.n == 0) return GP_EMPTY_INPUT;
     bool done = false;
     int rc = match_files(c, order / compress, paf * compress, fa, fb, f, n_pairs, &done);
-    if (done || rc) {
-        fclose(f);
-        return rc;
+    if (rc) return rc;
+    if (!done) {
+        std::string ta(fa.p.get(), fa.n), tb(fb.p.get(), fb.n), out;
+        fa.p.reset();
+        fb.p.reset();
+        rc = gp_match_texts(c, order / compress, compress, paf, ta, tb, out, n_pairs);
+        if (rc) return rc;
+        f.put(out.data(), out.size());
     }
-    std::string ta(fa.p.get(), fa.n), tb(fb.p.get(), fb.n), out;
-    fa.p.reset();
-    fb.p.reset();
-    rc = gp_match_texts(c, order / compress, compress, paf, ta, tb, out, n_pairs);
-    fwrite(out.data(), 1, out.size(), f);
-    fclose(f);
-    return rc;
+    return f.close() ? GP_OK : c->fail(GP_ERR_IO, "match: write failed: %s", out_path);
 }
 
 // No C++ exception (an allocation failure on a huge input) crosses the C ABI.
