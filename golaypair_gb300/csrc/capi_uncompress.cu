@@ -1833,7 +1833,14 @@ int uncompress_chain_impl(gp_ctx* c, int order, const int* compress, int ncomp, 
         if (!out) return c->fail(GP_ERR_IO, "uncompress: cannot open %s", out_pairs[lvl]);
         struct Closer {
             FILE* f;
-            ~Closer() { fclose(f); }
+            bool close() {
+                const bool ok = fclose(f) == 0;
+                f = nullptr;
+                return ok;
+            }
+            ~Closer() {
+                if (f) fclose(f);
+            }
         } closer{out};
         std::vector<int8_t> next;
         if (cc <= 1) {  // uncompression.cpp:42
@@ -1865,6 +1872,8 @@ int uncompress_chain_impl(gp_ctx* c, int order, const int* compress, int ncomp, 
         const bool more = lvl + 2 < ncomp;
         rc = run_level(c, lv, seqs, out, more ? &next : nullptr);
         if (rc) return rc;
+        // what the stream still holds is written here
+        if (!closer.close()) return c->fail(GP_ERR_IO, "uncompress: write failed: %s", out_pairs[lvl]);
         if (format_rc) return format_rc;  // the chain stops at a malformed input line
         carried.swap(next);
     }
