@@ -94,11 +94,12 @@ struct GroupPair {
     uint64_t first;  // index of this group's first pair in the flattened product
 };
 
-// one thread per candidate pair; flags[w] = 1 if the pair is complementary
-__global__ void pair_check_kernel(const GroupPair* gps, int64_t ng, uint64_t total, const int* pafa, const int* pafb,
-                                  int H, int target, uint32_t* flags) {
-    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total;
-         w += (uint64_t)gridDim.x * blockDim.x) {
+// one thread per candidate pair of [w0, w0 + n): flags[w - w0] = 1 if pair w is
+// complementary
+__global__ void pair_check_kernel(const GroupPair* gps, int64_t ng, uint64_t w0, uint64_t n, const int* pafa,
+                                  const int* pafb, int H, int target, uint32_t* flags) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t w = w0 + i;
         int64_t lo = 0, hi = ng - 1;
         while (lo < hi) {
             const int64_t mid = (lo + hi + 1) >> 1;
@@ -119,7 +120,7 @@ __global__ void pair_check_kernel(const GroupPair* gps, int64_t ng, uint64_t tot
                 ok = 0;
                 break;
             }
-        flags[w] = ok;
+        flags[i] = ok;
     }
 }
 
@@ -453,7 +454,7 @@ int find_lines(gp_ctx* c, const char* d_text, size_t n, DevBuf& start, DevBuf& l
 }
 
 struct Cand {
-    std::vector<uint32_t> tok_off, tok_len;  // first token in the text
+    std::vector<size_t> tok_off, tok_len;  // first token in the text (of any size)
     std::vector<int8_t> seqs;                // L per line
     size_t n = 0;
 };
@@ -479,8 +480,8 @@ bool parse_candidates(const std::string& text, int L, Cand& out, std::string& er
             if (q < nl) {
                 const char* t = q;
                 while (q < nl && *q != ' ') ++q;
-                o.tok_off.push_back((uint32_t)(t - base));
-                o.tok_len.push_back((uint32_t)(q - t));
+                o.tok_off.push_back((size_t)(t - base));
+                o.tok_len.push_back((size_t)(q - t));
                 int got = 0;
                 while (got < L) {
                     while (q < nl && *q == ' ') ++q;
@@ -533,14 +534,21 @@ void put_pair(std::string& s, const int8_t* a, const int8_t* b, int L) {
 
 }  // namespace
 
-// Shared with the uncompression stage: match two sorted candidate texts and
-// append the pairs to `out`.  Returns GP_EMPTY_INPUT if either is empty.
+// Candidate pairs checked at once: their indices in a slice are 32 bits, and the
+// slice's arrays 12 GB.
+constexpr uint64_t kMatchSlice = uint64_t(1) << 30;
+
+// Match two candidate texts and append the pairs to `out`: any size of text and
+// any number of candidate pairs, up to 2^32 - 1 lines a side.  Returns
+// GP_EMPTY_INPUT if either text is empty.
 int gp_match_texts(gp_ctx* c, int L, int compress, int paf, const std::string& ta, const std::string& tb,
                    std::string& out, int64_t* n_pairs) {
     if (ta.empty() || tb.empty()) return GP_EMPTY_INPUT;
     Cand A, B;
     std::string err;
     if (!parse_candidates(ta, L, A, err) || !parse_candidates(tb, L, B, err)) return c->fail(GP_ERR_FORMAT, "match: %s", err.c_str());
+    if (std::max(A.n, B.n) > UINT32_MAX)
+        return c->fail(GP_ERR_UNSUPPORTED, "match: %zu lines", std::max(A.n, B.n));
     // group boundaries and the merge on the first token (std::string order)
     auto tok = [](const std::string& t, const Cand& x, size_t i) {
         return std::string_view(t.data() + x.tok_off[i], x.tok_len[i]);
@@ -570,10 +578,10 @@ int gp_match_texts(gp_ctx* c, int L, int compress, int paf, const std::string& t
     cudaStream_t s = c->s_comp;
     const int H = L / 2;
     DevBuf da, db, dpa, dpb, dg, df, dpos, dscan, dlist;
-    const int64_t need_flags = (int64_t)total;
+    const int64_t slice = (int64_t)std::min(total, kMatchSlice);
     if (!da.ensure(A.seqs.size() + 16) || !db.ensure(B.seqs.size() + 16) || !dpa.ensure(A.n * (H + 1) * 4) ||
-        !dpb.ensure(B.n * (H + 1) * 4) || !dg.ensure(gps.size() * sizeof(GroupPair)) || !df.ensure(need_flags * 4) ||
-        !dpos.ensure(need_flags * 4) || !dscan.ensure(gp::scan_tmp_bytes(need_flags)) || !dlist.ensure(need_flags * 4 + 4))
+        !dpb.ensure(B.n * (H + 1) * 4) || !dg.ensure(gps.size() * sizeof(GroupPair)) || !df.ensure(slice * 4) ||
+        !dpos.ensure(slice * 4) || !dscan.ensure(gp::scan_tmp_bytes(slice)) || !dlist.ensure(slice * 4 + 4))
         return c->fail(GP_ERR_NOMEM, "match: device allocation");
     GP_CUDA_TRY(c, cudaMemcpyAsync(da.p, A.seqs.data(), A.seqs.size(), cudaMemcpyHostToDevice, s));
     GP_CUDA_TRY(c, cudaMemcpyAsync(db.p, B.seqs.data(), B.seqs.size(), cudaMemcpyHostToDevice, s));
@@ -582,18 +590,24 @@ int gp_match_texts(gp_ctx* c, int L, int compress, int paf, const std::string& t
         paf_kernel<<<grid_for((int64_t)A.n), 256, 0, s>>>(da.as<int8_t>(), (int64_t)A.n, L, H, dpa.as<int>());
         paf_kernel<<<grid_for((int64_t)B.n), 256, 0, s>>>(db.as<int8_t>(), (int64_t)B.n, L, H, dpb.as<int>());
     }
-    pair_check_kernel<<<grid_for((int64_t)total), 256, 0, s>>>(dg.as<GroupPair>(), (int64_t)gps.size(), total,
-                                                               dpa.as<int>(), dpb.as<int>(), H, paf * compress,
-                                                               df.as<uint32_t>());
-    GP_CUDA_TRY(c, cudaGetLastError());
-    uint32_t* d_cnt = dlist.as<uint32_t>() + need_flags;
-    GP_CUDA_TRY(c, gp::compact_flags(df.as<uint32_t>(), nullptr, dlist.as<uint32_t>(), need_flags, dpos.as<uint32_t>(),
-                                     dscan.as<uint32_t>(), d_cnt, s));
-    uint32_t nk = 0;
-    GP_CUDA_TRY(c, cudaMemcpyAsync(&nk, d_cnt, 4, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
-    std::vector<uint32_t> keep(nk);
-    if (nk) GP_CUDA_TRY(c, cudaMemcpy(keep.data(), dlist.p, (size_t)nk * 4, cudaMemcpyDeviceToHost));
+    std::vector<uint64_t> keep;  // in the flattened product
+    std::vector<uint32_t> kept;  // in a slice
+    for (uint64_t w0 = 0; w0 < total; w0 += slice) {
+        const int64_t n = (int64_t)std::min<uint64_t>(slice, total - w0);
+        pair_check_kernel<<<grid_for(n), 256, 0, s>>>(dg.as<GroupPair>(), (int64_t)gps.size(), w0, (uint64_t)n,
+                                                      dpa.as<int>(), dpb.as<int>(), H, paf * compress,
+                                                      df.as<uint32_t>());
+        GP_CUDA_TRY(c, cudaGetLastError());
+        uint32_t* d_cnt = dlist.as<uint32_t>() + n;
+        GP_CUDA_TRY(c, gp::compact_flags(df.as<uint32_t>(), nullptr, dlist.as<uint32_t>(), n, dpos.as<uint32_t>(),
+                                         dscan.as<uint32_t>(), d_cnt, s));
+        uint32_t nk = 0;
+        GP_CUDA_TRY(c, cudaMemcpyAsync(&nk, d_cnt, 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+        kept.resize(nk);
+        if (nk) GP_CUDA_TRY(c, cudaMemcpy(kept.data(), dlist.p, (size_t)nk * 4, cudaMemcpyDeviceToHost));
+        for (uint32_t k : kept) keep.push_back(w0 + k);
+    }
     // pair lines in order, formatted in blocks by host threads
     const size_t per = 1 << 14;
     const size_t nblk = (keep.size() + per - 1) / per;
@@ -602,11 +616,11 @@ int gp_match_texts(gp_ctx* c, int L, int compress, int paf, const std::string& t
         const size_t lo = bi * per, hi = std::min(keep.size(), lo + per);
         std::string& o = blk[bi];
         o.reserve((hi - lo) * (size_t)(6 * L + 2));
-        size_t g = (size_t)(std::upper_bound(gps.begin(), gps.end(), (uint64_t)keep[lo],
+        size_t g = (size_t)(std::upper_bound(gps.begin(), gps.end(), keep[lo],
                                              [](uint64_t w, const GroupPair& x) { return w < x.first; }) -
                             gps.begin()) - 1;
         for (size_t k = lo; k < hi; ++k) {
-            const uint32_t w = keep[k];
+            const uint64_t w = keep[k];
             while (g + 1 < gps.size() && gps[g + 1].first <= w) ++g;
             const uint64_t off = w - gps[g].first;
             const uint32_t ia = gps[g].a0 + (uint32_t)(off / gps[g].nb);
@@ -615,7 +629,7 @@ int gp_match_texts(gp_ctx* c, int L, int compress, int paf, const std::string& t
         }
     });
     for (const std::string& o : blk) out += o;
-    if (n_pairs) *n_pairs = nk;
+    if (n_pairs) *n_pairs = (int64_t)keep.size();
     return GP_OK;
 }
 
@@ -698,6 +712,9 @@ int gp_sort_text(gp_ctx* c, const std::string& text, std::string& out) {
     const int64_t n = (int64_t)start.size();
     out.clear();
     if (n == 0) return GP_OK;
+    // line numbers and lengths are 32 bits
+    if (n > UINT32_MAX || maxlen > UINT32_MAX)
+        return c->fail(GP_ERR_UNSUPPORTED, "sort: %lld lines, the longest of %zu bytes", (long long)n, maxlen);
     const int per = nibble ? 8 : 4;
     const int W = (int)((maxlen + per - 1) / per) + 0;
     const int Wk = W < 1 ? 1 : W;
