@@ -315,4 +315,4 @@ class Context:
 
 def unpack_mask(mask, n):
     # the unpacked bytes are 0 and 1: bools without a second pass over them
-    return np.unpackbits(mask.view(np.uint8), count=n, bitorder="little").view(np.bool_)
+    return np.unpackbits(mask.view(np.uint8), bitorder="little")[:n].view(np.bool_)
