@@ -1763,7 +1763,8 @@ int run_level(gp_ctx* c, const Level& lv, const std::vector<uint8_t>& seqs, FILE
             max_fc = std::max<uint64_t>(max_fc, sd.free_choices);
         }
         bt.smem = (size_t)(max_sc + max_fc) * lv.np * 16;
-        cudaError_t e = cudaFuncSetAttribute(bt.scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt.smem);
+        // (a side's suffixes are at most smax, its choices at most the whole term table)
+        cudaError_t e = gp::allow_smem(bt.scan, kScanSmemBudget);
         int per_sm = 0;
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bt.scan, kScanThreads, bt.smem);

@@ -278,6 +278,15 @@ __global__ void __launch_bounds__(kWarps * 32) finalize_multi_kernel(FinalizeMul
 
 size_t finalize_smem(int L) { return sizeof(double2) * L + kWarps * finalize_layout(L).per_warp; }
 
+size_t most_smem() {
+    static const size_t most = [] {
+        size_t m = 0;
+        for (int L = 1; L <= kMaxLen; ++L) m = std::max(m, finalize_smem(L));
+        return m;
+    }();
+    return most;
+}
+
 }  // namespace
 
 cudaError_t launch_mask_to_list(const uint32_t* mask, int64_t n, uint32_t* out, unsigned long long* count,
@@ -295,7 +304,7 @@ cudaError_t launch_finalize(const FinalizeArgs& a, int64_t max_rows, int num_sms
     int64_t blocks = (max_rows + kWarps - 1) / kWarps;
     if (blocks > (int64_t)num_sms * 16) blocks = (int64_t)num_sms * 16;
     const size_t smem = finalize_smem(a.src.L);
-    cudaError_t e = cudaFuncSetAttribute(finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(finalize_kernel, most_smem());
     if (e != cudaSuccess) return e;
     finalize_kernel<<<(unsigned)blocks, kWarps * 32, smem, st>>>(a);
     return cudaGetLastError();
@@ -328,8 +337,7 @@ cudaError_t launch_finalize_multi(const FinalizeMultiArgs& a, const int64_t* max
     // per job as many blocks as its own launch would take: blocks of a job
     // with fewer rows end at once
     if (blocks > (int64_t)num_sms * 16) blocks = (int64_t)num_sms * 16;
-    cudaError_t e =
-        cudaFuncSetAttribute(finalize_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(finalize_multi_kernel, most_smem());
     if (e != cudaSuccess) return e;
     finalize_multi_kernel<<<dim3((unsigned)blocks, (unsigned)a.njobs), kWarps * 32, smem, st>>>(a);
     return cudaGetLastError();

@@ -17,6 +17,15 @@ constexpr int kMaxTcK = 128;    // largest padded K of the tensor-core filter (L
 constexpr int kMaxLen = 512;    // longest sequence any kernel takes
 
 // ------------------------------------------------------------ PSD filter
+// The dynamic shared memory a kernel may be launched with is an attribute of the
+// function, so one for all threads and contexts of a device.  Every call sets the
+// same value, the most that any of its layouts takes: with each call's own size
+// there, a launch of another thread that needs more can fail between the two.
+template <class Kernel>
+cudaError_t allow_smem(Kernel* kern, size_t most) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 struct PsdTcArgs {
     const int8_t* seqs;      // n x L, row-major (int8 input), or nullptr
     const uint4* words;      // n packed words (packed input), or nullptr

@@ -7,7 +7,9 @@
 //     tensor-core path): bins k = 1..L/2, a few at a time for the rows that
 //     no bin has ruled out yet, those that cost least first;
 //   * psd_fp64_values: every bin of a batch (tests).
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <type_traits>
 
 #include "gp_device.cuh"
@@ -283,8 +285,12 @@ cudaError_t launch_psd_fp64(const PsdF64Args& a, cudaStream_t st) {
     if (a.n == 0) return cudaSuccess;
     const F64Layout lay = f64_layout(a.src.L, a.n, a.num_sms);
     const int64_t blocks = (a.n + lay.rows - 1) / lay.rows;
-    cudaError_t e =
-        cudaFuncSetAttribute(psd_fp64_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total);
+    static const size_t most = [] {
+        size_t m = 0;
+        for (int L = 1; L <= kMaxLen; ++L) m = std::max(m, f64_layout(L, INT64_MAX, 1).total);
+        return m;
+    }();
+    cudaError_t e = allow_smem(psd_fp64_filter_kernel, most);
     if (e != cudaSuccess) return e;
     psd_fp64_filter_kernel<<<(unsigned)blocks, kBlock, lay.total, st>>>(a, lay);
     return cudaGetLastError();
@@ -293,8 +299,9 @@ cudaError_t launch_psd_fp64(const PsdF64Args& a, cudaStream_t st) {
 cudaError_t launch_psd_fp64_values(const RowSrc& src, const double* tw, int64_t n, double* out, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     const int64_t blocks = (n + kBlock - 1) / kBlock;
-    const size_t smem = sizeof(double2) * src.L + (size_t)kBlock * src.L + 16;
-    cudaError_t e = cudaFuncSetAttribute(psd_values_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto bytes = [](int L) { return sizeof(double2) * L + (size_t)kBlock * L + 16; };
+    const size_t smem = bytes(src.L);
+    cudaError_t e = allow_smem(psd_values_kernel, bytes(kMaxLen));
     if (e != cudaSuccess) return e;
     psd_values_kernel<<<(unsigned)blocks, kBlock, smem, st>>>(src, tw, n, out);
     return cudaGetLastError();

@@ -59,6 +59,7 @@
 // stages as accumulators, the MMAs of a tile free its A stage when they
 // complete, so one commit (accumulator full) serves the epilogue and the
 // converters.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -77,6 +78,17 @@ __global__ void __launch_bounds__(kThreads, TcCfg<K, WRITE_PSD>::MIN_BLOCKS) psd
 // largest padded K with shifted int8 loads (one mask register per 4 bytes)
 constexpr int kMaxShiftK = 64;
 
+// The largest layout of any row length.
+template <int K, bool WP>
+uint32_t most_smem() {
+    static const uint32_t most = [] {
+        uint32_t m = 0;
+        for (int r = 1; r <= K; ++r) m = std::max(m, smem_layout<K, WP>(r).total);
+        return m;
+    }();
+    return most;
+}
+
 template <int K, int B, bool WP>
 cudaError_t launch_kb(const PsdTcArgs& a, int num_sms, cudaStream_t st) {
     using C = TcCfg<K, WP>;
@@ -94,7 +106,7 @@ cudaError_t launch_kb(const PsdTcArgs& a, int num_sms, cudaStream_t st) {
         if constexpr (K <= kMaxShiftK)
             if (a.trace && a.i8_shift) kern = psd_tc_kernel<K, B, WP, true, true>;
     }
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total);
+    cudaError_t e = allow_smem(kern, most_smem<K, WP>());
     if (e != cudaSuccess) return e;
     const int per_sm = a.grid_per_sm > 0 && a.grid_per_sm < C::MIN_BLOCKS ? a.grid_per_sm : C::MIN_BLOCKS;
     int64_t grid = (int64_t)num_sms * per_sm;

@@ -135,7 +135,7 @@ template <int KMAX>
 cudaError_t launch_multi(const PsdTcMultiArgs& a, int num_sms, cudaStream_t st) {
     const SmemLayout lay = multi_layout<KMAX>();
     auto kern = psd_tc_multi_kernel<KMAX>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total);
+    cudaError_t e = allow_smem(kern, lay.total);  // the same for every call
     if (e != cudaSuccess) return e;
     int64_t cap_tiles = 0;
     for (int j = 0; j < a.njobs; ++j) cap_tiles += (a.job[j].n + kTileM - 1) / kTileM;
