@@ -27,6 +27,7 @@
 #include "finalize.h"
 #include "gen_text.h"
 #include "host_math.h"
+#include "host_par.h"
 #include "survivors.h"
 
 namespace {
@@ -69,24 +70,24 @@ void parallel_sort(std::vector<T>& v, Cmp cmp) {
     std::vector<size_t> bounds;
     for (unsigned t = 0; t <= hw; ++t) bounds.push_back(n * t / hw);
     {
-        std::vector<std::thread> th;
+        gp::Workers th;
         for (unsigned t = 0; t < hw; ++t)
-            th.emplace_back([&, t] { std::sort(v.begin() + bounds[t], v.begin() + bounds[t + 1], cmp); });
-        for (auto& x : th) x.join();
+            th.run([&, t] { std::sort(v.begin() + bounds[t], v.begin() + bounds[t + 1], cmp); });
+        th.join();
     }
     std::vector<T> tmp(n);
     while (bounds.size() > 2) {
         std::vector<size_t> nb;
-        std::vector<std::thread> th;
+        gp::Workers th;
         for (size_t i = 0; i + 1 < bounds.size(); i += 2) {
             const size_t lo = bounds[i], mid = bounds[i + 1], hi = i + 2 < bounds.size() ? bounds[i + 2] : mid;
             nb.push_back(lo);
-            th.emplace_back([&, lo, mid, hi] {
+            th.run([&, lo, mid, hi] {
                 std::merge(v.begin() + lo, v.begin() + mid, v.begin() + mid, v.begin() + hi, tmp.begin() + lo, cmp);
             });
         }
         nb.push_back(n);
-        for (auto& x : th) x.join();
+        th.join();
         v.swap(tmp);
         bounds.swap(nb);
     }
@@ -101,6 +102,12 @@ int write_records(gp_ctx* c, const GenPlan& p, const RecordSet& recs, int role, 
     if (c->out_format == GP_FORMAT_BINARY) return write_records_binary(c, p, recs, order, role, path);
     FILE* f = fopen(path, "w");
     if (!f) return c->fail(GP_ERR_IO, "cannot open %s for writing", path);
+    struct Closer {
+        FILE* f;
+        ~Closer() {
+            if (f) fclose(f);
+        }
+    } closer{f};
     const size_t per_block = 1 << 13;  // lines per formatting task
     const size_t nblocks = (n + per_block - 1) / per_block;
     unsigned nthreads = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
@@ -109,11 +116,11 @@ int write_records(gp_ctx* c, const GenPlan& p, const RecordSet& recs, int role, 
     // rounds of nthreads blocks: format in parallel, write in order; the
     // next round is formatted while this one is written
     std::vector<std::string> bufs[2] = {std::vector<std::string>(nthreads), std::vector<std::string>(nthreads)};
+    gp::Workers th;
     auto format_round = [&](size_t b0, std::vector<std::string>& bs) {
-        std::vector<std::thread> th;
         const unsigned m = (unsigned)std::min<size_t>(nthreads, nblocks - b0);
         for (unsigned t = 0; t < m; ++t) {
-            th.emplace_back([&, t, b0] {
+            th.run([&, t, b0] {
                 std::string& out = bs[t];
                 out.clear();
                 const size_t lo = (b0 + t) * per_block, hi = std::min(n, lo + per_block);
@@ -124,19 +131,19 @@ int write_records(gp_ctx* c, const GenPlan& p, const RecordSet& recs, int role, 
                 }
             });
         }
-        return th;
     };
     if (nblocks) {
-        std::vector<std::thread> th = format_round(0, bufs[0]);
+        format_round(0, bufs[0]);
         for (size_t b0 = 0, r = 0; b0 < nblocks; b0 += nthreads, r ^= 1) {
-            for (auto& x : th) x.join();
+            th.join();
             const unsigned m = (unsigned)std::min<size_t>(nthreads, nblocks - b0);
-            th = b0 + nthreads < nblocks ? format_round(b0 + nthreads, bufs[r ^ 1]) : std::vector<std::thread>();
+            if (b0 + nthreads < nblocks) format_round(b0 + nthreads, bufs[r ^ 1]);
             for (unsigned t = 0; t < m && ok; ++t)
                 if (fwrite(bufs[r][t].data(), 1, bufs[r][t].size(), f) != bufs[r][t].size()) ok = false;
         }
-        for (auto& x : th) x.join();
+        th.join();
     }
+    closer.f = nullptr;
     ok = (fclose(f) == 0) && ok;
     return ok ? GP_OK : c->fail(GP_ERR_IO, "write failed: %s", path);
 }
@@ -826,7 +833,8 @@ int write_lines(gp_ctx* c, const char* text, size_t bytes, const char* path) {
 int finish(gp_ctx* c, const JobRun& j, const char* path_a, const char* path_b, gp_gen_stats* st) {
     const gp::GenText& t = j.text;
     int rc_a = GP_OK;
-    std::thread ta([&] {  // A and B files side by side
+    gp::Workers ta;
+    ta.run([&] {  // A and B files side by side
         rc_a = t.p ? write_lines(c, t.p.get(), t.bytes_a, path_a) : write_records(c, j.p, j.ra, 0, path_a);
     });
     const int rc_b = t.p ? write_lines(c, t.p.get() + t.bytes_a, t.bytes - t.bytes_a, path_b)
@@ -1039,8 +1047,8 @@ int64_t gp_job_ranges(int order, int compress, int paf, int proc_id, int proc_nu
     return (int64_t)ranges.size();
 }
 
-int gp_generate(gp_ctx* c, int order, int compress, int paf, int proc_id, int proc_num, const char* path_a,
-                const char* path_b, gp_gen_stats* stats) {
+static int gp_generate_impl(gp_ctx* c, int order, int compress, int paf, int proc_id, int proc_num, const char* path_a,
+                            const char* path_b, gp_gen_stats* stats) {
     if (!c || !path_a || !path_b) return GP_ERR_ARG;
     if (proc_num < 1 || proc_id < 0 || proc_id >= proc_num)
         return c->fail(GP_ERR_ARG, "bad job split %d of %d", proc_id, proc_num);
@@ -1077,9 +1085,19 @@ int gp_generate(gp_ctx* c, int order, int compress, int paf, int proc_id, int pr
     return GP_OK;
 }
 
-int gp_generate_window(gp_ctx* c, int order, int compress, int paf, uint64_t begin_hi, uint64_t begin_lo,
-                       uint64_t end_hi, uint64_t end_lo, const char* path_a, const char* path_b,
-                       gp_gen_stats* stats) {
+// No C++ exception (no host memory for the records or their text) crosses the C ABI.
+int gp_generate(gp_ctx* c, int order, int compress, int paf, int proc_id, int proc_num, const char* path_a,
+                const char* path_b, gp_gen_stats* stats) {
+    try {
+        return gp_generate_impl(c, order, compress, paf, proc_id, proc_num, path_a, path_b, stats);
+    } catch (const std::exception& e) {
+        return c ? c->fail(GP_ERR_NOMEM, "generation: %s", e.what()) : GP_ERR_NOMEM;
+    }
+}
+
+static int gp_generate_window_impl(gp_ctx* c, int order, int compress, int paf, uint64_t begin_hi, uint64_t begin_lo,
+                                   uint64_t end_hi, uint64_t end_lo, const char* path_a, const char* path_b,
+                                   gp_gen_stats* stats) {
     if (!c || !path_a || !path_b) return GP_ERR_ARG;
     const auto t0 = std::chrono::steady_clock::now();
     cudaSetDevice(c->device);
@@ -1107,10 +1125,21 @@ int gp_generate_window(gp_ctx* c, int order, int compress, int paf, uint64_t beg
     return GP_OK;
 }
 
+int gp_generate_window(gp_ctx* c, int order, int compress, int paf, uint64_t begin_hi, uint64_t begin_lo,
+                       uint64_t end_hi, uint64_t end_lo, const char* path_a, const char* path_b,
+                       gp_gen_stats* stats) {
+    try {
+        return gp_generate_window_impl(c, order, compress, paf, begin_hi, begin_lo, end_hi, end_lo, path_a, path_b,
+                                       stats);
+    } catch (const std::exception& e) {
+        return c ? c->fail(GP_ERR_NOMEM, "generation: %s", e.what()) : GP_ERR_NOMEM;
+    }
+}
+
 }  // extern "C"
 
-extern "C" int gp_generate_batch(gp_ctx* c, const gp_gen_job* jobs, int njobs, int autotune, gp_batch_config* cfg,
-                                 gp_gen_stats* stats) {
+static int gp_generate_batch_impl(gp_ctx* c, const gp_gen_job* jobs, int njobs, int autotune, gp_batch_config* cfg,
+                                  gp_gen_stats* stats) {
     if (!c || !jobs) return GP_ERR_ARG;
     if (njobs < 1 || njobs > gp::kMaxEnumJobs)
         return c->fail(GP_ERR_ARG, "batch of %d jobs (1..%d)", njobs, gp::kMaxEnumJobs);
@@ -1155,12 +1184,10 @@ extern "C" int gp_generate_batch(gp_ctx* c, const gp_gen_job* jobs, int njobs, i
     {
         // the jobs' files in parallel (each file is formatted by host threads too)
         std::vector<int> rcs(njobs, GP_OK);
-        std::vector<std::thread> th;
+        gp::Workers th;
         for (int i = 0; i < njobs; ++i)
-            th.emplace_back([&, i] {
-                rcs[i] = finish(c, run[i], jobs[i].path_a, jobs[i].path_b, &run[i].st);
-            });
-        for (auto& t : th) t.join();
+            th.run([&, i] { rcs[i] = finish(c, run[i], jobs[i].path_a, jobs[i].path_b, &run[i].st); });
+        th.join();
         for (int i = 0; i < njobs; ++i)
             if (rcs[i]) return rcs[i];
     }
@@ -1182,6 +1209,15 @@ extern "C" int gp_generate_batch(gp_ctx* c, const gp_gen_job* jobs, int njobs, i
         cfg->tune_seconds = tune_s;
     }
     return GP_OK;
+}
+
+extern "C" int gp_generate_batch(gp_ctx* c, const gp_gen_job* jobs, int njobs, int autotune, gp_batch_config* cfg,
+                                 gp_gen_stats* stats) {
+    try {
+        return gp_generate_batch_impl(c, jobs, njobs, autotune, cfg, stats);
+    } catch (const std::exception& e) {
+        return c ? c->fail(GP_ERR_NOMEM, "batch generation: %s", e.what()) : GP_ERR_NOMEM;
+    }
 }
 
 extern "C" int gp_generate_resumable(gp_ctx* c, int order, int compress, int paf, int proc_id, int proc_num,

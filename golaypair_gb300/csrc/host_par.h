@@ -1,17 +1,55 @@
-// host_par.h -- host-side helpers of the text stages: a block-parallel loop
-// over up to 16 threads, cutting a text into line-aligned chunks, and a
+// host_par.h -- host-side helpers of the text stages: threads that hand their
+// exceptions on, a block-parallel loop over up to 16 of them, cutting a text into line-aligned chunks, and a
 // decimal integer reader/writer for the small entries of candidate lines.
 #pragma once
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <exception>
+#include <mutex>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 namespace gp {
 
 inline unsigned host_threads() { return std::max(1u, std::min(16u, std::thread::hardware_concurrency())); }
+
+// Host threads of one call.  An exception in one (an allocation failure) would
+// end the process there: the first is kept and thrown by join() on the calling
+// thread instead.  They are joined on every way out.
+class Workers {
+public:
+    Workers() = default;
+    Workers(const Workers&) = delete;
+    Workers& operator=(const Workers&) = delete;
+    ~Workers() { wait(); }
+    template <class F>
+    void run(F fn) {
+        th.emplace_back([this, fn] {
+            try {
+                fn();
+            } catch (...) {
+                std::lock_guard<std::mutex> lock(mu);
+                if (!first) first = std::current_exception();
+            }
+        });
+    }
+    void join() {
+        wait();
+        if (std::exception_ptr e = std::exchange(first, nullptr)) std::rethrow_exception(e);
+    }
+
+private:
+    void wait() {
+        for (auto& t : th) t.join();
+        th.clear();
+    }
+    std::vector<std::thread> th;
+    std::mutex mu;
+    std::exception_ptr first;
+};
 
 // fn(b) for b in [0, nblocks), blocks dealt round robin to the threads.
 template <class F>
