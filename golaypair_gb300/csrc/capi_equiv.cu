@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "host_par.h"
 #include "pair_text.cuh"
 #include "prims.h"
 
@@ -1073,10 +1074,10 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
             const int64_t ng = (int64_t)(gens.size() / (size_t)W);
             std::vector<int16_t> items((size_t)ng * W);  // transposed: items[o * ng + g]
             {
-                const unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-                std::vector<std::thread> th;
+                const unsigned nt = gp::host_threads();
+                gp::Workers th;
                 for (unsigned t = 0; t < nt; ++t)
-                    th.emplace_back([&, t] {
+                    th.run([&, t] {
                         // blocks of 64 generators: each thread writes whole cache lines of every row
                         for (int64_t g0 = (int64_t)t * 64; g0 < ng; g0 += (int64_t)nt * 64)
                             for (int64_t g = g0; g < std::min<int64_t>(g0 + 64, ng); ++g) {
@@ -1084,7 +1085,7 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
                                 for (int o = 0; o < W; ++o) items[(size_t)o * ng + g] = s[o];
                             }
                     });
-                for (auto& x : th) x.join();
+                th.join();
             }
             lap("table");
             std::vector<int8_t> pairs((size_t)np * W);

@@ -2,6 +2,7 @@
 // the text exporter of binary survivor files (format in survivors.h), and
 // the spectral pruning switch (its lookup table).
 #include <cstdio>
+#include <exception>
 #include <string>
 #include <vector>
 
@@ -55,7 +56,7 @@ int gp_set_spectral_prune(gp_ctx* c, int on) {
     return GP_OK;
 }
 
-int gp_export_text(gp_ctx* c, const char* in_path, const char* out_path) {
+static int gp_export_text_impl(gp_ctx* c, const char* in_path, const char* out_path) {
     if (!in_path || !out_path) return c ? c->fail(GP_ERR_ARG, "export: null path") : GP_ERR_ARG;
     std::string bytes;
     if (!read_all(in_path, bytes)) return fail_or(c, GP_ERR_IO, "export: cannot read", in_path);
@@ -69,6 +70,15 @@ int gp_export_text(gp_ctx* c, const char* in_path, const char* out_path) {
     bool ok = text.empty() || fwrite(text.data(), 1, text.size(), f) == text.size();
     ok = (fclose(f) == 0) && ok;
     return ok ? GP_OK : fail_or(c, GP_ERR_IO, "export: write failed", out_path);
+}
+
+// No C++ exception (no room for the file or its text) crosses the C ABI.
+int gp_export_text(gp_ctx* c, const char* in_path, const char* out_path) {
+    try {
+        return gp_export_text_impl(c, in_path, out_path);
+    } catch (const std::exception& e) {
+        return fail_or(c, GP_ERR_NOMEM, "export", e.what());
+    }
 }
 
 }  // extern "C"

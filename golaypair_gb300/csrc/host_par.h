@@ -59,12 +59,12 @@ void par_for(size_t nblocks, F&& fn) {
         for (size_t b = 0; b < nblocks; ++b) fn(b);
         return;
     }
-    std::vector<std::thread> th;
+    Workers th;
     for (unsigned t = 0; t < nt; ++t)
-        th.emplace_back([&, t] {
+        th.run([&, t] {
             for (size_t b = t; b < nblocks; b += nt) fn(b);
         });
-    for (auto& x : th) x.join();
+    th.join();
 }
 
 // Start offsets of up to `parts` chunks of text[0, n), each starting at a

@@ -23,10 +23,10 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "host_math.h"
+#include "host_par.h"
 
 namespace gp {
 
@@ -128,17 +128,11 @@ inline bool surv_to_text(const SurvHeader& h, const uint8_t* body, std::string& 
     const uint64_t n = h.count;
     const uint64_t per = 1 << 14;
     const uint64_t nblocks = (n + per - 1) / per;
-    unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    if (nblocks < nt) nt = (unsigned)std::max<uint64_t>(1, nblocks);
     std::vector<std::string> parts(nblocks);
     std::vector<char> ok(nblocks, 1);
-    std::vector<std::thread> th;
-    for (unsigned t = 0; t < nt; ++t)
-        th.emplace_back([&, t] {
-            for (uint64_t b = t; b < nblocks; b += nt)
-                ok[b] = surv_format_range(h, body, b * per, std::min(n, (b + 1) * per), parts[b]);
-        });
-    for (auto& x : th) x.join();
+    par_for(nblocks, [&](uint64_t b) {
+        ok[b] = surv_format_range(h, body, b * per, std::min(n, (b + 1) * per), parts[b]);
+    });
     for (uint64_t b = 0; b < nblocks; ++b) {
         if (!ok[b]) return false;
         out += parts[b];

@@ -1,4 +1,4 @@
-// Calls a generation entry point while large host allocations fail: all from
+// Calls a generation entry point, or the text export (host only), while large host allocations fail: all from
 // the first-th on, `count` of them.  Prints the return code.  Exits with 2
 // when an exception crosses the C ABI, with 3 when one ends a thread.
 #include <atomic>
@@ -34,13 +34,15 @@ int main(int argc, char** argv) {
     fail_count = std::atol(argv[4]);
     std::set_terminate([] { _exit(3); });
     gp_ctx* c = nullptr;
-    if (gp_ctx_create(&c, 0) != GP_OK) return 1;
+    if (entry != "export" && gp_ctx_create(&c, 0) != GP_OK) return 1;
     const std::string a = dir + "/a", b = dir + "/b", a2 = dir + "/a2", b2 = dir + "/b2";
     int rc = 1;
     armed = true;
     try {
         if (entry == "generate") {
             rc = gp_generate(c, 45, 3, -2, 0, 1, a.c_str(), b.c_str(), nullptr);
+        } else if (entry == "export") {
+            rc = gp_export_text(nullptr, (dir + "/in").c_str(), a.c_str());
         } else if (entry == "window") {
             rc = gp_generate_window(c, 45, 3, -2, 0, 0, 0, 1u << 30, a.c_str(), b.c_str(), nullptr);
         } else {
@@ -56,6 +58,6 @@ int main(int argc, char** argv) {
     }
     armed = false;
     std::printf("%d\n", rc);
-    gp_ctx_destroy(c);
+    if (c) gp_ctx_destroy(c);
     return 0;
 }
