@@ -17,9 +17,10 @@
 // applies every element of the closure with the reference's application
 // rule (equivalence.cpp:97-144), hashing the images of several pairs per
 // pass over the transposed table and looking them up in a hash set of the
-// input pairs.  The pairs' text is read and written, and the pairs and least
-// images sorted, on the device too.  Either way the host then replays the reference's in-order
-// erase loop (filter.cpp:117-144) on those class sizes and member lists.
+// input pairs.  Text past kHostText is read and written, and its pairs and least
+// images sorted, on the device too.  Either way the host then replays the
+// reference's in-order erase loop (filter.cpp:117-144) on those class sizes and
+// member lists.
 #include <algorithm>
 #include <chrono>
 #include <stdexcept>
@@ -387,8 +388,8 @@ __global__ void __launch_bounds__(32 * kCanonWarps) canon_kernel(CanonArgs a) {
 }
 
 // ------------------------------------------------------------ pair text
-// The pair file is parsed, its pairs sorted and the kept ones written as text
-// on the device: on the host that took 57 of the 73 ms of 30,000 order-57
+// A pair file past kHostText is parsed, its pairs sorted and the kept ones written
+// as text on the device: on the host that took 57 of the 73 ms of 30,000 order-57
 // pairs (strtol, a vector per pair, std::sort, one digit at a time), here
 // about 1 ms beside the file itself.
 
@@ -735,6 +736,8 @@ struct PairSet {
     int8_t* rows = nullptr;
     int bits = 1, Wk = 1; // key layout
     const uint8_t* code = nullptr;
+    bool small = false;   // a small file: parsed, sorted and written by the host
+    std::vector<int8_t> host;  // then the rows here too
 };
 
 enum EqBuf { kEqText, kEqCount, kEqOffs, kEqScan, kEqVals, kEqInfo, kEqCode, kEqKeys, kEqIdx, kEqTmp, kEqFlag, kEqPos,
@@ -756,6 +759,50 @@ int sort_rows(PairSet& ps, const int8_t* rows, int64_t n, uint32_t* idx, uint32_
     return GP_OK;
 }
 
+// Files up to this size are the host's: parsing and sorting on the device is some
+// fifty launches and nine waits, as many for two pairs as for twenty thousand.
+// The two ways meet between 38 KB (length 6) and 90 KB (length 90).  On the host
+// and on the device: 2 pairs of length 6 91 and 330 us, 1,000 (32 KB) 328 and
+// 380, 2,000 571 and 417; 100 pairs of length 57 (29 KB) 268 and 485, 200 438 and
+// 504, 300 617 and 518.
+constexpr size_t kHostText = 40 << 10;
+
+// Numbers of the n rows of W bytes in the rows' order, equal rows in index order.
+std::vector<uint32_t> host_order(const uint8_t* rows, int64_t n, int W) {
+    std::vector<uint32_t> ord(n);
+    for (int64_t i = 0; i < n; ++i) ord[i] = (uint32_t)i;
+    std::sort(ord.begin(), ord.end(), [&](uint32_t x, uint32_t y) {
+        const int d = std::memcmp(rows + (size_t)x * W, rows + (size_t)y * W, (size_t)W);
+        return d != 0 ? d < 0 : x < y;
+    });
+    return ord;
+}
+
+// load_pairs on the host; the rows go to the device for canon_kernel.
+int load_pairs_host(PairSet& ps, const char* text, cudaStream_t s) {
+    gp_ctx* c = ps.c;
+    const int W = ps.W;
+    const std::vector<int8_t> vals = host_values(text);
+    const int64_t n = (int64_t)vals.size() / W;
+    std::vector<uint8_t> bytes((size_t)n * W);  // in the order of the values
+    for (size_t i = 0; i < bytes.size(); ++i) bytes[i] = (uint8_t)(vals[i] ^ 0x80);
+    const uint8_t* last = nullptr;
+    for (uint32_t i : host_order(bytes.data(), n, W)) {
+        const uint8_t* row = bytes.data() + (size_t)i * W;
+        if (last && std::memcmp(last, row, (size_t)W) == 0) continue;
+        last = row;
+        ps.host.insert(ps.host.end(), vals.begin() + (size_t)i * W, vals.begin() + (size_t)(i + 1) * W);
+    }
+    ps.small = true;
+    ps.np = (int64_t)ps.host.size() / W;
+    if (ps.np == 0) return GP_OK;
+    DevBuf& drow = c->eq[kEqRows];
+    if (!drow.ensure(ps.host.size())) return c->fail(GP_ERR_NOMEM, "equivalence filter: pairs");
+    ps.rows = drow.as<int8_t>();
+    GP_CUDA_TRY(c, cudaMemcpyAsync(ps.rows, ps.host.data(), ps.host.size(), cudaMemcpyHostToDevice, s));
+    return GP_OK;
+}
+
 // filter.cpp:45-62: L values for a, then (if the stream is still good) L for
 // b: whitespace-separated integers up to the first token that is not one, W
 // per pair, a trailing partial pair dropped; then the set of the pairs.
@@ -763,6 +810,7 @@ int sort_rows(PairSet& ps, const int8_t* rows, int64_t n, uint32_t* idx, uint32_
 int load_pairs(PairSet& ps, const char* text, size_t n, cudaStream_t s) {
     gp_ctx* c = ps.c;
     if (n == 0 || ps.W < 1) return GP_OK;  // no values, or none to a pair
+    if (n <= kHostText) return load_pairs_host(ps, text, s);
     const bool huge = n >> 32;  // more text than the device's 32-bit offsets reach
     const int64_t blocks = huge ? 1 : (int64_t)((n + kParseBlock - 1) / kParseBlock);
     DevBuf &dt = c->eq[kEqText], &dcnt = c->eq[kEqCount], &doff = c->eq[kEqOffs], &dscan = c->eq[kEqScan],
@@ -871,14 +919,25 @@ int canonical_classes(PairSet& ps, int L, int compress, std::vector<unsigned lon
     canon_kernel<<<(unsigned)grid, 32 * kCanonWarps, smem, s>>>(ca);
     GP_CUDA_TRY(c, cudaGetLastError());
     // the classes: runs of equal least images
-    const int rc = sort_rows(ps, ca.canon, np, didx.as<uint32_t>(), dflag.as<uint32_t>(), s);
-    if (rc) return rc;
     std::vector<uint32_t> fixers(np), flags(np);
-    member_list.resize(np);
-    GP_CUDA_TRY(c, cudaMemcpyAsync(fixers.data(), df.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaMemcpyAsync(flags.data(), dflag.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaMemcpyAsync(member_list.data(), didx.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
-    GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    if (ps.small) {
+        std::vector<uint8_t> canon((size_t)np * W);
+        GP_CUDA_TRY(c, cudaMemcpyAsync(fixers.data(), df.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(canon.data(), dc.p, canon.size(), cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+        member_list = host_order(canon.data(), np, W);
+        for (int64_t k = 0; k < np; ++k)
+            flags[k] = k == 0 || std::memcmp(&canon[(size_t)member_list[k - 1] * W],
+                                             &canon[(size_t)member_list[k] * W], (size_t)W) != 0;
+    } else {
+        const int rc = sort_rows(ps, ca.canon, np, didx.as<uint32_t>(), dflag.as<uint32_t>(), s);
+        if (rc) return rc;
+        member_list.resize(np);
+        GP_CUDA_TRY(c, cudaMemcpyAsync(fixers.data(), df.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(flags.data(), dflag.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaMemcpyAsync(member_list.data(), didx.p, (size_t)np * 4, cudaMemcpyDeviceToHost, s));
+        GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+    }
     const uint64_t G = pair_group_size(L, compress);
     for (int64_t i = 0; i < np; ++i) {
         if (fixers[i] == 0 || G % fixers[i] != 0)
@@ -901,6 +960,18 @@ int pair_lines(PairSet& ps, const std::vector<char>& alive, std::string& out, cu
     out.clear();
     if (ps.np == 0) return GP_OK;
     const int64_t np = ps.np;
+    if (ps.small) {
+        const int W = ps.W, L = W / 2;
+        for (int64_t i = 0; i < np; ++i) {
+            if (!alive[i]) continue;
+            for (int o = 0; o < W; ++o) {
+                if (o == L) out.push_back(' ');
+                gp::put_int_sp(out, ps.host[(size_t)i * W + o]);
+            }
+            out.push_back('\n');
+        }
+        return GP_OK;
+    }
     // rows at a time: a block's text stays below 2^31 bytes (5 bytes a value at most)
     const int64_t step = std::min<int64_t>(np, (int64_t(1) << 31) / (5 * ps.W + 2));
     DevBuf &da = c->eq[kEqAlive], &db = c->eq[kEqBytes], &dat = c->eq[kEqPos], &dscan = c->eq[kEqScan],
@@ -1073,24 +1144,20 @@ static int gp_equiv_filter_impl(gp_ctx* c, int order, int compress, const char* 
             lap("group");
             const int64_t ng = (int64_t)(gens.size() / (size_t)W);
             std::vector<int16_t> items((size_t)ng * W);  // transposed: items[o * ng + g]
-            {
-                const unsigned nt = gp::host_threads();
-                gp::Workers th;
-                for (unsigned t = 0; t < nt; ++t)
-                    th.run([&, t] {
-                        // blocks of 64 generators: each thread writes whole cache lines of every row
-                        for (int64_t g0 = (int64_t)t * 64; g0 < ng; g0 += (int64_t)nt * 64)
-                            for (int64_t g = g0; g < std::min<int64_t>(g0 + 64, ng); ++g) {
-                                const auto s = as_sources(gens.data() + (size_t)g * W, L);
-                                for (int o = 0; o < W; ++o) items[(size_t)o * ng + g] = s[o];
-                            }
-                    });
-                th.join();
-            }
+            // blocks of 64 generators: each thread writes whole cache lines of every row
+            gp::par_for((size_t)((ng + 63) / 64), [&](size_t blk) {
+                for (int64_t g = (int64_t)blk * 64; g < std::min<int64_t>((int64_t)blk * 64 + 64, ng); ++g) {
+                    const auto src = as_sources(gens.data() + (size_t)g * W, L);
+                    for (int o = 0; o < W; ++o) items[(size_t)o * ng + g] = src[o];
+                }
+            });
             lap("table");
-            std::vector<int8_t> pairs((size_t)np * W);
-            GP_CUDA_TRY(c, cudaMemcpyAsync(pairs.data(), ps.rows, pairs.size(), cudaMemcpyDeviceToHost, s));
-            GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+            std::vector<int8_t> pairs = ps.host;
+            if (!ps.small) {
+                pairs.resize((size_t)np * W);
+                GP_CUDA_TRY(c, cudaMemcpyAsync(pairs.data(), ps.rows, pairs.size(), cudaMemcpyDeviceToHost, s));
+                GP_CUDA_TRY(c, cudaStreamSynchronize(s));
+            }
             // hash set of the pairs (the image lookup), same hash as the kernel's
             uint32_t set_size = 1;
             while (set_size < 2 * (uint64_t)np) set_size <<= 1;
