@@ -77,6 +77,9 @@ constexpr int kBucketTarget = 512;  // survivors per join bucket (mean)
 constexpr int kJoinTab = 4096;      // shared hash slots of the join kernel
 constexpr int kJoinMaxB = kJoinTab / 2;
 constexpr size_t kScanSmemBudget = 96 * 1024;
+// The context's scratch for the matched pairs and their lines, ux[36] to ux[43]:
+// some hundred bytes a match, so a call of many gives them back.
+constexpr int kUxMatch = 36, kUxMatchCount = 8;
 
 // ------------------------------------------------------------ device side
 
@@ -1624,8 +1627,9 @@ int Batcher::run(int64_t p0, int64_t p1, bool* overflowed) {
     const int digits = (int)std::to_string(std::abs((long long)bound)).size() + 1;
     const int W = 1 + ((N - 1) * digits + 2 + 2 * N * 5 + 7) / 8;
     const uint64_t chunk = std::min<uint64_t>(nm, (uint64_t(1) << 31) / (uint64_t)(10 * N + 2));  // lines at once
-    DevBuf &dseqs = c->ux[36], &dkey = c->ux[37], &dord = c->ux[38], &dtmp = c->ux[39], &dbytes = c->ux[40],
-           &doff = c->ux[41], &dtext = c->ux[42], &dkept = c->ux[43];
+    DevBuf* mb = &c->ux[kUxMatch];
+    DevBuf &dseqs = mb[0], &dkey = mb[1], &dord = mb[2], &dtmp = mb[3], &dbytes = mb[4], &doff = mb[5], &dtext = mb[6],
+           &dkept = mb[7];
     if (nm > INT32_MAX || !dseqs.ensure(nm * 2 * N) || !dkey.ensure(nm * W * 4) || !dord.ensure(nm * 4) ||
         !dtmp.ensure(std::max(gp::radix_sort_tmp_bytes((int64_t)nm, W), gp::scan_tmp_bytes((int64_t)chunk + 1))) ||
         !dbytes.ensure((chunk + 1) * 4) || !doff.ensure((chunk + 1) * 4) || !dkept.ensure(4)) {
@@ -1823,6 +1827,7 @@ int uncompress_chain_impl(gp_ctx* c, int order, const int* compress, int ncomp, 
     if (first < 0 || step < 1) return c->fail(GP_ERR_ARG, "uncompress: bad line range (first %lld, step %lld)",
                                               (long long)first, (long long)step);
     cudaSetDevice(c->device);
+    KeepSmall keep{&c->ux[kUxMatch], kUxMatchCount};  // the others are kept across calls
     std::vector<int8_t> carried;  // the previous level's pairs (values), 2 L per pair
     bool have_input = true;
     for (int lvl = 0; lvl + 1 < ncomp; ++lvl) {

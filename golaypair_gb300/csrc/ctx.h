@@ -84,6 +84,7 @@ struct KeepSmall {
     size_t n;
     template <size_t N>
     explicit KeepSmall(DevBuf (&bufs)[N]) : b(bufs), n(N) {}
+    KeepSmall(DevBuf* first, size_t count) : b(first), n(count) {}
     ~KeepSmall() {
         for (size_t i = 0; i < n; ++i)
             if (b[i].cap > (size_t(64) << 20)) b[i].release();

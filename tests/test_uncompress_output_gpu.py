@@ -1,5 +1,6 @@
 """The uncompression's output file and buffers."""
 import ctypes
+import threading
 
 import pytest
 
@@ -37,3 +38,34 @@ def test_uncompress_onto_a_full_disk(tmp_path, whole):
         # the first pairs' lines stay in the stream's buffer until it is closed
         assert size > 1 << 16 if whole else 0 < size < 4096
         assert _uncompress(ctx, tmp_path, 16, 2, 1, 0, "/dev/full") == -6  # GP_ERR_IO
+
+
+def test_many_matches_leave_no_buffers_of_theirs(tmp_path):
+    # a match of this order takes 260 bytes of sort key alone; a call's match
+    # buffers are there while it runs, and those above 64 MB gone after it
+    torch = pytest.importorskip("torch")
+    with gp.Context(0) as ctx:
+        lines = _pairs(ctx, tmp_path, 39, 3, -2)
+        (tmp_path / "in").write_text("".join(lines))
+        assert _uncompress(ctx, tmp_path, 39, 3, 1, -2, tmp_path / "out") == 0
+        per_copy = (tmp_path / "out").read_text().count("\n")
+        copies = -(-(1 << 20) // per_copy)
+        (tmp_path / "in").write_text("".join(lines) * copies)
+        assert _uncompress(ctx, tmp_path, 39, 3, 1, -2, tmp_path / "out") == 0  # every other buffer has its size
+        after, least = torch.cuda.mem_get_info()[0], []
+        done = threading.Event()
+
+        def watch():
+            while not done.is_set():
+                least.append(torch.cuda.mem_get_info()[0])
+
+        t = threading.Thread(target=watch)
+        t.start()
+        try:
+            assert _uncompress(ctx, tmp_path, 39, 3, 1, -2, tmp_path / "out") == 0
+        finally:
+            done.set()
+            t.join()
+        assert (tmp_path / "out").stat().st_size > 1 << 26
+        assert after - min(least) >= 260 << 20
+        assert torch.cuda.mem_get_info()[0] >= after - (1 << 20)
