@@ -16,6 +16,16 @@ double threshold(int order, int paf) { return 2.0 * order - paf + 0.001; }
 // configured guard band: 1e-3 * 2n (absolute PSD units)
 float guard_band(int order) { return (float)(2e-3 * order); }
 
+gp::RowSrc int8_src(const int8_t* d, int L) {
+    gp::RowSrc r;
+    r.seqs = d;
+    r.words = nullptr;
+    r.L = L;
+    r.pack_bits = 0;
+    r.alpha_c = 0;
+    return r;
+}
+
 }  // namespace
 
 const void* gp_ctx::twiddle_image(int L, bool int8_rows, int* shift, bool both) {
@@ -48,14 +58,13 @@ const double* gp_ctx::twiddle64(int L) {
     return b.as<double>();
 }
 
-int gp_ctx::enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf, int mode, uint32_t* d_mask,
+int gp_ctx::enqueue_filter(const int8_t* d_seqs, int L, int64_t n, int order, int paf, int mode, uint32_t* d_mask,
                            uint32_t* d_unsure, unsigned long long* d_ucount, cudaStream_t st) {
-    const int L = src.L;
     const int64_t words = (n + 31) / 32;
     const double* tw = twiddle64(L);
     if (!tw) return fail(GP_ERR_NOMEM, "twiddle table");
     if (mode == GP_PSD_FP64) {
-        gp::PsdF64Args a{src, tw, n, threshold(order, paf), d_mask, words, num_sms};
+        gp::PsdF64Args a{int8_src(d_seqs, L), tw, n, threshold(order, paf), d_mask, words, num_sms};
         cudaEvent_t tb;
         time_begin(st, &tb);
         GP_CUDA_TRY(this, gp::launch_psd_fp64(a, st));
@@ -63,19 +72,17 @@ int gp_ctx::enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf,
         return GP_OK;
     }
     int shift = 0;
-    const void* img = twiddle_image(L, src.seqs != nullptr, &shift);
+    const void* img = twiddle_image(L, true, &shift);
     if (!img) return fail(GP_ERR_UNSUPPORTED, "tensor-core filter: unsupported length %d", L);
-    if (src.words && !gp::tc_packed_supported(L, src.pack_bits))
-        return fail(GP_ERR_UNSUPPORTED, "tensor-core filter: packed length %d x %d bits", L, src.pack_bits);
     if (d_ucount) GP_CUDA_TRY(this, cudaMemsetAsync(d_ucount, 0, sizeof(unsigned long long), st));
     gp::PsdTcArgs a;
     a.recheck = 1;
     a.thr64 = threshold(order, paf);
     a.i8_shift = shift;
-    a.seqs = src.seqs;
-    a.words = src.words;
-    a.pack_bits = src.pack_bits;
-    a.alpha_c = src.alpha_c;
+    a.seqs = d_seqs;
+    a.words = nullptr;
+    a.pack_bits = 0;
+    a.alpha_c = 0;
     a.n = n;
     a.L = L;
     a.bimage = img;
@@ -359,16 +366,6 @@ int gp_kernel_time(gp_ctx* c, double* total_ms, int64_t* launches) {
 
 int gp_device_sm_count(const gp_ctx* c) { return c ? c->num_sms : 0; }
 
-static gp::RowSrc int8_src(const int8_t* d, int L) {
-    gp::RowSrc r;
-    r.seqs = d;
-    r.words = nullptr;
-    r.L = L;
-    r.pack_bits = 0;
-    r.alpha_c = 0;
-    return r;
-}
-
 // *out += number of set bits in w[0 .. nwords)
 __global__ void popcount_add_kernel(const uint32_t* w, int64_t nwords, unsigned long long* out) {
     unsigned long long s = 0;
@@ -426,7 +423,7 @@ int gp_psd_filter(gp_ctx* c, const int8_t* seqs, int64_t n, int L, int order, in
             GP_CUDA_TRY(c, cudaEventRecord(c->ev_part[q], c->s_copies[q]));
             GP_CUDA_TRY(c, cudaStreamWaitEvent(c->s_comp, c->ev_part[q], 0));
         }
-        rc = c->enqueue_filter(int8_src(c->seq_buf[b].as<int8_t>(), L), rows, order, paf, mode,
+        rc = c->enqueue_filter(c->seq_buf[b].as<int8_t>(), L, rows, order, paf, mode,
                                c->mask_buf[b].as<uint32_t>(), c->unsure_buf[b].as<uint32_t>(), d_counts + b, c->s_comp);
         if (rc) return rc;
         GP_CUDA_TRY(c, cudaMemcpyAsync(pass_mask + r0 / 32, c->mask_buf[b].p, (size_t)(rows + 31) / 32 * 4,
@@ -476,7 +473,7 @@ int gp_psd_filter_device(gp_ctx* c, const int8_t* d_seqs, int64_t n, int L, int 
     if (mode == GP_PSD_TC_GUARDED && !c->unsure_buf[0].ensure((size_t)std::max<int64_t>(n, 1) * 4))
         return c->fail(GP_ERR_NOMEM, "psd filter: device allocation failed");
     // without stats nothing is counted: the call is one launch
-    rc = c->enqueue_filter(int8_src(d_seqs, L), n, order, paf, mode, d_mask, c->unsure_buf[0].as<uint32_t>(),
+    rc = c->enqueue_filter(d_seqs, L, n, order, paf, mode, d_mask, c->unsure_buf[0].as<uint32_t>(),
                            stats ? c->counts.as<unsigned long long>() : nullptr, st);
     if (rc) return rc;
     if (stats) {

@@ -125,7 +125,6 @@ struct gp_ctx {
     DevBuf status;          // int
     DevBuf counts;          // unsigned long long [8]
     HostPinned h_counts;    // mirror of counts, per chunk
-    HostPinned h_ux;        // uncompression: record counts of the two sides
     // PSD filter staging
     DevBuf seq_buf[2];
     DevBuf mask_buf[2];
@@ -193,10 +192,10 @@ struct gp_ctx {
                              unsigned long long* const* d_ucount, int njobs, int grid_per_sm, cudaStream_t st);
     // device FP64 twiddle table for length L
     const double* twiddle64(int L);
-    // Enqueues the PSD filter of a device batch (int8 rows or packed words)
-    // on st: mask bit = pass; TC mode rechecks its unsure rows in FP64 and
-    // counts them in *d_ucount unless it is null.
-    int enqueue_filter(const gp::RowSrc& src, int64_t n, int order, int paf, int mode, uint32_t* d_mask,
+    // Enqueues the PSD filter of a device batch of int8 rows on st: mask bit =
+    // pass; TC mode rechecks its unsure rows in FP64 and counts them in
+    // *d_ucount unless it is null.
+    int enqueue_filter(const int8_t* d_seqs, int L, int64_t n, int order, int paf, int mode, uint32_t* d_mask,
                        uint32_t* d_unsure, unsigned long long* d_ucount, cudaStream_t st);
     // TC-mode filter of a device batch whose row count is read on the device
     // (*n_dev, at most cap rows): nothing here depends on the count, so the

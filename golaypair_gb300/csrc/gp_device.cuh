@@ -202,13 +202,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v) {
         : "memory");
 }
 
-// 4 consecutive 32-bit columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t* v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
-                 "r"(v[2]), "r"(v[3])
-                 : "memory");
-}
-
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }

@@ -42,7 +42,7 @@ struct PsdTcArgs {
     float err_coef;          // per-row |X| error bound = S_row * err_coef
     uint32_t* mask;          // ceil(n/32) words; bit = sure pass or unsure
     int64_t mask_words;
-    // Unsure rows (near the bound): with recheck, the CTA that found them
+    // Unsure rows (near the bound): with recheck (int8 rows), the CTA that found them
     // decides them in FP64 against thr64 before it ends, from its own part of
     // `unsure` (n entries: the p-th of a CTA at the place of its p-th row);
     // without, their mask bits stay set for a caller that filters exactly.

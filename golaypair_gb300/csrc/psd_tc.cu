@@ -96,6 +96,7 @@ cudaError_t launch_kb(const PsdTcArgs& a, int num_sms, cudaStream_t st) {
     const int64_t ntiles = (a.n + kTileM - 1) / kTileM;
     if (ntiles == 0) return cudaSuccess;
     if (a.n >= (int64_t(1) << 31)) return cudaErrorInvalidValue;  // 32-bit row indices
+    if (a.recheck && B != 0) return cudaErrorInvalidValue;  // packed rows: finalize filters exactly
     if (a.i8_shift && (B != 0 || !tc_i8_shifted(a.L))) return cudaErrorInvalidValue;
     // the counting variant exists for the int8 input only (diagnostics)
     auto kern = psd_tc_kernel<K, B, WP, false, false>;

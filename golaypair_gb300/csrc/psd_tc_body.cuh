@@ -253,27 +253,6 @@ __device__ __forceinline__ void psd_chunk(uint32_t taddr, int c0, float& pmax, f
     }
 }
 
-// The hi twiddles alone: eight bins from column c0, p = c_hi^2 + s_hi^2.
-template <int HB>
-__device__ __forceinline__ void psd_chunk_hi(uint32_t taddr, int c0, float& pmax, float& x0) {
-    float chi[8], shi[8];
-    tmem_ld8(taddr + c0, chi);
-    tmem_ld8(taddr + HB + c0, shi);
-    tmem_wait_ld();
-#pragma unroll
-    for (int k = 0; k < 8; k += 2) {
-        const float2 re = make_float2(chi[k], chi[k + 1]);
-        const float2 im = make_float2(shi[k], shi[k + 1]);
-        const float2 p = __ffma2_rn(re, re, __fmul2_rn(im, im));
-        if (c0 + k + 1 == HB - 1) {
-            pmax = fmaxf(pmax, p.x);
-            x0 = re.y;  // the ones row has no lo part: X_0 is exact here
-        } else {
-            pmax = fmax3(pmax, p.x, p.y);
-        }
-    }
-}
-
 // The hi twiddles alone over all HB bins: every load issued before one wait.
 // t_ld: the cycle counter when the loads have landed (TR builds).
 template <int HB, bool TR>
@@ -402,8 +381,9 @@ __device__ __noinline__ float2 near_rows(const PsdTcArgs& a, const float2* s_tw,
 // memset and a recheck kernel: 2^12 rows of length 45 take 5.6 us (10.8 with
 // three), 2^20 rows 20.5 us (28.8), 2^26 rows of length 8, of which 4 % lie at
 // the bound, 1.02 ms (5.77: one atomic on one counter per warp, one warp per row).
+// int8 rows only: packed rows come from the generation engine, whose finalize
+// kernel filters the unsure ones exactly.
 constexpr int kFoldEntries = (kMaxTcK - 1) / 2 + 1;
-template <int B>
 __device__ __noinline__ void recheck_own(const PsdTcArgs& a, uint8_t* smem, int cnt, int first, int stride) {
     const int L = a.L, H = L / 2, J = (L - 1) / 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -418,22 +398,8 @@ __device__ __noinline__ void recheck_own(const PsdTcArgs& a, uint8_t* smem, int 
     for (int i0 = warp * R; i0 < cnt; i0 += (kThreads / 32) * R) {
         const int i = i0 + sub;
         const bool has = i < cnt;
-        uint32_t row = 0;
-        uint64_t lo = 0, hi = 0;
-        if (has) {
-            row = a.unsure[(int64_t)(first + (i >> 7) * stride) * kTileM + (i & 127)];
-            if constexpr (B != 0) {
-                const uint4 w = a.words[row];
-                lo = ((uint64_t)w.y << 32) | w.x;
-                hi = ((uint64_t)w.w << 32) | w.z;
-            }
-        }
-        auto value = [&](int j) -> int {
-            if constexpr (B == 0)
-                return a.seqs[(int64_t)row * L + j];
-            else
-                return 2 * word_digit(lo, hi, B, L, j) - a.alpha_c;
-        };
+        const uint32_t row = has ? a.unsure[(int64_t)(first + (i >> 7) * stride) * kTileM + (i & 127)] : 0u;
+        auto value = [&](int j) -> int { return a.seqs[(int64_t)row * L + j]; };
         __syncwarp();
         int x0 = 0, xm = 0;
         if (has) {
@@ -825,7 +791,7 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
             if (ub) {
                 int base = 0;
                 if (lane == 0) base = atomicAdd(n_unsure, __popc(ub));
-                if (!WRITE_PSD && a.recheck) {
+                if (B == 0 && !WRITE_PSD && a.recheck) {
                     base = __shfl_sync(0xFFFFFFFFu, base, 0);
                     const int pos = base + __popc(ub & ((1u << lane) - 1u));
                     if (unsure) a.unsure[(int64_t)(first + (pos >> 7) * stride) * kTileM + (pos & 127)] = (uint32_t)row;
@@ -968,8 +934,8 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
     const int cnt = *n_unsure;
     if (cnt == 0) return;
     if (threadIdx.x == 0 && a.unsure_count) atomicAdd(a.unsure_count, (unsigned long long)cnt);
-    if constexpr (!WRITE_PSD)
-        if (a.recheck && !*abort_flag) recheck_own<B>(a, sRaw, cnt, first, stride);
+    if constexpr (B == 0 && !WRITE_PSD)
+        if (a.recheck && !*abort_flag) recheck_own(a, sRaw, cnt, first, stride);
 }
 
 }  // namespace

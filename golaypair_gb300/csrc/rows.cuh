@@ -13,10 +13,6 @@
 
 namespace gp {
 
-struct u128w {
-    uint64_t lo, hi;
-};
-
 __host__ __device__ __forceinline__ int word_digit(uint64_t lo, uint64_t hi, int b, int L, int j) {
     const int pos = b * (L - 1 - j);  // lowest bit of digit j
     const uint64_t m = (1ull << b) - 1ull;
