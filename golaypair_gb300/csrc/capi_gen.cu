@@ -215,7 +215,7 @@ constexpr int kCounterWords = kCumBase + kCumSlots * gp::kMaxEnumJobs;
 
 struct BatchCfg {
     int enum_variant = 0;        // enumerator kernel variant (see launch_enumerate)
-    int windows_per_thread = 1;  // rank windows per enumerator thread
+    int windows_per_thread = 1;  // rank windows per enumerator thread and job
     int64_t cand_cap = int64_t(1) << 22;  // candidates per job per iteration (soft)
     int tc_ctas_per_sm = 0;      // tensor-core filter CTAs per SM (0 = as many as fit)
     int use_graph = 1;

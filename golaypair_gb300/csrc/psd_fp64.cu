@@ -61,7 +61,7 @@ __device__ __forceinline__ double bin_power(const int8_t* x, int L, int k, const
 constexpr int kBins = 4;
 constexpr int kFoldMax = 256;  // range of the table (x_j +- x_{L-j} of int8 rows)
 
-// rows per block: up to eight per thread (full warps until the last rounds),
+// rows per block: up to four per thread (full warps until the last rounds),
 // fewer where shared memory or the number of rows asks for it
 struct F64Layout {
     int rows;

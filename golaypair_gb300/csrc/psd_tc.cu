@@ -21,13 +21,13 @@
 // max_k p_k, which gives the per-row error bound from the values the
 // epilogue computes anyway.
 //
-// The hi and lo twiddles sit side by side along N: the B image is 2K x K,
+// Up to K = 48 the hi and lo twiddles sit side by side along N: the B image is 2K x K,
 // one UMMA of N = 2K per 16-wide K step.  A tcgen05.mma of M = 128, K = 16
 // takes ~46 cycles for any N up to 96 (measured on GB300), so one N = 2K
 // instruction per step costs half of two N = K instructions.  The epilogue
 // decides from the hi columns alone, with a guard widened by the hi-only
 // twiddle error; only a warp with a row inside that wider band reads the lo
-// columns too and decides again (about 1e-5 of the warps on int8 input).
+// columns too and decides again (2e-5 of the int8 rows of length 45).
 // Above K = 48 the accumulator holds the hi columns alone (N = K), so that two
 // CTAs fit an SM, and a row inside the band is decided again in fp32 by its
 // epilogue warp.
@@ -42,7 +42,8 @@
 //   int8 rows    n x L bytes (the batched filter's input);
 //   packed words one 16-byte word per candidate, digit j in bits
 //                [b(L-1-j), b(L-j)), value = 2*digit - c (the enumerator's
-//                and the uncompression expander's output).
+//                output).  Their unsure rows keep their mask bits: the
+//                finalize kernel filters the survivors exactly.
 //
 // The A operand (the candidates) lives in tensor memory: each converter
 // thread owns one row = one TMEM lane and writes its fp16 pairs with

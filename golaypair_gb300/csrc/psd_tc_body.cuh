@@ -315,7 +315,8 @@ __device__ __forceinline__ void psd_hi_blocks(uint32_t taddr, float& pmax, float
 // with the bins over the lanes; lane i of a flagged row gets its pair, the
 // others keep theirs.  The sum over at most 127 terms of products rounded to
 // 2^-24 each is within the accumulator's own error bound (tc_err_coef).
-// Out of line: about 1e-5 of the rows of int8 input.
+// Out of line: of int8 rows with a permitted row sum 9e-5 at length 57, 1.5e-4 at
+// 52, 3e-5 at 65, below 1e-6 from 98 on.
 template <int B>
 __device__ __noinline__ float2 near_rows(const PsdTcArgs& a, const float2* s_tw, uint32_t near, int r0, float2 mine) {
     const int lane = threadIdx.x & 31, L = a.L, H = L / 2;
@@ -459,7 +460,7 @@ __device__ __noinline__ void partial_row_store(const int8_t* seqs, int row, int 
 }
 
 // Both twiddle halves over all HB bins (the exact pass): max p and X_0.
-// Out of line: it runs for about 1e-5 of the warps of the int8 workload.
+// Out of line: 2e-5 of the int8 rows of length 45 ask for it, 6e-4 of the warps.
 template <int HB, bool WRITE_PSD>
 __device__ __noinline__ float2 exact_pass(uint32_t taddr, float* psd_row) {
     float pmax = 0.f, x0 = 0.f;
@@ -741,8 +742,8 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
             // row clearly below or above the bound is decided there.  Only
             // a warp with a row inside that band reads the lo columns too,
             // or, where the accumulator has none, takes that row's bins
-            // again in fp32 (rare: about 1e-5 of the rows of the int8
-            // workload).
+            // again in fp32 (rare: 2e-5 of the int8 rows of length 45, 9e-5
+            // of length 57).
             float pmax = 0.f, x0 = 0.f, g = 0.f;
             long long c_ld = c1t;
             bool exact = WRITE_PSD;
@@ -895,8 +896,8 @@ __device__ __forceinline__ void tc_body(const PsdTcArgs& a, const SmemLayout& la
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(b * C::N);
                 const uint32_t a0 = tmem_base + (uint32_t)(C::A_COL0 + as * (K / 2));
-                // one instruction per 16-wide K step covers the hi and lo
-                // twiddles side by side (N = 2K)
+                // one instruction per 16-wide K step: the hi and lo twiddles
+                // side by side (N = 2K) up to K = 48, the hi ones (N = K) above
 #pragma unroll
                 for (int ks = 0; ks < C::KSTEPS; ++ks)
                     umma_f16_ts_lead(d, a0 + (uint32_t)(8 * ks), bdesc0 + (uint64_t)((2 * ks * C::B_KSTRIDE) >> 4), idesc,

@@ -68,11 +68,12 @@ int gp_psd_filter(gp_ctx* ctx, const int8_t* seqs, int64_t n, int L, int order, 
  * (a cudaStream_t; NULL = the context's stream).  n < 2^31.  With stats !=
  * NULL the call synchronises and returns any device-side error.  With
  * stats == NULL it only enqueues: the mask is valid once gp_check(ctx,
- * stream) has returned GP_OK, which reports a bounded device wait that gave
- * up (GP_ERR_TIMEOUT) or an overflow (GP_ERR_OVERFLOW) of this call; until
- * then the error stays pending in the context.  The unsure list and counters
- * of the FP64 recheck belong to the context: calls on one context must not
- * overlap on the GPU (enqueue them on one stream, or wait in between).
+ * stream) has returned GP_OK, which reports a bounded device wait of this call
+ * that gave up (GP_ERR_TIMEOUT); until then the error stays pending in the
+ * context.  (The unsure list holds every row: it cannot overflow.)  The list
+ * and the counters of the FP64 recheck belong to the context: calls on one
+ * context must not overlap on the GPU (enqueue them on one stream, or wait in
+ * between).
  * d_seqs may start at any byte; the tensor-core filter streams whole tiles
  * through the bulk-copy engine only when it is 16-byte aligned, and reads
  * the rows with plain loads otherwise (same verdicts, slower). */
