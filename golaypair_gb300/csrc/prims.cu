@@ -7,7 +7,7 @@
 // is the same for every key is skipped.  One kernel counts every digit of every
 // key first, so the passes run without waiting for the host in between, and a
 // pass is two launches (block histograms, scatter) up to kScatterScanBlocks
-// blocks: the scatter sums the blocks before its own.
+// blocks and kTotalWords words: the scatter sums the blocks before its own.
 // The passes take the leading digits only, as many as hold twice the entropy
 // that n distinct rows need; rows that still agree stand next to each other
 // then and are ranked by whole keys, unless more than kRunMax of them do.
@@ -73,6 +73,9 @@ constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int64_t kScatterScanBlocks = 256;  // 2^19 keys
 constexpr int kRunMax = 32;
+// Words whose digit totals are held at once: 4 MB here and on the host (a line of
+// 8 MB held whole took 4 GB of either).  Candidate lines have some 20 words.
+constexpr int kTotalWords = 1024;
 constexpr int kTailPasses = 4;  // about what the two kernels for runs and the wait cost
 
 template <int RB>
@@ -328,7 +331,7 @@ size_t radix_sort_tmp_bytes(int64_t n, int sort_words) {
     const int64_t nb = (n + kSortTile - 1) / kSortTile;
     return (size_t)n * 4                      // ping-pong index
            + (size_t)nb * 256 * 4 * 2         // counts + offsets
-           + scan_tmp_bytes(nb * 256) + (size_t)sort_words * 4096 + 1024;
+           + scan_tmp_bytes(nb * 256) + (size_t)std::min(sort_words, kTotalWords) * 4096 + 1024;
 }
 
 // Sorts idx (a permutation of row numbers) by the keys' first `sort_words`
@@ -340,7 +343,7 @@ cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_
     if (radix_bits != 4 && radix_bits != 8) return cudaErrorInvalidValue;
     const int NB = 1 << radix_bits;
     const int per_word = 32 / radix_bits;
-    const int digits = per_word * sort_words;
+    const int64_t digits = (int64_t)per_word * sort_words;
     const int64_t nb = (n + kSortTile - 1) / kSortTile;
     uint8_t* t = static_cast<uint8_t*>(tmp);
     uint32_t* alt = reinterpret_cast<uint32_t*>(t);
@@ -351,54 +354,63 @@ cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_
     t += (size_t)nb * 256 * 4;
     t = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(t) + 255) & ~uintptr_t(255));
     uint32_t* stmp = reinterpret_cast<uint32_t*>(t);
-    // every digit's totals (at most 4 KB a word), read back once
+    // every digit's totals (at most 4 KB a word), read back for up to
+    // kTotalWords words at a time, the leading ones first
+    const int slice = std::min(sort_words, kTotalWords);
     int* longer = reinterpret_cast<int*>(stmp);
     uint32_t* total = stmp + 16;
-    stmp += 16 + (size_t)sort_words * 1024;
-    cudaError_t e = cudaMemsetAsync(longer, 0, 64 + (size_t)digits * NB * 4, st);
-    if (e != cudaSuccess) return e;
-    const dim3 tg((unsigned)std::min<int64_t>((n + kSortThreads - 1) / kSortThreads, 1216), (unsigned)std::min(sort_words, 65535));
-    if (radix_bits == 8)
-        radix_totals_kernel<8><<<tg, kSortThreads, 0, st>>>(keys, W, sort_words, n, total);
-    else
-        radix_totals_kernel<4><<<tg, kSortThreads, 0, st>>>(keys, W, sort_words, n, total);
-    std::vector<uint32_t> htotal((size_t)digits * NB);
-    e = cudaMemcpyAsync(htotal.data(), total, htotal.size() * 4, cudaMemcpyDeviceToHost, st);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return e;
+    stmp += 16 + (size_t)slice * 1024;
     // Digits that differ, and the leading ones [lead, digits) that the first
     // passes sort by.  Digits that go together (a candidate's spectrum) hold
     // less than the sum of their entropies, hence twice log2 n; 43 passes of
     // an order-51 file of 380,000 lines become 7 (35 us each there).
     std::vector<char> varies(digits, 0);
-    int lead = 0, below = 0;
+    std::vector<uint32_t> htotal((size_t)slice * per_word * NB);
+    int64_t lead = 0, below = 0;
     double entropy = 0.0;
-    for (int bi = digits - 1; bi >= 0; --bi) {
-        double h = 0.0;
-        for (int d = 0; d < NB; ++d) {
-            const uint32_t c = htotal[(size_t)bi * NB + d];
-            if (c == 0 || c == (uint32_t)n) continue;
-            varies[bi] = 1;
-            h -= (double)c / (double)n * std::log2((double)c / (double)n);
-        }
-        if (entropy >= 2.0 * std::log2((double)n)) {
-            below += varies[bi];
-        } else {
-            entropy += h;
-            lead = bi;
+    cudaError_t e;
+    for (int w0 = 0; w0 < sort_words; w0 += slice) {
+        const int words = std::min(slice, sort_words - w0);
+        const int64_t last = per_word * (int64_t)(sort_words - w0 - words);  // the slice's last digit
+        e = cudaMemsetAsync(longer, 0, 64 + (size_t)words * per_word * NB * 4, st);
+        if (e != cudaSuccess) return e;
+        const dim3 tg((unsigned)std::min<int64_t>((n + kSortThreads - 1) / kSortThreads, 1216), (unsigned)words);
+        if (radix_bits == 8)
+            radix_totals_kernel<8><<<tg, kSortThreads, 0, st>>>(keys + w0, W, words, n, total);
+        else
+            radix_totals_kernel<4><<<tg, kSortThreads, 0, st>>>(keys + w0, W, words, n, total);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        e = cudaMemcpyAsync(htotal.data(), total, (size_t)words * per_word * NB * 4, cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) return e;
+        e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return e;
+        for (int bi = per_word * words - 1; bi >= 0; --bi) {
+            double h = 0.0;
+            for (int d = 0; d < NB; ++d) {
+                const uint32_t c = htotal[(size_t)bi * NB + d];
+                if (c == 0 || c == (uint32_t)n) continue;
+                varies[last + bi] = 1;
+                h -= (double)c / (double)n * std::log2((double)c / (double)n);
+            }
+            if (entropy >= 2.0 * std::log2((double)n)) {
+                below += varies[last + bi];
+            } else {
+                entropy += h;
+                lead = last + bi;
+            }
         }
     }
     if (below <= kTailPasses) lead = below = 0;
-    const bool rows = nb <= kScatterScanBlocks;
+    const bool rows = nb <= kScatterScanBlocks && sort_words <= slice;  // the totals of every digit are there
     uint32_t* cur = idx;
     uint32_t* nxt = alt;
-    auto sort_by = [&](int from) {
-        for (int bi = from; bi < digits; ++bi) {
+    auto sort_by = [&](int64_t from) {
+        for (int64_t bi = from; bi < digits; ++bi) {
             if (!varies[bi]) continue;  // every key has the same digit here
-            const int word = sort_words - 1 - bi / per_word;
-            const int shift = radix_bits * (bi % per_word);
-            const uint32_t* tot = total + (size_t)bi * NB;
+            const int word = (int)(sort_words - 1 - bi / per_word);
+            const int shift = (int)(radix_bits * (bi % per_word));
+            const uint32_t* tot = rows ? total + (size_t)bi * NB : nullptr;
             auto pass = [&](auto rb) {
                 constexpr int RB = decltype(rb)::value;
                 if (rows) {
@@ -424,7 +436,7 @@ cudaError_t radix_sort_keys(const uint32_t* keys, int W, int sort_words, uint32_
     e = sort_by(lead);
     if (e != cudaSuccess) return e;
     if (below) {
-        const int w = sort_words - 1 - lead / per_word;
+        const int w = (int)(sort_words - 1 - lead / per_word);
         const uint32_t mask = ~0u << (radix_bits * (lead % per_word));
         uint8_t* first = reinterpret_cast<uint8_t*>(counts);  // counts and offs: a byte per row at least
         run_starts_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys, W, cur, n, w, mask, first, longer);
