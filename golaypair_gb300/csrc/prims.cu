@@ -74,7 +74,7 @@ constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int64_t kScatterScanBlocks = 256;  // 2^19 keys
 constexpr int kRunMax = 32;
 // Words whose digit totals are held at once: 4 MB here and on the host (a line of
-// 8 MB held whole took 4 GB of either).  Candidate lines have some 20 words.
+// 8 MB held whole took 8 GB of either).  Candidate lines have some 20 words.
 constexpr int kTotalWords = 1024;
 constexpr int kTailPasses = 4;  // about what the two kernels for runs and the wait cost
 

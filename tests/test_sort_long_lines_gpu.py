@@ -37,7 +37,7 @@ def test_lines_around_a_slice_of_totals(tmp_path, chars, per, same):
 
 
 def test_lines_of_megabytes_take_no_gigabytes(tmp_path):
-    """The totals of every digit of an 8 MB line would take 4 GB of host memory."""
+    """The totals of every digit of an 8 MB line would take 8 GB of host memory."""
     code = """if True:
         import ctypes, random, resource, sys
         import golaypair_gb300 as gp
